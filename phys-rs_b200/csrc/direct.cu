@@ -139,7 +139,7 @@ direct_exact_kernel(int64_t n, int64_t t0, int64_t t1, const double* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// F64: same law with FMA and rsqrt, accumulating sum m_j r / s^3 (G applied
+// F64: same law with FMA and inv_cubed, accumulating sum m_j r / s^3 (G applied
 // at the end).  Sources in [slice_lo, slice_hi); tile-aligned, so the tile
 // holding the block's own targets (the only one that can contain j == i) is
 // warp-uniform and takes the checked loop.
@@ -160,8 +160,7 @@ __device__ __forceinline__ void f64_tile(const double4* __restrict__ t, int cnt,
       mj = 0.0;
       r2 = 1.0;
     }
-    const double inv = rsqrt(r2);
-    const double w = mj * (inv * inv * inv);
+    const double w = mj * inv_cubed(r2);
     ax = fma(rx, w, ax);
     ay = fma(ry, w, ay);
     az = fma(rz, w, az);
@@ -348,7 +347,7 @@ __global__ void slice_reduce_kernel(int64_t n, int64_t t0, int64_t t1, int nslic
 
 // Subset of targets (index list), all sources; one thread per (target,
 // slice).  The self pair is skipped by index.  F64_EXACT keeps the reference
-// op order with one slice; F64 / F32C use FMA + rsqrt in f64 (the subset
+// op order with one slice; F64 / F32C use FMA + inv_cubed (the subset
 // serves as the f64 reference, so F32C is not used here).
 __global__ void __launch_bounds__(kTile)
 direct_targets_kernel(int64_t n, int64_t nt, const int64_t* __restrict__ tidx, int64_t slice_len,
@@ -392,8 +391,7 @@ direct_targets_kernel(int64_t n, int64_t nt, const int64_t* __restrict__ tidx, i
         const double rx = s.x - xi, ry = s.y - yi, rz = s.z - zi;
         const bool self = base + k == i;
         const double r2 = self ? 1.0 : fma(rx, rx, fma(ry, ry, fma(rz, rz, eps2)));
-        const double inv = rsqrt(r2);
-        const double w = self ? 0.0 : s.w * (inv * inv * inv);
+        const double w = self ? 0.0 : s.w * inv_cubed(r2);
         ax = fma(rx, w, ax);
         ay = fma(ry, w, ay);
         az = fma(rz, w, az);

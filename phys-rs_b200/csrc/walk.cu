@@ -17,7 +17,7 @@
 //              0 + sum of its children in octant order, added into the parent
 //              as one term.  Per-lane accumulators per depth live in local
 //              memory; closing a level adds it into the level above.
-//   F64        flat f64 sum of m_j r / s^3, FMA + rsqrt.
+//   F64        flat f64 sum of m_j r / s^3, FMA + inv_cubed.
 //   F32C       f32 pair terms on double-float relative coordinates
 //              r = (hi_j - hi_i) + (lo_j - lo_i); f32 partial sums folded
 //              into a (hi, lo) accumulator with two-sum every 16 nodes.
@@ -150,8 +150,7 @@ walk_kernel(int q0, int n, int nnodes, const Rec32* __restrict__ w32, const Rec6
       acc = L.y >= 0 || s2d[d] < theta2 * d2;  // gravity_tree.rs:194
       const bool use = act && acc && L.y != p;
       if (use) {
-        const double inv = rsqrt(d2 + eps2);
-        const double w = A64.w * (inv * inv * inv);
+        const double w = A64.w * inv_cubed(d2 + eps2);
         ax = fma(rx, w, ax);
         ay = fma(ry, w, ay);
         az = fma(rz, w, az);
@@ -180,8 +179,7 @@ walk_kernel(int q0, int n, int nnodes, const Rec32* __restrict__ w32, const Rec6
             const double4 b = body64[q];
             if (use) {
               const double rx = b.x - tx, ry = b.y - ty, rz = b.z - tz;
-              const double inv = rsqrt(fma(rx, rx, fma(ry, ry, fma(rz, rz, eps2))));
-              const double w = b.w * (inv * inv * inv);
+              const double w = b.w * inv_cubed(fma(rx, rx, fma(ry, ry, fma(rz, rz, eps2))));
               ax = fma(rx, w, ax);
               ay = fma(ry, w, ay);
               az = fma(rz, w, az);
