@@ -195,6 +195,7 @@ int sector_normalize(phys_ctx* c, int32_t* shifted);
 // direct.cu
 int direct_eval(phys_ctx* c, const phys_params* p, bool want_force, double* ox, double* oy,
                 double* oz);
+int direct_exact_tick(phys_ctx* c, const phys_params* p, double dt, bool to_scratch);
 int direct_targets(phys_ctx* c, const phys_params* p, int64_t nt, const int64_t* d_tidx,
                    double* ox, double* oy, double* oz);
 // Launches on stream s with caller-provided scratch; returns the launch error.
@@ -314,6 +315,57 @@ __device__ __forceinline__ bool div_recip_den_ok(double b) {
 __device__ __forceinline__ bool div_recip_num_ok(double a) {
   const long long bits = __double_as_longlong(a);
   return (unsigned long long)((bits >> 52) & 0x7ff) - 523ull <= 1000ull || bits == 0;
+}
+
+// RN(a / RN(x RN(sqrt x))), the reference's pair weight (gravity.rs:60-64),
+// in 26 FP64 operations without a branch, so that several pairs' chains
+// overlap; the library's square root and division each end in a range branch
+// that keeps the next pair behind it.
+//   y    1/sqrt(x) within 1.01 u (u = 2^-53): the 21-bit f64 estimate (PTX
+//        rsqrt.approx.ftz.f64) and two terms of the series (1 - h)^(-1/2)
+//   root s = RN(x y) has an exact remainder r = x - s^2 in an FMA, and
+//        RN(s + r y/2) is RN(sqrt x) (Markstein 1990, as in div_recip):
+//        the value before that rounding is within 2^-104 of sqrt x, and
+//        every x whose root lies closer than 2^-95 to a midpoint (the
+//        solutions of K^2 = c mod 2^54 and 2^55, |c| < 2^14) was compared
+//   z    RN(1/s3): y^3 is within 7 u, one Newton step within 1 u, and the
+//        second step's value before rounding within 2^-106 of 1/s3.  The
+//        significand B = 2^53 - d of s3 has 1/s3 within 2^-53 ulp of a
+//        midpoint only for d = 1, where rounding to either side keeps
+//        div_recip's condition B^2 (1 + 2^-53) < 2^106
+// div_recip's range test is left to the caller, who makes sure of it for
+// many pairs at once: x in [2^-200, 2^200) (scale_eps2_ok, and scale_pos_ok
+// of both positions), a the product of two scale_mass_ok values (the sign of
+// a zero result may differ from the library's).  Elsewhere the caller takes
+// exact_scale_ieee.  4 x 10^10 random pairs over these ranges equal the
+// library's results.
+__device__ __forceinline__ double exact_scale(double a, double x) {
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+  const double h = __fma_rn(-x, __dmul_rn(y0, y0), 1.0);
+  const double y = __fma_rn(__dmul_rn(y0, h), __fma_rn(h, 0.375, 0.5), y0);
+  const double s = __dmul_rn(x, y);
+  const double root = __fma_rn(__fma_rn(-s, s, x), __dmul_rn(0.5, y), s);
+  const double s3 = __dmul_rn(x, root);
+  const double z0 = __dmul_rn(__dmul_rn(y, y), y);
+  const double z1 = __fma_rn(__fma_rn(-s3, z0, 1.0), z0, z0);
+  const double z = __fma_rn(__fma_rn(-s3, z1, 1.0), z1, z1);
+  return div_recip(a, s3, z);
+}
+__host__ __device__ inline bool scale_eps2_ok(double eps2) {
+  return eps2 >= 0x1p-200 && eps2 < 0x1p199;
+}
+// Coordinates within +-2^98: |r|^2 < 3 x 2^198.
+__device__ __forceinline__ bool scale_pos_ok(double x, double y, double z) {
+  return fmax(fmax(fabs(x), fabs(y)), fabs(z)) < 0x1p98 && x == x && y == y && z == z;
+}
+// |v| in [2^-250, 2^250) or 0.
+__device__ __forceinline__ bool scale_mass_ok(double v) {
+  return ((unsigned)__double2hiint(v) & 0x7fffffffu) - (773u << 20) < (500u << 20) || v == 0.0;
+}
+// The same with the library's operations.
+static __device__ __noinline__ double exact_scale_ieee(double a, double x) {
+  return xdiv(a, xmul(x, xsqrt(x)));
 }
 
 // Knuth two-sum: s + e == a + b exactly.

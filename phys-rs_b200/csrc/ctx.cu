@@ -351,9 +351,20 @@ int verlet_steps(phys_ctx* c, const phys_params* p, double dt, int64_t nsteps, b
   }
   c->accel_params = *p;
   // the direct sum's ticks have no host synchronisation: the middle ones
-  // replay a captured graph of one tick (one launch instead of a handful)
-  const bool by_graph = p->method == PHYS_DIRECT && nsteps >= 4 && !c->copy_x[0];
+  // replay a captured graph of one tick (one launch instead of a handful), or
+  // in the exact form run as one kernel per tick (pairs of ticks, so that the
+  // positions end where they began)
+  const bool fused = p->method == PHYS_DIRECT && p->precision == PHYS_F64_EXACT && !c->halo_on &&
+                     c->n >= 2;
+  const bool by_graph = p->method == PHYS_DIRECT && !fused && nsteps >= 4 && !c->copy_x[0];
   for (int64_t s = 0; s < nsteps; ++s) {
+    if (fused && s > 0) {
+      for (; s + 2 < nsteps; s += 2) {
+        c->accel_valid = false;
+        PHYS_TRY(direct_exact_tick(c, p, dt, true));
+        PHYS_TRY(direct_exact_tick(c, p, dt, false));
+      }
+    }
     if (by_graph && s == 1 && tick_graph(c, p, dt)) {
       // ticks 1 .. nsteps-2: force pass, velocity step, next position step
       for (; s + 1 < nsteps; ++s) {

@@ -5,6 +5,8 @@
 // warp reads the same source (shared-memory broadcast) while owning one
 // target.  For small N the source range is split into `slices` so the grid
 // covers all SMs; slice partials are reduced in slice order (deterministic).
+#include <utility>
+
 #include "common.cuh"
 
 namespace phys {
@@ -15,127 +17,193 @@ namespace {
 //   r = x_j - x_i; r2 = len2(r); s2 = r2 + eps2; s3 = s2 * sqrt(s2)
 //   sc = ((G*m_i)*m_j)/s3; F += r*sc            (gravity.rs:58-65)
 // Only the additions into F are ordered; the terms r*sc are independent.  A
-// block takes kXT targets: in round k its compute warps evaluate the terms
-// of sources [k kXJ, (k+1) kXJ) against every target into shared memory
-// (each thread one source against two targets, the source of round k+1
-// loaded ahead), while lane t of warp 0 adds round k-1's terms of target t
-// in j order, skipping j == i as the reference does.  The divides and square
-// roots, whose latency bounded the one-thread-per-target form, run in
-// parallel; the sum is the reference's bit for bit.  The floor of any exact
-// form is the ordered chain of N - 1 dependent f64 additions per component
-// (an f64 add waits ≈ 8 cycles for the one before it: ≈ 4 us at N = 1024);
-// the kernel takes ≈ 4 times that.
+// block takes kXT targets.  Producer warps evaluate the terms: producer p
+// takes the chunks p, p + kProd, ... of 32 sources, a lane holding one
+// source against half of the targets at a time (that many independent chains of
+// exact_scale), and hands each chunk to warp 0 through its own shared-memory
+// slot.  Lane l of warp 0 adds component l / kXT of target l % kXT in j
+// order: one dependent f64 addition per source and nothing else on the chain
+// (the next chunk's terms are read while the current chunk's are added).  A
+// skipped term (j == i, past the end) is stored as +-0: the sum starts from
+// +0 and so is never -0, and adding a zero leaves every value as it is.  A
+// lane whose source, or a block one of whose targets, is outside
+// exact_scale's range forms its terms again with the library's square root
+// and division.
+//
+// The floor of any exact form is the ordered chain, N - 1 additions of 8.2
+// cycles (4.3 us at N = 1024; the adding warp takes 10.6 per source), and for
+// many targets the FP64 pipe, 37 operations per pair.  A tick of 1024 bodies
+// (force pass, velocity and position step) takes 12.7 us where the form with
+// one round barrier and the library's operations took 21.1 us in two
+// kernels; 20000 bodies 1.40 ms against 2.46 (about 60 % of the FP64 pipe, the
+// shared-memory traffic of the terms close behind).
+// kTick also performs the velocity step of the tick and the position step of
+// the next one on the finished components, the new positions going to a
+// second set of arrays because other blocks still read the old ones.
 // ---------------------------------------------------------------------------
-constexpr int kXT = 8;                    // targets per block
-constexpr int kXJ = 64;                   // sources per round
-constexpr int kXCompute = kXT * kXJ / 2;  // compute threads: two targets each
-// Warp 0 adds; the compute warps are the first kXCompute / 32 warps whose
-// index is not a multiple of 4, so none shares warp 0's scheduler (warps are
-// spread over an SM's four schedulers by index): warps 1-3, 5-7, 9, 10 of
-// 12; warps 4, 8 and 11 return at once.  The round barrier is a named
-// barrier over the 9 working warps only.
-constexpr int kXWarps = 12;
-constexpr int kXBlock = 32 * kXWarps;
-constexpr int kXWorking = 32 + kXCompute;
-static_assert(kXT <= 32 && kXCompute % 32 == 0 && kXJ % 32 == 0, "exact block layout");
-static_assert(kXCompute / 32 == 8 && kXWorking == 288, "bar.sync count below");
+__device__ __forceinline__ void pair_sync(int id) {  // one producer warp and warp 0
+  asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+}
+__device__ __forceinline__ void pair_arrive(int id) {
+  asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
+}
 
-__global__ void __launch_bounds__(kXBlock)
+// A tick's integration state beside the force pass: kicked velocities,
+// previous accelerations, positions written to nx/ny/nz.
+struct TickArgs {
+  double dt;
+  double *vx, *vy, *vz, *pax, *pay, *paz, *nx, *ny, *nz;
+};
+
+// kProd = 6, 8 warps, 8 targets: warps 1-3 and 5-7 produce, so that no
+// producer shares warp 0's scheduler (warps go to an SM's four schedulers by
+// index) while a block has an SM to itself (N = 1024: 9.5 us a launch inside a
+// graph, 13.0 with the other layout); kProd = 4, 5 warps, 10 targets, four
+// blocks per SM: more adding warps per SM once there are more blocks than SMs
+// (N = 4096: 68 us against 78).
+// kFast: eps^2 is in exact_scale's range; else (no softening) every pair
+// takes the library's operations.
+template <bool kFast>
+__device__ __forceinline__ double pair_weight(double a, double x) {
+  return kFast ? exact_scale(a, x) : exact_scale_ieee(a, x);
+}
+
+constexpr int x_block(int prod) { return prod == 6 ? 256 : 32 * (prod + 1); }
+constexpr int x_targets(int prod) { return prod == 6 ? 8 : 10; }
+
+template <int kProd, bool kTick, bool kFast>
+__global__ void __launch_bounds__(x_block(kProd), kProd == 6 ? 2 : 4)
 direct_exact_kernel(int64_t n, int64_t t0, int64_t t1, const double* __restrict__ x,
                     const double* __restrict__ y, const double* __restrict__ z,
                     const double* __restrict__ m, double G, double eps2, int want_force,
                     double* __restrict__ ox, double* __restrict__ oy, double* __restrict__ oz,
-                    int32_t* status) {
-  __shared__ double term[2][3][kXT][kXJ + 1];  // [round parity][x, y, z][target][source]
-  __shared__ double4 tgt[kXT];                 // x_i, y_i, z_i, G*m_i
-  const int w = threadIdx.x >> 5;
-  const int cw = (w % 4 == 0) ? -1 : w - 1 - w / 4;  // compute warp 0..7, or -1
-  if (w != 0 && (cw < 0 || cw >= kXCompute / 32)) return;  // idle: no barrier
-  // tid: warp 0 keeps its lanes; compute warp cw acts as threads 32 + 32 cw + lane
-  const int tid = w == 0 ? (int)threadIdx.x : 32 + cw * 32 + (int)(threadIdx.x & 31);
+                    TickArgs tick, int32_t* status) {
+  constexpr int kXT = x_targets(kProd), kXGroup = kXT / 2;
+  constexpr int kXRows = 3 * kXT;  // ordered sums per block, one per lane
+  static_assert(kXRows <= 32, "one adding warp");
+  __shared__ double term[kProd][kXRows][33];  // [producer][component, target][source]
+  __shared__ double4 tgt[kXT];                // x_i, y_i, z_i, G*m_i
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t i0 = t0 + blockIdx.x * (int64_t)kXT;
-  if (tid < kXT) {
-    const int64_t i = i0 + tid;
-    tgt[tid] = i < t1 ? make_double4(x[i], y[i], z[i], xmul(G, m[i]))
-                      : make_double4(0.0, 0.0, 0.0, 0.0);
+  if (threadIdx.x < kXT) {
+    const int64_t i = i0 + threadIdx.x;
+    tgt[threadIdx.x] = i < t1 ? make_double4(x[i], y[i], z[i], xmul(G, m[i]))
+                              : make_double4(0.0, 0.0, 0.0, 0.0);
   }
-  asm volatile("bar.sync 1, 288;" ::: "memory");  // kXWorking
-  const int64_t rounds = ceil_div(n, kXJ);
-  // compute threads: source slot jj, targets ta and ta + kXT/2
-  const int c = tid - 32, jj = c % kXJ, ta = c / kXJ;
-  double4 src = make_double4(0.0, 0.0, 0.0, 0.0);
-  if (tid >= 32 && jj < n) src = make_double4(x[jj], y[jj], z[jj], m[jj]);
-  double fx = 0.0, fy = 0.0, fz = 0.0;  // warp 0, lane t < kXT: target t
-  for (int64_t k = 0; k <= rounds; ++k) {
-    const int b = (int)(k & 1);
-    if (tid >= 32) {
-      if (k < rounds) {
-        const int64_t j = k * kXJ + jj;
-        const int64_t jn = j + kXJ;
-        double4 next = make_double4(0.0, 0.0, 0.0, 0.0);
-        if (jn < n) next = make_double4(x[jn], y[jn], z[jn], m[jn]);
+  __syncthreads();
+  const int chunks = (int)ceil_div(n, 32);
+  // barrier ids: 1 + p a full slot, 1 + kProd + p a slot read out
+  if (w > 0) {
+    if (kProd == 6 && w == 4) return;
+    const int p = kProd == 6 ? w - 1 - (w > 4) : w - 1;
+    bool targets_ok = true;
+    for (int t = 0; t < kXT; ++t)
+      targets_ok &= scale_mass_ok(tgt[t].w) && scale_pos_ok(tgt[t].x, tgt[t].y, tgt[t].z);
+    auto load = [&](int64_t j) {
+      return j < n ? make_double4(x[j], y[j], z[j], m[j]) : make_double4(0.0, 0.0, 0.0, 0.0);
+    };
+    for (int k = p; k < chunks; k += kProd) {
+      const int64_t j = k * (int64_t)32 + lane;
+      const double4 src = load(j);
+      if (k >= kProd) pair_sync(1 + kProd + p);
+#pragma unroll 1
+      for (int tg = 0; tg < kXT; tg += kXGroup) {
+        // every weight of the group first: a store between two of them would
+        // keep the second pair's chain behind the first's
+        double rx[kXGroup], ry[kXGroup], rz[kXGroup], wt[kXGroup];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int t = ta + h * (kXT / 2);
+        for (int u = 0; u < kXGroup; ++u) {
+          const int t = tg + u;
           const double4 T = tgt[t];
-          double ax = 0.0, ay = 0.0, az = 0.0;
-          if (j < n && i0 + t < t1) {
-            const double rx = xsub(src.x, T.x), ry = xsub(src.y, T.y), rz = xsub(src.z, T.z);
-            const double s2 = xadd(xlen2(rx, ry, rz), eps2);
-            const double sc = xdiv(xmul(T.w, src.w), xmul(s2, xsqrt(s2)));
-            ax = xmul(rx, sc);
-            ay = xmul(ry, sc);
-            az = xmul(rz, sc);
-          }
-          term[b][0][t][jj] = ax;
-          term[b][1][t][jj] = ay;
-          term[b][2][t][jj] = az;
+          rx[u] = xsub(src.x, T.x), ry[u] = xsub(src.y, T.y), rz[u] = xsub(src.z, T.z);
+          wt[u] = pair_weight<kFast>(xmul(T.w, src.w), xadd(xlen2(rx[u], ry[u], rz[u]), eps2));
+          if (j >= n || j == i0 + t) wt[u] = 0.0;
         }
-        src = next;
+#pragma unroll
+        for (int u = 0; u < kXGroup; ++u) {
+          term[p][tg + u][lane] = xmul(rx[u], wt[u]);
+          term[p][kXT + tg + u][lane] = xmul(ry[u], wt[u]);
+          term[p][2 * kXT + tg + u][lane] = xmul(rz[u], wt[u]);
+        }
       }
-    } else if (k > 0 && tid < kXT) {
-      const int pb = b ^ 1;
-      const int64_t jb = (k - 1) * kXJ;
-      const int cnt = (int)min64(kXJ, n - jb);
-      // j == i sits at slot self, if in [0, cnt): the slots before and after
-      // it as two straight runs, so that the loads run ahead of the adds
-      const int64_t self = i0 + tid - jb;
-      const int q1 = (int)(self < 0 ? 0 : self < cnt ? self : cnt);
-      const int q2 = self >= 0 && self < cnt ? q1 + 1 : q1;
-      const double* tx = term[pb][0][tid];
-      const double* ty = term[pb][1][tid];
-      const double* tz = term[pb][2][tid];
-#pragma unroll 16
-      for (int q = 0; q < q1; ++q) {
-        fx = xadd(fx, tx[q]);
-        fy = xadd(fy, ty[q]);
-        fz = xadd(fz, tz[q]);
+      if (kFast && !(targets_ok && scale_pos_ok(src.x, src.y, src.z) && scale_mass_ok(src.w))) {
+        for (int t = 0; t < kXT; ++t) {  // out of range: this lane's terms again
+          const double4 T = tgt[t];
+          if (j >= n || j == i0 + t) continue;
+          const double rx = xsub(src.x, T.x), ry = xsub(src.y, T.y), rz = xsub(src.z, T.z);
+          const double wt = exact_scale_ieee(xmul(T.w, src.w), xadd(xlen2(rx, ry, rz), eps2));
+          term[p][t][lane] = xmul(rx, wt);
+          term[p][kXT + t][lane] = xmul(ry, wt);
+          term[p][2 * kXT + t][lane] = xmul(rz, wt);
+        }
       }
-#pragma unroll 16
-      for (int q = q2; q < cnt; ++q) {
-        fx = xadd(fx, tx[q]);
-        fy = xadd(fy, ty[q]);
-        fz = xadd(fz, tz[q]);
-      }
+      __syncwarp();
+      pair_arrive(1 + p);
     }
-    asm volatile("bar.sync 1, 288;" ::: "memory");  // kXWorking
+    return;
   }
-  if (tid >= 32) return;
-  const int64_t i = i0 + tid;
-  const bool valid = tid < kXT && i < t1;
+  const int row = lane < kXRows ? lane : 0;
+  double f = 0.0, cur[32];
+  pair_sync(1);
+#pragma unroll
+  for (int q = 0; q < 32; ++q) cur[q] = term[0][row][q];
+  if (kProd < chunks) pair_arrive(1 + kProd);
+  for (int k = 1, p = 1; k < chunks; ++k) {
+    double nxt[32];
+    pair_sync(1 + p);
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      nxt[q] = term[p][row][q];
+      f = xadd(f, cur[q]);
+    }
+    if (k + kProd < chunks) pair_arrive(1 + kProd + p);
+#pragma unroll
+    for (int q = 0; q < 32; ++q) cur[q] = nxt[q];
+    p = p + 1 == kProd ? 0 : p + 1;
+  }
+#pragma unroll
+  for (int q = 0; q < 32; ++q) f = xadd(f, cur[q]);
+
+  const int c = row / kXT;
+  const int64_t i = i0 + row % kXT;
+  const bool valid = lane < kXRows && i < t1;
+  bool bad = false;
   if (valid) {
-    if (!want_force) {  // compute_acceleration_system: a = F / m (integrators.rs:115)
-      const double mi = m[i];
-      fx = xdiv(fx, mi);
-      fy = xdiv(fy, mi);
-      fz = xdiv(fz, mi);
+    // compute_acceleration_system: a = F / m (integrators.rs:115)
+    if (kTick || !want_force) f = xdiv(f, m[i]);
+    (c == 0 ? ox : c == 1 ? oy : oz)[i] = f;
+    bad = !isfinite(f);
+    if (kTick) {  // kick_drift_kernel's operations on this component
+      double* v = c == 0 ? tick.vx : c == 1 ? tick.vy : tick.vz;
+      double* pa = c == 0 ? tick.pax : c == 1 ? tick.pay : tick.paz;
+      const double* xo = c == 0 ? x : c == 1 ? y : z;
+      const double hdt = xmul(0.5, tick.dt), h2 = xmul(xmul(0.5, tick.dt), tick.dt);
+      const double v1 = xadd(v[i], xmul(xadd(pa[i], f), hdt));
+      const double x1 = xadd(xo[i], xadd(xmul(v1, tick.dt), xmul(f, h2)));
+      v[i] = v1;
+      pa[i] = f;
+      (c == 0 ? tick.nx : c == 1 ? tick.ny : tick.nz)[i] = x1;
+      bad |= !isfinite(v1) || !isfinite(x1);
     }
-    ox[i] = fx;
-    oy[i] = fy;
-    oz[i] = fz;
   }
-  bool bad = valid && (!isfinite(fx) || !isfinite(fy) || !isfinite(fz));
-  if (__any_sync(0xffffffffu, bad) && tid == 0) atomicOr(status, kStatNonfinite);
+  if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(status, kStatNonfinite);
+}
+
+template <bool kTick>
+int launch_exact(phys_ctx* c, const phys_params* p, int64_t t0, int64_t t1, const double* x,
+                 const double* y, const double* z, int want_force, double* ox, double* oy,
+                 double* oz, const TickArgs& tick) {
+  const bool solo = t1 - t0 <= 148 * x_targets(6);  // each block has an SM to itself
+  const int64_t blocks = ceil_div(t1 - t0, solo ? x_targets(6) : x_targets(4));
+  const double eps2 = p->eps * p->eps;
+  const bool fast = scale_eps2_ok(eps2);
+  auto kernel = solo ? (fast ? direct_exact_kernel<6, kTick, true>
+                             : direct_exact_kernel<6, kTick, false>)
+                     : (fast ? direct_exact_kernel<4, kTick, true>
+                             : direct_exact_kernel<4, kTick, false>);
+  PHYS_LAUNCH(c, kernel, (int)blocks, solo ? x_block(6) : x_block(4), 0, c->n, t0, t1, x, y, z,
+              c->m, p->G, eps2, want_force, ox, oy, oz, tick, c->d_status);
+  return PHYS_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -428,7 +496,6 @@ int direct_eval(phys_ctx* c, const phys_params* p, bool want_force, double* ox, 
                 double* oz) {
   const int64_t n = c->n;
   const double eps2 = p->eps * p->eps;
-  PHYS_CUDA(c, cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned long long), c->stream));
   if (!c->capturing) PHYS_CUDA(c, cudaEventRecord(c->ev[6], c->stream));
   // targets [t0, t1): all, or the share (t0 a multiple of kTile); the slices
   // follow from n alone, so a target's sum does not depend on the share
@@ -442,8 +509,8 @@ int direct_eval(phys_ctx* c, const phys_params* p, bool want_force, double* ox, 
     return PHYS_OK;
   }
   if (p->precision == PHYS_F64_EXACT) {
-    PHYS_LAUNCH(c, direct_exact_kernel, (int)ceil_div(nt, kXT), kXBlock, 0, n, t0, t1, c->x, c->y,
-                c->z, c->m, p->G, eps2, (int)want_force, ox, oy, oz, c->d_status);
+    PHYS_TRY(launch_exact<false>(c, p, t0, t1, c->x, c->y, c->z, (int)want_force, ox, oy, oz,
+                                 TickArgs{}));
   } else {
     const int64_t slices = choose_slices(n);
     const int64_t slice_len = ceil_div(ceil_div(n, slices), kTile) * kTile;
@@ -481,6 +548,18 @@ int direct_eval(phys_ctx* c, const phys_params* p, bool want_force, double* ox, 
   c->tm.nodes = 0;
   c->tm.max_depth = 0;
   return PHYS_OK;
+}
+
+// The force pass of an F64_EXACT tick fused with its velocity step and the
+// next position step: positions from x/y/z into the force scratch arrays
+// (to_scratch) or back, so a run takes these in pairs.
+int direct_exact_tick(phys_ctx* c, const phys_params* p, double dt, bool to_scratch) {
+  double *from[3] = {c->x, c->y, c->z}, *to[3] = {c->fx, c->fy, c->fz};
+  if (!to_scratch)
+    for (int k = 0; k < 3; ++k) std::swap(from[k], to[k]);
+  const TickArgs tick{dt, c->vx, c->vy, c->vz, c->pax, c->pay, c->paz, to[0], to[1], to[2]};
+  return launch_exact<true>(c, p, 0, c->n, from[0], from[1], from[2], 0, c->ax, c->ay, c->az,
+                            tick);
 }
 
 // Sliced F64 / F32C direct sum on caller-owned device buffers and stream,

@@ -10,7 +10,7 @@ import pytest
 
 import oracle
 import physgpu.ics as ics
-from physgpu import BARNES_HUT, DIRECT, F64, GROUP_WALK, make_params
+from physgpu import BARNES_HUT, DIRECT, F64, F64_EXACT, GROUP_WALK, make_params
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +57,36 @@ def test_f64_group_layouts(ctx, n):
     f = ctx.gravity_forces(make_params(1.0, 0.01, 0.0, BARNES_HUT, F64, 1, GROUP_WALK))
     assert ctx.timings()["interactions"] == (n + 70) * (n + 69)
     assert rel_err(f, oracle.direct_forces(pos, m, 1.0, 0.01)).max() < 1e-12
+
+
+@pytest.mark.parametrize("n", [2, 7, 8, 9, 33, 1183, 1184, 1185, 1301])
+@pytest.mark.parametrize("eps", [0.0, 0.01])
+def test_exact_direct_blocks_and_ranges(ctx, n, eps):
+    """Bit-identical at the edges of the target blocks (8 targets up to 1184
+    bodies, 10 beyond), with sources and targets whose masses or coordinates
+    leave the range of the branch-free weight, massless bodies, and without
+    softening."""
+    pos, _, m = ics.plummer(n, seed=n)
+    m[::5] *= 1e-120
+    m[1::7] = 0.0
+    pos[n // 2] *= 1e35
+    if n > 30:
+        pos[3] *= 1e-40 if eps else 1.0
+        m[17] *= 1e200
+    ctx.upload(pos, None, m)
+    f = ctx.gravity_forces(make_params(1.0, eps, method=DIRECT, precision=F64_EXACT))
+    assert np.array_equal(f, oracle.direct_forces(pos, m, 1.0, eps))
+
+
+@pytest.mark.parametrize("steps", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("n", [9, 130, 1190])
+def test_exact_fused_ticks(ctx, n, steps):
+    """Runs of ticks with one kernel per pair-wise tick equal the reference's
+    tick loop bit for bit whatever the number of ticks, state and all."""
+    pos, vel, m = ics.plummer(n, seed=n + 1)
+    ctx.upload(pos, vel, m)
+    p = make_params(1.0, 0.05, method=DIRECT, precision=F64_EXACT)
+    ctx.verlet_steps(p, 1e-3, steps)
+    x, v, a = ctx.download()
+    xr, vr, ar = oracle.vv_run(pos, vel, m, 1.0, 0.05, 1e-3, steps)[:3]
+    assert np.array_equal(x, xr) and np.array_equal(v, vr) and np.array_equal(a, ar)
