@@ -37,6 +37,7 @@ int grid_for(int64_t n) { return (int)std::min<int64_t>(std::max<int64_t>(ceil_d
 // x += v dt + a dt^2/2 ; per component arrays of n.
 __global__ void adj_drift(int64_t n, double dt, double* __restrict__ x,
                           const double* __restrict__ v, const double* __restrict__ a) {
+  wait_for_previous();
   const double h2 = xmul(xmul(0.5, dt), dt);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * n;
        i += (int64_t)gridDim.x * blockDim.x)
@@ -46,6 +47,7 @@ __global__ void adj_drift(int64_t n, double dt, double* __restrict__ x,
 // v += (a_old + a_new) dt/2
 __global__ void adj_kick(int64_t n, double dt, double* __restrict__ v,
                          const double* __restrict__ a0, const double* __restrict__ a1) {
+  wait_for_previous();
   const double hdt = xmul(0.5, dt);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * n;
        i += (int64_t)gridDim.x * blockDim.x)
@@ -56,6 +58,7 @@ __global__ void adj_kick(int64_t n, double dt, double* __restrict__ v,
 __global__ void loss_kernel(int64_t n, const double* __restrict__ x,
                             const double* __restrict__ t, double* __restrict__ xbar,
                             double* __restrict__ part) {
+  wait_for_previous();
   __shared__ double sh[kBlock];
   double s = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * n;
@@ -74,6 +77,7 @@ __global__ void loss_kernel(int64_t n, const double* __restrict__ x,
 }
 
 __global__ void sum_kernel(int nparts, const double* __restrict__ part, double* __restrict__ out) {
+  wait_for_previous();
   if (threadIdx.x != 0) return;
   double s = 0.0;
   for (int b = 0; b < nparts; ++b) s += part[b];
@@ -83,6 +87,7 @@ __global__ void sum_kernel(int nparts, const double* __restrict__ part, double* 
 // abar += h * vbar
 __global__ void adj_pre(int64_t n, double h, double* __restrict__ abar,
                         const double* __restrict__ vbar) {
+  wait_for_previous();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * n;
        i += (int64_t)gridDim.x * blockDim.x)
     abar[i] = fma(h, vbar[i], abar[i]);
@@ -91,6 +96,7 @@ __global__ void adj_pre(int64_t n, double h, double* __restrict__ abar,
 // abar = h vbar + h2 xbar ; vbar += dt xbar
 __global__ void adj_post(int64_t n, double dt, double* __restrict__ abar,
                          double* __restrict__ vbar, const double* __restrict__ xbar) {
+  wait_for_previous();
   const double h = 0.5 * dt, h2 = 0.5 * dt * dt;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -108,6 +114,7 @@ vjp_kernel(int64_t n, int64_t slice_len, const double* __restrict__ x,
            const double* __restrict__ m, const double* __restrict__ wx,
            const double* __restrict__ wy, const double* __restrict__ wz, double eps2,
            double* __restrict__ part) {
+  wait_for_previous();
   __shared__ double4 ts[kTile];
   __shared__ double4 tw[kTile];
   const int64_t j = blockIdx.x * (int64_t)kTile + threadIdx.x;
@@ -163,6 +170,7 @@ vjp_kernel(int64_t n, int64_t slice_len, const double* __restrict__ x,
 // thread per (target, component), its slices' loads in flight together.
 __global__ void vjp_reduce(int64_t n, int nsl, const double* __restrict__ part, double G,
                            double* __restrict__ xbar, double* __restrict__ mbar) {
+  wait_for_previous();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 4 * n;
        e += (int64_t)gridDim.x * blockDim.x) {
     const int k = (int)(e / n);

@@ -249,9 +249,33 @@ int probe_peaks(phys_ctx* c, double* fp32, double* fp32x2, double* fp64);
 int debug_divide(phys_ctx* c, int64_t n, const double* a, const double* b, double* q);
 }  // namespace phys
 
+// Every kernel is launched with programmatic stream serialization and calls
+// wait_for_previous() before anything else: its blocks are set up while the
+// kernel before it drains, and start once that kernel has finished and its
+// writes are visible.  Back-to-back small kernels otherwise start in steps of
+// about 2 us on a B200 (a kernel of 2.9 us takes 4.2 us of the stream, 3.1 us
+// this way; one of 7.5 us 10.3 against 7.6).
+namespace phys {
+template <class... KArgs, class... Args>
+cudaError_t launch_kernel(cudaStream_t s, dim3 grid, dim3 block, size_t smem,
+                          void (*kernel)(KArgs...), Args&&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+}  // namespace phys
+
 #define PHYS_LAUNCH_ON(c, strm, kernel, grid, block, smem, ...)            \
   do {                                                                     \
-    kernel<<<(grid), (block), (smem), (strm)>>>(__VA_ARGS__);              \
+    phys::launch_kernel((strm), (grid), (block), (smem), kernel, __VA_ARGS__); \
     (c)->launches++;                                                       \
     int _st = phys::check_launch((c), #kernel);                            \
     if (_st) return _st;                                                   \
@@ -274,6 +298,11 @@ int debug_divide(phys_ctx* c, int64_t n, const double* a, const double* b, doubl
 
 // ---- device helpers ----
 namespace phys {
+
+// The kernel before this one on the stream has finished (see launch_kernel).
+__device__ __forceinline__ void wait_for_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // IEEE double ops that the compiler may not contract into FMAs: the
 // reference's Rust arithmetic rounds every + and * separately.

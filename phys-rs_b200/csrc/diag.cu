@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(kBlock)
 ke_mom_kernel(int64_t n, const double* __restrict__ vx, const double* __restrict__ vy,
               const double* __restrict__ vz, const double* __restrict__ m,
               double* __restrict__ part) {
+  wait_for_previous();
   __shared__ double sh[4][kBlock];
   CSum ke, px, py, pz;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -58,6 +59,7 @@ __global__ void __launch_bounds__(kTile)
 pe_kernel(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
           const double* __restrict__ z, const double* __restrict__ m, double G,
           double* __restrict__ part) {
+  wait_for_previous();
   __shared__ double4 tile[kTile];
   __shared__ double red[kTile];
   const int64_t i = blockIdx.x * (int64_t)kTile + threadIdx.x;
@@ -91,6 +93,7 @@ pe_kernel(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
 
 __global__ void final_kernel(int nke, int npe, const double* __restrict__ ke_part,
                              const double* __restrict__ pe_part, double* __restrict__ out) {
+  wait_for_previous();
   if (threadIdx.x != 0) return;
   CSum ke, px, py, pz, pe;
   for (int b = 0; b < nke; ++b) {
@@ -109,6 +112,7 @@ __global__ void final_kernel(int nke, int npe, const double* __restrict__ ke_par
 
 // FMA-rate probes: 8 independent chains per thread.
 __global__ void ffma_probe(int iters, float seed, float* out) {
+  wait_for_previous();
   float a[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) a[k] = seed + k * 1e-3f + threadIdx.x * 1e-7f;
@@ -124,6 +128,7 @@ __global__ void ffma_probe(int iters, float seed, float* out) {
 }
 
 __global__ void ffma2_probe(int iters, float seed, float* out) {
+  wait_for_previous();
   float2 a[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) a[k] = make_float2(seed + k * 1e-3f, seed - k * 1e-3f + threadIdx.x * 1e-7f);
@@ -139,6 +144,7 @@ __global__ void ffma2_probe(int iters, float seed, float* out) {
 }
 
 __global__ void dfma_probe(int iters, double seed, double* out) {
+  wait_for_previous();
   double a[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) a[k] = seed + k * 1e-3 + threadIdx.x * 1e-9;

@@ -78,6 +78,7 @@ direct_exact_kernel(int64_t n, int64_t t0, int64_t t1, const double* __restrict_
                     const double* __restrict__ m, double G, double eps2, int want_force,
                     double* __restrict__ ox, double* __restrict__ oy, double* __restrict__ oz,
                     TickArgs tick, int32_t* status) {
+  wait_for_previous();
   constexpr int kXT = x_targets(kProd), kXGroup = kXT / 2;
   constexpr int kXRows = 3 * kXT;  // ordered sums per block, one per lane
   static_assert(kXRows <= 32, "one adding warp");
@@ -241,6 +242,7 @@ direct_f64_kernel(int64_t n, int64_t t0, int64_t t1, int64_t slice_len,
                   const double* __restrict__ z, const double* __restrict__ m, double G,
                   double eps2, int want_force, double* __restrict__ ox, double* __restrict__ oy,
                   double* __restrict__ oz, double* __restrict__ part, int32_t* status) {
+  wait_for_previous();
   __shared__ double4 tile[kTile];
   const int64_t tbase = t0 + blockIdx.x * (int64_t)kTile;  // t0: a multiple of kTile
   const int64_t i = tbase + threadIdx.x;
@@ -286,6 +288,7 @@ __global__ void split_bodies_kernel(int64_t n, const double* __restrict__ x,
                                     const double* __restrict__ y, const double* __restrict__ z,
                                     const double* __restrict__ m, float4* __restrict__ bh,
                                     float4* __restrict__ bl, int32_t* status) {
+  wait_for_previous();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     float4 h, l;
@@ -334,6 +337,7 @@ direct_f32c_kernel(int64_t n, int64_t t0, int64_t t1, int64_t slice_len,
                    const double* __restrict__ m, double G, float eps2, int want_force,
                    double* __restrict__ ox, double* __restrict__ oy, double* __restrict__ oz,
                    double* __restrict__ part, int32_t* status) {
+  wait_for_previous();
   __shared__ float4 th[kTile];
   __shared__ float4 tl[kTile];
   const int64_t tbase = t0 + blockIdx.x * (int64_t)kTile;  // t0: a multiple of kTile
@@ -399,6 +403,7 @@ __global__ void slice_reduce_kernel(int64_t n, int64_t t0, int64_t t1, int nslic
                                     const double* __restrict__ m, double G, int want_force,
                                     double* __restrict__ ox, double* __restrict__ oy,
                                     double* __restrict__ oz, int32_t* status) {
+  wait_for_previous();
   const int64_t nt = t1 - t0;
   bool bad = false;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 3 * nt;
@@ -423,6 +428,7 @@ direct_targets_kernel(int64_t n, int64_t nt, const int64_t* __restrict__ tidx, i
                       const double* __restrict__ z, const double* __restrict__ m, double G,
                       double eps2, int exact, double* __restrict__ part, double* __restrict__ ox,
                       double* __restrict__ oy, double* __restrict__ oz, int32_t* status) {
+  wait_for_previous();
   __shared__ double4 tile[kTile];
   const int64_t t = blockIdx.x * (int64_t)kTile + threadIdx.x;
   const bool valid = t < nt;
@@ -578,16 +584,16 @@ cudaError_t direct_accel_launch_scratch(cudaStream_t s, int64_t n, const double*
   dim3 grid((unsigned)ceil_div(n, kTile), (unsigned)nsl);
   const int g = (int)min64(ceil_div(n, 256), 148 * 8);
   if (precision == PHYS_F64) {
-    direct_f64_kernel<<<grid, kTile, 0, s>>>(n, 0, n, slice_len, x, y, z, m, G, eps2, 0, ox, oy,
-                                             oz, part, status);
+    launch_kernel(s, grid, kTile, 0, direct_f64_kernel, n, 0, n, slice_len, x, y, z, m, G, eps2,
+                  0, ox, oy, oz, part, status);
   } else {
-    split_bodies_kernel<<<g, 256, 0, s>>>(n, x, y, z, m, bh, bl, status);
-    direct_f32c_kernel<<<grid, kTile, 0, s>>>(n, 0, n, slice_len, bh, bl, m, G, (float)eps2, 0,
-                                              ox, oy, oz, part, status);
+    launch_kernel(s, g, 256, 0, split_bodies_kernel, n, x, y, z, m, bh, bl, status);
+    launch_kernel(s, grid, kTile, 0, direct_f32c_kernel, n, 0, n, slice_len, bh, bl, m, G, eps2,
+                  0, ox, oy, oz, part, status);
   }
   if (nsl > 1)
-    slice_reduce_kernel<<<(int)min64(ceil_div(3 * n, 256), 148 * 8), 256, 0, s>>>(
-        n, 0, n, (int)nsl, part, m, G, 0, ox, oy, oz, status);
+    launch_kernel(s, (int)min64(ceil_div(3 * n, 256), 148 * 8), 256, 0, slice_reduce_kernel, n,
+                  0, n, nsl, part, m, G, 0, ox, oy, oz, status);
   return cudaGetLastError();  // the launch error, if any (and clears it)
 }
 

@@ -441,6 +441,7 @@ __device__ void drain(S_t* S, const EnsArgs& a, int lo, int hi, int* ctr, int ma
 template <int G, int BW, bool kExact>
 __global__ void __launch_bounds__(32 * BW)
 ensemble_kernel(EnsArgs a) {
+  wait_for_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if constexpr (G != 0) {
@@ -553,7 +554,7 @@ int enqueue_run(phys_ctx* c, const phys_params* p, const LaunchCfg& cfg, double 
     a.nsteps = (int)k_steps;
     a.need_accel = need ? 1 : 0;
     PHYS_CUDA(c, cudaMemsetAsync(a.queue, 0, 4 * sizeof(int), c->stream));
-    cfg.k<<<(unsigned)cfg.grid, cfg.block, cfg.smem, c->stream>>>(a);
+    launch_kernel(c->stream, (unsigned)cfg.grid, cfg.block, cfg.smem, cfg.k, a);
     c->launches++;
     PHYS_TRY(check_launch(c, "ensemble_kernel"));
     need = false;

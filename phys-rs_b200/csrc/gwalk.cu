@@ -958,6 +958,7 @@ glist_kernel(int n, int q0, int q1, int nnodes, const GNode* __restrict__ gn,
              int64_t pool_per_warp, int64_t nspill, int32_t* __restrict__ spill_ctr,
              int4* __restrict__ items, int32_t* __restrict__ nitems, int2* __restrict__ retry,
              int32_t* __restrict__ nretry, int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;  // records built on an unfinished sort
   extern __shared__ __align__(16) unsigned char gsm[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1050,6 +1051,7 @@ geval_kernel(int n, const GNode* __restrict__ gn, const int4* __restrict__ items
              const uint32_t* __restrict__ perm, double G, double eps2, int want_force,
              double* __restrict__ ox, double* __restrict__ oy, double* __restrict__ oz,
              unsigned long long* counter, int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;  // records built on an unfinished sort
   extern __shared__ __align__(16) unsigned char gsm[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1090,6 +1092,7 @@ gwalk_kernel(int n, int nnodes, const GNode* __restrict__ gn, const int2* __rest
              double eps2, float theta2f, int want_force, double* __restrict__ ox,
              double* __restrict__ oy, double* __restrict__ oz, unsigned long long* counter,
              int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;  // records built on an unfinished sort
   extern __shared__ __align__(16) unsigned char gsm[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;

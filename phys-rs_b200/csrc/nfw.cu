@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(kBlock)
 nfw_force_kernel(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
                  const double* __restrict__ z, const double* __restrict__ m, Halo h,
                  double* __restrict__ fx, double* __restrict__ fy, double* __restrict__ fz) {
+  wait_for_previous();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     double f0, f1, f2;
@@ -66,6 +67,7 @@ nfw_accel_kernel(int64_t n, const double* __restrict__ x, const double* __restri
                  const double* __restrict__ fx, const double* __restrict__ fy,
                  const double* __restrict__ fz, double* __restrict__ ax, double* __restrict__ ay,
                  double* __restrict__ az, int32_t* status) {
+  wait_for_previous();
   bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {

@@ -27,6 +27,7 @@ flatten_from_kernel(int64_t n, const int64_t* __restrict__ sx, const int64_t* __
                     const double* __restrict__ ly, const double* __restrict__ lz, double ss,
                     int bh_quirk, double* __restrict__ x, double* __restrict__ y,
                     double* __restrict__ z) {
+  wait_for_previous();
   const int64_t ox = sx[0], oy = sy[0], oz = sz[0];
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(kBlock)
 normalize_kernel(int64_t n, int64_t* __restrict__ sx, int64_t* __restrict__ sy,
                  int64_t* __restrict__ sz, double* __restrict__ lx, double* __restrict__ ly,
                  double* __restrict__ lz, double ss, int32_t* __restrict__ shifted) {
+  wait_for_previous();
   bool any = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {

@@ -27,6 +27,7 @@ __global__ void share_pack_kernel(int64_t lo, int64_t hi, int64_t chunk,
                                   const uint32_t* __restrict__ perm, const double* __restrict__ ax,
                                   const double* __restrict__ ay, const double* __restrict__ az,
                                   double* __restrict__ out) {
+  wait_for_previous();
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < chunk;
        j += (int64_t)gridDim.x * blockDim.x) {
     const int64_t q = lo + j;
@@ -48,6 +49,7 @@ __global__ void share_unpack_kernel(int64_t n, int64_t chunk, const uint32_t* __
                                     const double* __restrict__ g, double* __restrict__ ax,
                                     double* __restrict__ ay, double* __restrict__ az,
                                     int32_t* status) {
+  wait_for_previous();
   bool bad = false;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
        q += (int64_t)gridDim.x * blockDim.x) {

@@ -57,6 +57,7 @@ constexpr int kDigitsSmem = (kDigitsThreads / 32) * kMaxPasses * kBins * 4;
 __global__ void __launch_bounds__(kDigitsThreads)
 radix_digits_kernel(const uint64_t* __restrict__ keys, int64_t n, int begin_bit, int npass,
                     uint32_t* __restrict__ ghist) {
+  wait_for_previous();
   extern __shared__ __align__(16) unsigned char dsm[];
   uint32_t* cnt = reinterpret_cast<uint32_t*>(dsm);  // [warp][pass][digit]
   const int warp = threadIdx.x >> 5;
@@ -82,6 +83,7 @@ radix_digits_kernel(const uint64_t* __restrict__ keys, int64_t n, int begin_bit,
 // Exclusive scan of `count` u32 values in one block (in place allowed).
 __global__ void __launch_bounds__(1024)
 scan_single_kernel(const uint32_t* in, uint32_t* out, int64_t count, uint32_t* total) {
+  wait_for_previous();
   __shared__ uint32_t wsum[32];
   __shared__ uint32_t carry_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -151,6 +153,7 @@ radix_pass_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restrict__
                   uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n, int shift,
                   const uint32_t* __restrict__ counts, uint32_t* __restrict__ status,
                   int32_t* __restrict__ tile_ctr, int32_t* __restrict__ err, int64_t spin_limit) {
+  wait_for_previous();
   extern __shared__ __align__(16) unsigned char ssm[];
   uint64_t* skey = reinterpret_cast<uint64_t*>(ssm);                          // kTileKeys
   uint32_t* sval = reinterpret_cast<uint32_t*>(ssm + kTileKeys * 8);          // kTileKeys
@@ -332,6 +335,7 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t s, uint32_t* wsum, 
 
 __global__ void __launch_bounds__(kScanBlock)
 scan_block_sums_kernel(const int32_t* __restrict__ in, int64_t n, uint32_t* __restrict__ sums) {
+  wait_for_previous();
   __shared__ uint32_t wsum[33];
   uint32_t s = 0;
 #pragma unroll
@@ -347,6 +351,7 @@ scan_block_sums_kernel(const int32_t* __restrict__ in, int64_t n, uint32_t* __re
 __global__ void __launch_bounds__(kScanBlock)
 scan_apply_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, int64_t n,
                   const uint32_t* __restrict__ offs) {
+  wait_for_previous();
   __shared__ uint32_t wsum[33];
   uint32_t v[kScanItems];
   uint32_t s = 0;

@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(kBlock)
 bbox_partial_kernel(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
                     const double* __restrict__ z, const double* __restrict__ m,
                     double* __restrict__ part, int32_t* status) {
+  wait_for_previous();
   __shared__ double sh[7][kBlock / 32];
   double v[7] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY, INFINITY};
   bool bad = false;
@@ -95,6 +96,7 @@ bbox_partial_kernel(int64_t n, const double* __restrict__ x, const double* __res
 // derives the cube and the per-depth constants.
 __global__ void bbox_final_kernel(int nparts, const double* __restrict__ part, double theta,
                                   TreeHeader* hdr, const int32_t* status) {
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   if (threadIdx.x >= 32) return;
   double mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -146,6 +148,7 @@ keys_kernel(int64_t n, const double* __restrict__ x, const double* __restrict__ 
             const double* __restrict__ z, const double* __restrict__ m,
             const TreeHeader* __restrict__ hdr, uint64_t* __restrict__ khi,
             uint64_t* __restrict__ klo, uint32_t* __restrict__ idx, double4* __restrict__ rec) {
+  wait_for_previous();
   const double c0 = hdr->center[0], c1 = hdr->center[1], c2 = hdr->center[2];
   const double h0 = hdr->half;
   const int D = hdr->dstar;
@@ -184,6 +187,7 @@ __device__ __forceinline__ bool key_less(const uint64_t* klo, uint32_t a, uint32
 __global__ void run_fixup_kernel(int64_t n, const uint64_t* __restrict__ hs,
                                  uint32_t* __restrict__ perm, const uint64_t* __restrict__ klo,
                                  uint32_t* __restrict__ tmp, const int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p + 1 < n;
        p += (int64_t)gridDim.x * blockDim.x) {
@@ -231,6 +235,7 @@ gather_sorted_kernel(int64_t n, const uint32_t* __restrict__ perm, const uint64_
                      double4* __restrict__ body64,
                      float4* __restrict__ body_hi, float4* __restrict__ body_lo,
                      Body32x2* __restrict__ body2, const int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
        p += (int64_t)gridDim.x * blockDim.x) {
@@ -269,6 +274,7 @@ __global__ void __launch_bounds__(kBlock)
 lcp_count_kernel(int64_t n, const uint64_t* __restrict__ hs, const uint64_t* __restrict__ ls,
                  const TreeHeader* __restrict__ hdr, int32_t* __restrict__ L,
                  int32_t* __restrict__ cnt) {
+  wait_for_previous();
   const int D = hdr->dstar;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p <= n;
        p += (int64_t)gridDim.x * blockDim.x) {
@@ -341,6 +347,7 @@ emit_nodes_kernel(int64_t n, const uint64_t* __restrict__ hs, const uint64_t* __
                   const int32_t* __restrict__ L, const int32_t* __restrict__ cnt,
                   const int32_t* __restrict__ first, const TreeHeader* __restrict__ hdr,
                   int4* __restrict__ link) {
+  wait_for_previous();
   const int D = hdr->dstar;
   const int32_t total = first[n];
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
@@ -380,6 +387,7 @@ emit_nodes_kernel(int64_t n, const uint64_t* __restrict__ hs, const uint64_t* __
 __global__ void __launch_bounds__(kBlock)
 prune_count_kernel(int64_t n, const int32_t* __restrict__ L, const TreeHeader* __restrict__ hdr,
                    int C, int32_t* __restrict__ cnt, int32_t* __restrict__ emax) {
+  wait_for_previous();
   const int D = hdr->dstar;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p <= n;
        p += (int64_t)gridDim.x * blockDim.x) {
@@ -415,6 +423,7 @@ emit_pruned_kernel(int64_t n, const uint64_t* __restrict__ hs, const uint64_t* _
                    const int32_t* __restrict__ L, const int32_t* __restrict__ cnt,
                    const int32_t* __restrict__ first, const TreeHeader* __restrict__ hdr,
                    int4* __restrict__ link) {
+  wait_for_previous();
   const int D = hdr->dstar;
   const int32_t total = first[n];
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
@@ -450,6 +459,7 @@ emit_pruned_kernel(int64_t n, const uint64_t* __restrict__ hs, const uint64_t* _
 __global__ void __launch_bounds__(kBlock)
 children_kernel(int64_t nnodes, const int4* __restrict__ link, int32_t* __restrict__ parent,
                 int32_t* __restrict__ nchild, int32_t* status) {
+  wait_for_previous();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnodes;
        k += (int64_t)gridDim.x * blockDim.x) {
     const int4 lk = link[k];
@@ -490,6 +500,7 @@ com_upward_kernel(int64_t nnodes, const int4* __restrict__ link,
                   const int32_t* __restrict__ parent, const int32_t* __restrict__ nchild,
                   int32_t* __restrict__ arrive, const double4* __restrict__ body64,
                   double4* __restrict__ sums, int32_t* status) {
+  wait_for_previous();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnodes;
        k += (int64_t)gridDim.x * blockDim.x) {
     const int4 lk = link[k];
@@ -538,6 +549,7 @@ com_upward_kernel(int64_t nnodes, const int4* __restrict__ link,
 // ---------------------------------------------------------------------------
 __global__ void node_count_kernel(int64_t nnodes, const int4* __restrict__ link,
                                   int32_t* __restrict__ cnt) {
+  wait_for_previous();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k <= nnodes;
        k += (int64_t)gridDim.x * blockDim.x)
     cnt[k] = k < nnodes ? link[k].z - link[k].y : 0;
@@ -547,6 +559,7 @@ __global__ void __launch_bounds__(kBlock)
 expand_kernel(int64_t total, int64_t nnodes, const int32_t* __restrict__ eoff,
               const int4* __restrict__ link, const uint32_t* __restrict__ perm,
               uint64_t* __restrict__ entries) {
+  wait_for_previous();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
     int64_t lo = 0, hi = nnodes;  // last k with eoff[k] <= e
@@ -588,6 +601,7 @@ gather_entries_kernel(int64_t total, const uint64_t* __restrict__ entries,
                       const double* __restrict__ z, const double* __restrict__ m,
                       const int4* __restrict__ link, const TreeHeader* __restrict__ hdr,
                       int skip_unused, double4* __restrict__ eb, const int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;
   const bool can_skip = skip_unused && hdr->min_mass > 0.0;
   const double bound = hdr->theta2 * 12.0 * hdr->half * hdr->half * (1.0 + 1e-6);
@@ -669,6 +683,7 @@ com_recurrence_kernel(int64_t nnodes, const int32_t* __restrict__ eoff,
                       const double4* __restrict__ eb, double4* __restrict__ mc,
                       const int4* __restrict__ link, const TreeHeader* __restrict__ hdr,
                       int skip_unused, int32_t* __restrict__ longs, const int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;
   // the bound holds when every centre of mass is a convex combination of
   // bodies (all masses positive)
@@ -810,6 +825,7 @@ __global__ void __launch_bounds__(32 * kLongWarps)
 com_recurrence_long_kernel(int64_t nnodes, const int32_t* __restrict__ eoff,
                            const double4* __restrict__ eb, double4* __restrict__ mc,
                            const int32_t* __restrict__ longs, const int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;
   __shared__ LongStage stage[kLongWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -831,6 +847,7 @@ com_recurrence_long_kernel(int64_t nnodes, const int32_t* __restrict__ eoff,
 __global__ void __launch_bounds__(kBlock)
 debug_divide_kernel(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
                     double* __restrict__ q) {
+  wait_for_previous();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const double x = a[i], d = b[i];
@@ -846,6 +863,7 @@ finalize_kernel(int64_t nnodes, int4* __restrict__ link, double4* __restrict__ m
                 int leaf_cap, const double4* __restrict__ body64, const TreeHeader* __restrict__ hdr,
                 double4* __restrict__ rec64, Rec32* __restrict__ w32, Rec64* __restrict__ w64,
                 Rec32x2* __restrict__ w32x2) {
+  wait_for_previous();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnodes;
        k += (int64_t)gridDim.x * blockDim.x) {
     int4 lk = link[k];
@@ -909,6 +927,7 @@ finalize_kernel(int64_t nnodes, int4* __restrict__ link, double4* __restrict__ m
 // pre-order input); inverse map.
 __global__ void depth_key_kernel(int64_t nnodes, const int4* __restrict__ link,
                                  uint64_t* __restrict__ key, uint32_t* __restrict__ val) {
+  wait_for_previous();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnodes;
        k += (int64_t)gridDim.x * blockDim.x) {
     key[k] = (uint64_t)(link[k].w & kMetaDepth);
@@ -918,6 +937,7 @@ __global__ void depth_key_kernel(int64_t nnodes, const int4* __restrict__ link,
 
 __global__ void invert_kernel(int64_t nnodes, const uint32_t* __restrict__ bfs2pre,
                               int32_t* __restrict__ pre2bfs, const int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nnodes;
        j += (int64_t)gridDim.x * blockDim.x)
@@ -930,6 +950,7 @@ gnode_kernel(int64_t nnodes, const uint32_t* __restrict__ bfs2pre,
              const double4* __restrict__ mc, const int32_t* __restrict__ nchild, int leaf_cap,
              const double4* __restrict__ body64, const TreeHeader* __restrict__ hdr,
              GNode* __restrict__ g, const int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nnodes;
        j += (int64_t)gridDim.x * blockDim.x) {
@@ -993,6 +1014,7 @@ __global__ void group_kernel(int64_t nnodes, const uint32_t* __restrict__ bfs2pr
                              const uint32_t* __restrict__ perm,
                              int32_t* __restrict__ cnt, const int32_t* __restrict__ off,
                              int2* __restrict__ out, int64_t cap, const int32_t* status) {
+  wait_for_previous();
   if (sort_failed(status)) return;
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j <= nnodes;
        j += (int64_t)gridDim.x * blockDim.x) {

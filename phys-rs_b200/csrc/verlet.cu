@@ -16,6 +16,7 @@ __global__ void drift_kernel(int64_t n, double dt, double* __restrict__ x, doubl
                              const double* __restrict__ ax, const double* __restrict__ ay,
                              const double* __restrict__ az, double* __restrict__ pax,
                              double* __restrict__ pay, double* __restrict__ paz) {
+  wait_for_previous();
   const double h2 = xmul(xmul(0.5, dt), dt);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -36,6 +37,7 @@ __global__ void kick_kernel(int64_t n, double dt, double* __restrict__ vx, doubl
                             const double* __restrict__ ay, const double* __restrict__ az,
                             const double* __restrict__ pax, const double* __restrict__ pay,
                             const double* __restrict__ paz, int32_t* status) {
+  wait_for_previous();
   const double hdt = xmul(0.5, dt);
   bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -61,6 +63,7 @@ __global__ void kick_drift_kernel(int64_t n, double dt, double* __restrict__ x,
                                   const double* __restrict__ ay, const double* __restrict__ az,
                                   double* __restrict__ pax, double* __restrict__ pay,
                                   double* __restrict__ paz, int32_t* status) {
+  wait_for_previous();
   const double hdt = xmul(0.5, dt);
   const double h2 = xmul(xmul(0.5, dt), dt);
   bool bad = false;
@@ -95,6 +98,7 @@ __global__ void flatten_kernel(int64_t n, const int64_t* __restrict__ sx,
                                const int64_t* __restrict__ sy, const int64_t* __restrict__ sz,
                                double* __restrict__ x, double* __restrict__ y,
                                double* __restrict__ z, double ss, int bh_quirk) {
+  wait_for_previous();
   const int64_t ox = sx[0], oy = sy[0], oz = sz[0];
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {

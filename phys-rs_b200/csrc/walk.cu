@@ -53,6 +53,7 @@ walk_kernel(int q0, int n, int nnodes, const Rec32* __restrict__ w32, const Rec6
             const TreeHeader* __restrict__ hdr, double G, double eps2, int want_force,
             double* __restrict__ ox, double* __restrict__ oy, double* __restrict__ oz,
             unsigned long long* counter, int32_t* status) {
+  wait_for_previous();
   __shared__ double s2d[kWDepth + 1];
   if (!kF32) {
     for (int d = threadIdx.x; d <= kWDepth; d += blockDim.x)
@@ -254,6 +255,7 @@ walk2_kernel(int q64, int n, int nnodes, const Rec32x2* __restrict__ w, const Bo
              const double4* __restrict__ body64, const uint32_t* __restrict__ perm, double G,
              double eps2, int want_force, double* __restrict__ ox, double* __restrict__ oy,
              double* __restrict__ oz, unsigned long long* counter, int32_t* status) {
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   // targets [64 q64, n), 64 per warp (a multiple of 64: pa even)
   const int base = (q64 + blockIdx.x * (kWalk2Block / 32) + (threadIdx.x >> 5)) * 64;
@@ -379,6 +381,7 @@ walk_exact_kernel(int64_t q0, int64_t n, int64_t nnodes, const int4* __restrict_
                   const uint32_t* __restrict__ perm, const TreeHeader* __restrict__ hdr, double G,
                   double eps2, int want_force, double* __restrict__ ox, double* __restrict__ oy,
                   double* __restrict__ oz, unsigned long long* counter, int32_t* status) {
+  wait_for_previous();
   __shared__ double s2d[kMaxLevels];
   for (int d = threadIdx.x; d < kMaxLevels; d += blockDim.x) s2d[d] = hdr->s2[d];
   __syncthreads();
