@@ -75,12 +75,32 @@ struct __align__(16) Rec64 {
   int4 l;
 };
 
+// Exact walk, traversal record: the node's position relative to the root
+// cube's centre in units of its half size (f32: decides almost every opening,
+// the f64 record the rest), the skip pointer (int bits in w), the depth and
+// flags of `link` and the stored body of a leaf.
+struct __align__(16) RecX {
+  float4 a;  // x, y, z, next
+  int4 b;    // meta, stored body (leaf), -, -
+};
+// The exact walk's split over subtrees: the cells of more than `most` bodies
+// (upper cells) and their other children (tasks), in pre-order.
+struct TopTree {
+  int max_tasks = 0, max_top = 0;    // room in the arrays
+  int32_t* counts = nullptr;         // tasks << 16 | top nodes
+  int32_t* task = nullptr;           // node of each task
+  int4* top = nullptr;               // node, task (-1: upper cell), depth, -
+  const int32_t* parent = nullptr;   // of every node
+};
+
 struct BhTree {
   int64_t n = 0;
   int64_t nnodes = 0;
   int leaf_cap = 1;
   const int4* link = nullptr;
   const double4* rec64 = nullptr;     // exact walk: record per node (with `link`)
+  const RecX* wx = nullptr;           // exact walk: traversal record per node
+  TopTree top;                        // exact walk split over subtrees (max_tasks > 0)
   const Rec32* w32 = nullptr;         // F32C walk records
   const Rec32x2* w32x2 = nullptr;     // F32C paired walk records
   const Body32x2* body2 = nullptr;    // sorted bodies, paired layout
@@ -106,6 +126,9 @@ struct BhTree {
 int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool need_group = false,
              bool full_com = true);
 // walk.cu
+// Tasks that the exact walk of this evaluation may be split into (0: one walk
+// per target).
+int exact_walk_tasks(const phys_ctx* c, int64_t n);
 int bh_group_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force,
                   double* ox, double* oy, double* oz);
 int bh_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force, double* ox,

@@ -39,6 +39,7 @@ struct TreeHeader {
   int32_t nonfinite;             // any non-finite input coordinate
   int64_t nnodes;                // nodes of the current tree
   double min_mass;               // smallest body mass
+  double min_abs, max_abs;       // smallest nonzero and largest |mass|
 };
 
 }  // namespace phys

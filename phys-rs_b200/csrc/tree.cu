@@ -39,6 +39,7 @@ int grid_for(int64_t n, int block = kBlock, int cap = 148 * 16) {
 // K2: bounding cube, gravity_tree.rs:305-317.
 // ---------------------------------------------------------------------------
 constexpr int kBboxGrid = 296;
+constexpr int kBboxVals = 9;  // reduced values per block
 
 __device__ __forceinline__ double warp_min(double v) {
 #pragma unroll
@@ -56,13 +57,18 @@ bbox_partial_kernel(int64_t n, const double* __restrict__ x, const double* __res
                     const double* __restrict__ z, const double* __restrict__ m,
                     double* __restrict__ part, int32_t* status) {
   wait_for_previous();
-  __shared__ double sh[7][kBlock / 32];
-  double v[7] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY, INFINITY};
+  // x, y, z minima and maxima, smallest mass, smallest nonzero |mass|,
+  // largest |mass|
+  __shared__ double sh[kBboxVals][kBlock / 32];
+  double v[kBboxVals] = {INFINITY,  INFINITY, INFINITY, -INFINITY, -INFINITY,
+                         -INFINITY, INFINITY, INFINITY, 0.0};
   bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const double a = x[i], b = y[i], cc = z[i], mm = m[i];
     v[6] = fmin(v[6], mm);
+    if (mm != 0.0) v[7] = fmin(v[7], fabs(mm));
+    v[8] = fmax(v[8], fabs(mm));
     v[0] = fmin(v[0], a);
     v[1] = fmin(v[1], b);
     v[2] = fmin(v[2], cc);
@@ -77,17 +83,19 @@ bbox_partial_kernel(int64_t n, const double* __restrict__ x, const double* __res
 #pragma unroll
   for (int k = 3; k < 6; ++k) v[k] = warp_max(v[k]);
   v[6] = warp_min(v[6]);
+  v[7] = warp_min(v[7]);
+  v[8] = warp_max(v[8]);
   if (lane == 0)
-    for (int k = 0; k < 7; ++k) sh[k][warp] = v[k];
+    for (int k = 0; k < kBboxVals; ++k) sh[k][warp] = v[k];
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(status, kStatNonfinite);
   __syncthreads();
   if (warp == 0) {
 #pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      const bool mn = k < 3 || k == 6;
+    for (int k = 0; k < kBboxVals; ++k) {
+      const bool mn = k < 3 || k == 6 || k == 7;
       double t = lane < kBlock / 32 ? sh[k][lane] : (mn ? INFINITY : -INFINITY);
       t = mn ? warp_min(t) : warp_max(t);
-      if (lane == 0) part[blockIdx.x * 7 + k] = t;
+      if (lane == 0) part[blockIdx.x * kBboxVals + k] = t;
     }
   }
 }
@@ -100,13 +108,16 @@ __global__ void bbox_final_kernel(int nparts, const double* __restrict__ part, d
   const int lane = threadIdx.x & 31;
   if (threadIdx.x >= 32) return;
   double mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-  double mmin = INFINITY;
+  double mmin = INFINITY, amin = INFINITY, amax = 0.0;
   for (int b = lane; b < nparts; b += 32) {
+    const double* q = part + b * kBboxVals;
     for (int k = 0; k < 3; ++k) {
-      mn[k] = fmin(mn[k], part[b * 7 + k]);
-      mx[k] = fmax(mx[k], part[b * 7 + 3 + k]);
+      mn[k] = fmin(mn[k], q[k]);
+      mx[k] = fmax(mx[k], q[3 + k]);
     }
-    mmin = fmin(mmin, part[b * 7 + 6]);
+    mmin = fmin(mmin, q[6]);
+    amin = fmin(amin, q[7]);
+    amax = fmax(amax, q[8]);
   }
   for (int o = 16; o > 0; o >>= 1) {
     for (int k = 0; k < 3; ++k) {
@@ -114,9 +125,13 @@ __global__ void bbox_final_kernel(int nparts, const double* __restrict__ part, d
       mx[k] = fmax(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
     }
     mmin = fmin(mmin, __shfl_xor_sync(0xffffffffu, mmin, o));
+    amin = fmin(amin, __shfl_xor_sync(0xffffffffu, amin, o));
+    amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   }
   if (lane != 0) return;
   hdr->min_mass = mmin;
+  hdr->min_abs = amin;
+  hdr->max_abs = amax;
   // extent = max - min; max_extent = x.max(y).max(z); half = max_extent*0.55 + 1
   const double ex = xsub(mx[0], mn[0]), ey = xsub(mx[1], mn[1]), ez = xsub(mx[2], mn[2]);
   const double max_extent = fmax(fmax(ex, ey), ez);
@@ -861,8 +876,8 @@ debug_divide_kernel(int64_t n, const double* __restrict__ a, const double* __res
 __global__ void __launch_bounds__(kBlock)
 finalize_kernel(int64_t nnodes, int4* __restrict__ link, double4* __restrict__ mc, int sums,
                 int leaf_cap, const double4* __restrict__ body64, const TreeHeader* __restrict__ hdr,
-                double4* __restrict__ rec64, Rec32* __restrict__ w32, Rec64* __restrict__ w64,
-                Rec32x2* __restrict__ w32x2) {
+                double4* __restrict__ rec64, RecX* __restrict__ wx, Rec32* __restrict__ w32,
+                Rec64* __restrict__ w64, Rec32x2* __restrict__ w32x2) {
   wait_for_previous();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnodes;
        k += (int64_t)gridDim.x * blockDim.x) {
@@ -891,6 +906,17 @@ finalize_kernel(int64_t nnodes, int4* __restrict__ link, double4* __restrict__ m
     }
     if (self >= 0) r = body64[self];
     if (rec64) rec64[k] = r;
+    if (wx) {
+      // the root's own position is left to the f64 test (it may be anything
+      // when the total mass is not positive)
+      const double ih = 1.0 / hdr->half;
+      RecX o;
+      o.a = make_float4((float)((r.x - hdr->center[0]) * ih), (float)((r.y - hdr->center[1]) * ih),
+                        (float)((r.z - hdr->center[2]) * ih), __int_as_float(lk.x));
+      if (k == 0) o.a.x = __int_as_float(0x7fc00000);
+      o.b = make_int4(lk.w, leaf ? (cntb == 1 ? lk.y : lk.z - 1) : -1, 0, 0);
+      wx[k] = o;
+    }
     int wmeta = (gate || k == 0) ? d : kWSkip;
     if (leaf && self < 0) wmeta |= kWLeaf | (cntb << 8);
     const int4 wl = make_int4(lk.x, self, lk.y, wmeta);
@@ -920,6 +946,35 @@ finalize_kernel(int64_t nnodes, int4* __restrict__ link, double4* __restrict__ m
         w32x2[k] = q;
       }
     }
+  }
+}
+
+// The exact walk's split over subtrees: a node is in the top tree when its
+// parent is an upper cell (or it is the root), and a task when it is not an
+// upper cell itself.  Pass 1 counts (tasks << 16 | top nodes), pass 2 writes
+// both lists from the scanned counts.
+template <bool kEmit>
+__global__ void __launch_bounds__(kBlock)
+top_tree_kernel(int64_t nnodes, const int4* __restrict__ link, const int32_t* __restrict__ parent,
+                int most, int32_t* __restrict__ cnt, const int32_t* __restrict__ off,
+                int max_tasks, int max_top, int32_t* __restrict__ task, int4* __restrict__ top) {
+  wait_for_previous();
+  auto upper = [&](int4 l) { return !(l.w & kMetaLeaf) && l.z - l.y > most; };
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k <= nnodes;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    int v = 0;
+    if (k < nnodes) {
+      const int4 l = link[k];
+      const bool in = k == 0 || upper(link[parent[k]]);
+      const bool is_task = in && !upper(l);
+      v = (is_task ? 1 << 16 : 0) | (in ? 1 : 0);
+      if (kEmit && in) {
+        const int ti = off[k] >> 16, pi = off[k] & 0xffff;
+        if (is_task && ti < max_tasks) task[ti] = (int)k;
+        if (pi < max_top) top[pi] = make_int4((int)k, is_task ? ti : -1, l.w & kMetaDepth, 0);
+      }
+    }
+    if (!kEmit) cnt[k] = v;
   }
 }
 
@@ -1099,11 +1154,11 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
   PHYS_TRY(ws_alloc(c, WS_NCOUNT, n + 1, &cnt));
   int32_t* first = nullptr;
   PHYS_TRY(ws_alloc(c, WS_NFIRST, n + 1, &first));
-  if (!c->d_partials || c->partials_cap < 7 * kBboxGrid) {
+  if (!c->d_partials || c->partials_cap < kBboxVals * kBboxGrid) {
     if (c->d_partials) cudaFree(c->d_partials);
     c->d_partials = nullptr;
-    PHYS_CUDA(c, cudaMalloc(&c->d_partials, sizeof(double) * 8 * kBboxGrid));
-    c->partials_cap = 8 * kBboxGrid;
+    PHYS_CUDA(c, cudaMalloc(&c->d_partials, sizeof(double) * kBboxVals * kBboxGrid));
+    c->partials_cap = kBboxVals * kBboxGrid;
   }
 
   PHYS_CUDA(c, cudaEventRecord(c->ev[2], c->stream));
@@ -1217,10 +1272,33 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
                 arrive, body64, mc, c->d_status);
   }
   double4* rec64 = nullptr;
+  RecX* wx = nullptr;
+  TopTree top;
   Rec32* w32 = nullptr;
   Rec64* w64 = nullptr;
   Rec32x2* w32x2 = nullptr;
-  if (exact) PHYS_TRY(ws_alloc(c, WS_NODE_PM, nnodes, &rec64));
+  if (exact) {
+    PHYS_TRY(ws_alloc(c, WS_NODE_PM, nnodes, &rec64));
+    top.max_tasks = exact_walk_tasks(c, n);
+    if (top.max_tasks > 0) {
+      PHYS_TRY(ws_alloc(c, WS_NODE_HI, nnodes, &wx));
+      int32_t *cnt2 = nullptr, *off2 = nullptr, *lists = nullptr;
+      top.max_top = 4096;
+      PHYS_TRY(ws_alloc(c, WS_NCOUNT, nnodes + 1, &cnt2));
+      PHYS_TRY(ws_alloc(c, WS_GROUP_OFF, nnodes + 1, &off2));
+      PHYS_TRY(ws_alloc(c, WS_GROUPS, 4 * top.max_top + top.max_tasks, &lists));
+      top.top = reinterpret_cast<int4*>(lists);
+      top.task = lists + 4 * top.max_top;
+      top.counts = off2 + nnodes;
+      top.parent = parent;
+      const int most = (int)(n / 8);
+      PHYS_LAUNCH(c, top_tree_kernel<false>, grid_for(nnodes + 1), kBlock, 0, nnodes, link, parent,
+                  most, cnt2, off2, top.max_tasks, top.max_top, top.task, top.top);
+      PHYS_TRY(scan_exclusive_i32(c, cnt2, off2, nnodes + 1));
+      PHYS_LAUNCH(c, top_tree_kernel<true>, grid_for(nnodes + 1), kBlock, 0, nnodes, link, parent,
+                  most, cnt2, off2, top.max_tasks, top.max_top, top.task, top.top);
+    }
+  }
 #ifndef WALK_PAIRED
 #define WALK_PAIRED 1
 #endif
@@ -1231,7 +1309,7 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
   else if (!exact && !need_group)
     PHYS_TRY(ws_alloc(c, WS_NODE_LO, nnodes, &w64));
   PHYS_LAUNCH(c, finalize_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, mc, exact ? 0 : 1,
-              p->leaf_cap, body64, c->d_hdr, rec64, w32, w64, w32x2);
+              p->leaf_cap, body64, c->d_hdr, rec64, wx, w32, w64, w32x2);
   if (need_group) {
     // breadth-first records for the group walk
     uint64_t *dk = nullptr, *dk_alt = nullptr;
@@ -1273,6 +1351,8 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
   t->leaf_cap = p->leaf_cap;
   t->link = link;
   t->rec64 = rec64;
+  t->wx = wx;
+  t->top = top;
   t->w32 = w32;
   t->w64 = w64;
   t->w32x2 = w32x2;

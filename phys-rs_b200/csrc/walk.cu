@@ -374,7 +374,326 @@ walk2_kernel(int q64, int n, int nnodes, const Rec32x2* __restrict__ w, const Bo
 
 // ---------------------------------------------------------------------------
 // F64_EXACT walk (leaf capacity 1).
+//
+// The traversal only decides: a node that some lane takes (a monopole or a
+// stored body) becomes an entry of the warp's queue in shared memory, with
+// the mask of those lanes, the level that the open partial sums close to
+// before it and its own level.  A full queue is evaluated kXU entries at a
+// time: every lane forms the weights (exact_scale, independent chains, the
+// node's record read once for the warp), then the terms are added in order,
+// the masked lanes' only.  Levels are opened and closed by the warp's path
+// for all lanes at once: a lane that did not open a cell has +0 in its level,
+// and adding that changes nothing.  The deepest level's sum is in registers,
+// the ones around it in local memory; closing a level adds it to the one
+// above, as the reference's nested sums do.
+//
+// Opening is decided in f32 on coordinates relative to the root cube: each
+// coordinate is within 2^-25 of its value, their difference within 2^-23, so
+// the distance is within 2.1e-7 of the half size and the lane's choice is the
+// f64 one outside a band of 4e-7 (and 1e-6 relative) around side / theta;
+// inside it, or when the masses do not all have one sign (a centre of mass
+// may then lie outside the cube), the warp takes the reference's f64 test.
+//
+// Few targets would leave most of the chip idle behind the longest walk, so
+// the children of the cells of more than n/8 bodies become tasks of their own
+// (grid.y; n/16 to n/64 make more tasks than they save walking: 10 000 bodies
+// 0.44 ms against 0.45, 0.55 and 0.68), each leaving its cell's contribution to each target in `part`;
+// exact_combine_kernel walks the cells above and sums them with the
+// reference's nesting.  Bound by the issue of the traversal and of the terms,
+// about 125 instructions per visit and warp, 37 of them on the FP64 pipe.
 // ---------------------------------------------------------------------------
+constexpr int kXQ = 32;  // queue entries per warp
+constexpr int kXU = 4;   // entries evaluated together
+constexpr float kXBand = 4e-7f;
+
+// Whether every pair of an evaluation is in exact_scale's range: masses of
+// one sign within [2^-190, 2^240 / n] or 0 (so are the sums over cells),
+// bodies and centres of mass within 2^98, softening.
+__device__ __forceinline__ bool walk_in_range(const TreeHeader* hdr, int64_t n, double eps2) {
+  const double c = fmax(fmax(fabs(hdr->center[0]), fabs(hdr->center[1])), fabs(hdr->center[2]));
+  return scale_eps2_ok(eps2) && hdr->min_mass >= 0.0 && hdr->min_abs >= 0x1p-190 &&
+         hdr->max_abs * (double)n < 0x1p240 && c + 2.0 * hdr->half < 0x1p98;
+}
+
+struct ExactTarget {
+  double x, y, z, gm;
+};
+
+// Term of compute_gravity_pair (gravity_tree.rs:218-234): its weight, and
+// the separation.
+template <bool kFast>
+__device__ __forceinline__ double exact_weight(const ExactTarget& t, double4 s, double eps2,
+                                               double& rx, double& ry, double& rz) {
+  rx = xsub(s.x, t.x), ry = xsub(s.y, t.y), rz = xsub(s.z, t.z);
+  const double s2 = xadd(xlen2(rx, ry, rz), eps2), a = xmul(t.gm, s.w);
+  return kFast ? exact_scale(a, s2) : exact_scale_ieee(a, s2);
+}
+
+// The nested sums of one target: the deepest level with a term in registers.
+struct NestedSum {
+  double st[kMaxLevels + 1][3];
+  double x, y, z;
+  int d;
+  __device__ __forceinline__ void init(int depth) {
+    x = y = z = 0.0;
+    d = depth;
+  }
+  // close the levels below m
+  __device__ __forceinline__ void close_to(int m) {
+    while (d > m) {
+      --d;
+      x = xadd(st[d][0], x);
+      y = xadd(st[d][1], y);
+      z = xadd(st[d][2], z);
+    }
+  }
+  // open levels up to depth, at 0
+  __device__ __forceinline__ void open_to(int depth) {
+    while (d < depth) {
+      st[d][0] = x;
+      st[d][1] = y;
+      st[d][2] = z;
+      x = y = z = 0.0;
+      ++d;
+    }
+  }
+  __device__ __forceinline__ void add(double tx, double ty, double tz) {
+    x = xadd(x, tx);
+    y = xadd(y, ty);
+    z = xadd(z, tz);
+  }
+};
+
+// The reference's opening test in f64 (gravity_tree.rs:192-194).
+__device__ __forceinline__ bool exact_open(double4 s, const ExactTarget& t, double s2,
+                                           double theta2) {
+  const double rx = xsub(s.x, t.x), ry = xsub(s.y, t.y), rz = xsub(s.z, t.z);
+  return !(s2 < xmul(theta2, xlen2(rx, ry, rz)));
+}
+
+__device__ __forceinline__ ExactTarget exact_target(const double4* body64, int64_t p, bool valid,
+                                                    double G) {
+  const double4 b = valid ? body64[p] : make_double4(0.0, 0.0, 0.0, 0.0);
+  return ExactTarget{b.x, b.y, b.z, xmul(G, b.w)};
+}
+
+// Number of tasks; a tree with more top nodes than there is room for is
+// walked as one task, the root.
+__device__ __forceinline__ int top_tasks(const TopTree& top) {
+  const int c = *top.counts, nt = c >> 16;
+  return nt <= top.max_tasks && (c & 0xffff) <= top.max_top ? nt : 1;
+}
+
+__global__ void __launch_bounds__(kWalkBlock, 4)
+walk_task_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const RecX* __restrict__ wx,
+                 const double4* __restrict__ rec64, const double4* __restrict__ body64,
+                 const TreeHeader* __restrict__ hdr, TopTree top, double G, double eps2,
+                 double* __restrict__ part, unsigned long long* counter, int32_t* status) {
+  wait_for_previous();
+  __shared__ double s2d[kMaxLevels];
+  __shared__ float2 band[kMaxLevels];
+  __shared__ uint4 queue[kWalkBlock / 32][kXQ];  // node, lane mask, close to, level
+  const int task = (int)blockIdx.y;
+  const int ntask = top_tasks(top);
+  if (task >= ntask) return;
+  const int root = ntask == 1 ? 0 : top.task[task];
+  const double theta2 = hdr->theta2, half = hdr->half;
+  for (int d = threadIdx.x; d < kMaxLevels; d += blockDim.x) {
+    s2d[d] = hdr->s2[d];
+    // side / theta in units of the half size, and the band around it
+    const double r = sqrt(hdr->s2[d] / theta2) / half;
+    const double lo = fmax(r - (double)kXBand, 0.0), hi = r + (double)kXBand;
+    band[d] = make_float2((float)(lo * lo * (1.0 - 1e-6)), (float)(hi * hi * (1.0 + 1e-6)));
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t p = q0 + blockIdx.x * (int64_t)kWalkBlock + threadIdx.x;  // targets [q0, n)
+  const bool valid = p < n;
+  const ExactTarget t = exact_target(body64, p, valid, G);
+  const bool coarse = hdr->min_mass >= 0.0;
+  const bool fast =
+      !__any_sync(0xffffffffu, !scale_mass_ok(t.gm)) && walk_in_range(hdr, nbody, eps2);
+  const double ih = 1.0 / half;
+  const float fx = (float)((t.x - hdr->center[0]) * ih), fy = (float)((t.y - hdr->center[1]) * ih),
+              fz = (float)((t.z - hdr->center[2]) * ih);
+
+  NestedSum sum;
+  unsigned ninter = 0;
+  int cnt = 0;
+  uint4* const q = queue[wid];
+  auto drain = [&]() {
+    __syncwarp();
+    for (int k0 = 0; k0 < cnt; k0 += kXU) {
+      double rx[kXU], ry[kXU], rz[kXU], w[kXU];
+      uint4 e[kXU];
+      if (fast) {
+#pragma unroll
+        for (int u = 0; u < kXU; ++u) {
+          e[u] = q[min(k0 + u, cnt - 1)];
+          w[u] = exact_weight<true>(t, rec64[e[u].x], eps2, rx[u], ry[u], rz[u]);
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < kXU; ++u) {
+          e[u] = q[min(k0 + u, cnt - 1)];
+          w[u] = exact_weight<false>(t, rec64[e[u].x], eps2, rx[u], ry[u], rz[u]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kXU; ++u) {
+        if (k0 + u < cnt) {
+          sum.close_to((int)e[u].z);
+          sum.open_to((int)e[u].w);
+          if ((e[u].y >> lane) & 1u) {
+            sum.add(xmul(rx[u], w[u]), xmul(ry[u], w[u]), xmul(rz[u], w[u]));
+            ++ninter;
+          }
+        }
+      }
+    }
+    __syncwarp();
+    cnt = 0;
+  };
+
+  // open_to: opened levels on the current path (a lane is active at a node
+  // of depth d iff open_to == d); low: the least depth of the warp's path
+  // since its last entry
+  // the task's cells above were all opened by the lane?
+  const int base = wx[root].b.x & kMetaDepth;
+  int open_to = -1;
+  if (valid) {
+    bool in = true;
+    for (int k = root, d = base - 1; d >= 0; --d) {
+      k = top.parent[k];
+      in = in && (k == 0 || (wx[k].b.x & kMetaGate)) && exact_open(rec64[k], t, s2d[d], theta2);
+    }
+    if (in) open_to = base;
+  }
+  const bool counted = open_to >= 0;
+  sum.init(base);
+  int low = base;
+  int node = root;
+  const int end = __float_as_int(wx[root].a.w);
+  auto ld_a = [&](int k) { return __ldg(&wx[k].a); };
+  auto ld_b = [&](int k) { return __ldg(reinterpret_cast<const int2*>(&wx[k].b)); };
+  float4 A = ld_a(node);
+  int2 B = ld_b(node);
+  while (node < end) {
+    const int next = __float_as_int(A.w);
+    if (next <= node || next > nnodes) {  // malformed tree: report, never spin
+      if (lane == 0) atomicOr(status, kStatOverflow);
+      break;
+    }
+    // both nodes that may follow are read while this one is decided
+    const int k0 = min(node + 1, nnodes - 1), k1 = min(next, nnodes - 1);
+    const float4 A0 = ld_a(k0), A1 = ld_a(k1);
+    const int2 B0 = ld_b(k0), B1 = ld_b(k1);
+    const int d = B.x & kMetaDepth;
+    open_to = min(open_to, d);
+    low = min(low, d);
+    const bool act = open_to == d && ((B.x & kMetaGate) || node == 0);
+    bool take;
+    int go = next;
+    if (B.x & kMetaLeaf) {
+      take = act && B.y != (int)p;
+    } else {
+      const float rx = A.x - fx, ry = A.y - fy, rz = A.z - fz;
+      const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+      const float2 bd = band[d];
+      bool open = act && d2 < bd.x;
+      if (__any_sync(0xffffffffu, act && !(coarse && (d2 < bd.x || d2 > bd.y))))
+        open = act && exact_open(rec64[node], t, s2d[d], theta2);
+      take = act && !open;
+      if (open) open_to = d + 1;
+      if (__any_sync(0xffffffffu, open)) go = node + 1;
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, take);
+    if (mask) {
+      if (lane == 0) q[cnt] = make_uint4((unsigned)node, mask, (unsigned)low, (unsigned)d);
+      low = d;
+      if (++cnt == kXQ) drain();
+    }
+    A = go == next ? A1 : A0;
+    B = go == next ? B1 : B0;
+    node = go;
+  }
+  drain();
+  sum.close_to(base);
+  warp_count(ninter, counter);
+  if (counted) {
+    double* o = part + ((size_t)task * (size_t)(n - q0) + (size_t)(p - q0)) * 3;
+    o[0] = sum.x;
+    o[1] = sum.y;
+    o[2] = sum.z;
+  }
+}
+
+// A target's force from its tasks' contributions: the walk over the upper
+// cells, nested as in compute_force (gravity_tree.rs:194-205).
+__global__ void __launch_bounds__(kWalkBlock)
+exact_combine_kernel(int64_t q0, int64_t n, const RecX* __restrict__ wx,
+                     const double4* __restrict__ rec64, const double4* __restrict__ body64,
+                     const uint32_t* __restrict__ perm, const TreeHeader* __restrict__ hdr,
+                     TopTree top, double G, double eps2, int want_force,
+                     const double* __restrict__ part, double* __restrict__ ox,
+                     double* __restrict__ oy, double* __restrict__ oz,
+                     unsigned long long* counter, int32_t* status) {
+  wait_for_previous();
+  const int64_t p = q0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const bool valid = p < n;
+  const ExactTarget t = exact_target(body64, valid ? p : q0, true, G);
+  const double theta2 = hdr->theta2;
+  const int ntop = top_tasks(top) == 1 ? 1 : *top.counts & 0xffff;
+  unsigned ninter = 0;
+  NestedSum sum;
+  sum.init(0);
+  int open_to = 0;
+  for (int i = 0; i < ntop; ++i) {
+    const int4 e = ntop == 1 ? make_int4(0, 0, 0, 0) : top.top[i];
+    const int node = e.x, d = e.z;
+    open_to = min(open_to, d);
+    sum.close_to(d);
+    const bool act = open_to == d && (node == 0 || (wx[node].b.x & kMetaGate));
+    if (e.y >= 0) {
+      sum.open_to(d);
+      if (act && valid) {
+        const double* q = part + ((size_t)e.y * (size_t)(n - q0) + (size_t)(p - q0)) * 3;
+        sum.add(q[0], q[1], q[2]);
+      }
+    } else {
+      const double4 r = rec64[node];
+      const bool open = act && exact_open(r, t, hdr->s2[d], theta2);
+      if (open) open_to = d + 1;
+      if (act && !open) {  // taken as a monopole
+        double rx, ry, rz;
+        const double w = exact_weight<false>(t, r, eps2, rx, ry, rz);
+        sum.open_to(d);
+        sum.add(xmul(rx, w), xmul(ry, w), xmul(rz, w));
+        ninter += valid;
+      }
+    }
+  }
+  sum.close_to(0);
+  warp_count(ninter, counter);
+  if (!valid) return;
+  double f[3] = {sum.x, sum.y, sum.z};
+  const double mi = body64[p].w;
+  const uint32_t i = perm[p];
+  double* o[3] = {ox, oy, oz};
+  bool bad = false;
+  for (int k = 0; k < 3; ++k) {
+    if (!want_force) f[k] = xdiv(f[k], mi);  // a = F / m (integrators.rs:115)
+    o[k][i] = f[k];
+    bad |= !isfinite(f[k]);
+  }
+  if (bad) atomicOr(status, kStatNonfinite);
+}
+
+// One walk per target over the whole tree, terms evaluated as they are
+// taken: 48 registers and more warps per SM hide the latency of a visit, so
+// with enough targets to fill the SMs this is the faster form (2^20 bodies:
+// 19.8 ms against 28.7 for walk_task_kernel over the root, 100 000: 2.9
+// against 3.0; 65 536: 2.7 against 2.1, 10 000: 1.64 against 0.44).
 __global__ void __launch_bounds__(kWalkBlock)
 walk_exact_kernel(int64_t q0, int64_t n, int64_t nnodes, const int4* __restrict__ link,
                   const double4* __restrict__ rec64, const double4* __restrict__ body64,
@@ -475,6 +794,14 @@ walk_exact_kernel(int64_t q0, int64_t n, int64_t nnodes, const int4* __restrict_
 
 }  // namespace
 
+int exact_walk_tasks(const phys_ctx* c, int64_t n) {
+  int64_t q0 = 0, q1 = n;
+  target_range(c, n, q0, q1);
+  const int64_t nt = q1 - q0;
+  // `part` holds 24 bytes per task and target: at most 100 MB
+  return nt > 0 && nt <= 65536 ? (int)min64(512, (int64_t(1) << 22) / nt) : 0;
+}
+
 int bh_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force, double* ox,
             double* oy, double* oz) {
   const int64_t n = t.n;
@@ -489,8 +816,21 @@ int bh_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force,
   if (p->flags & PHYS_FLAG_GROUP_WALK) {
     PHYS_TRY(bh_group_walk(c, p, t, want_force, ox, oy, oz));
   } else if (p->precision == PHYS_F64_EXACT) {
-    PHYS_LAUNCH(c, walk_exact_kernel, grid, kWalkBlock, 0, q0, q1, t.nnodes, t.link, t.rec64, t.body64,
-                t.perm, t.hdr, p->G, eps2, (int)want_force, ox, oy, oz, c->d_counter, c->d_status);
+    const int tasks = t.top.max_tasks;
+    if (tasks > 0) {
+      double* part = nullptr;
+      PHYS_TRY(ws_alloc(c, WS_DIRECT_PART, 3 * nt * tasks, &part));
+      PHYS_LAUNCH(c, walk_task_kernel, dim3(grid, tasks), kWalkBlock, 0, q0, q1, n, t.nnodes,
+                  t.wx, t.rec64, t.body64, t.hdr, t.top, p->G, eps2, part, c->d_counter,
+                  c->d_status);
+      PHYS_LAUNCH(c, exact_combine_kernel, (int)ceil_div(nt, 64), 64, 0, q0, q1, t.wx, t.rec64,
+                  t.body64, t.perm, t.hdr, t.top, p->G, eps2, want_force, part, ox, oy, oz,
+                  c->d_counter, c->d_status);
+    } else {
+      PHYS_LAUNCH(c, walk_exact_kernel, grid, kWalkBlock, 0, q0, q1, t.nnodes, t.link, t.rec64,
+                  t.body64, t.perm, t.hdr, p->G, eps2, want_force, ox, oy, oz, c->d_counter,
+                  c->d_status);
+    }
   } else if (p->precision == PHYS_F64) {
     PHYS_LAUNCH(c, walk_kernel<false>, grid, kWalkBlock, 0, (int)q0, (int)q1, (int)t.nnodes, t.w32, t.w64,
                 t.body64, t.body_hi, t.body_lo, t.perm, t.hdr, p->G, eps2, (int)want_force, ox, oy,
