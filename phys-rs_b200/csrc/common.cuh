@@ -144,7 +144,7 @@ struct phys_ctx {
   int32_t* h_small = nullptr;                // pinned scalars for status / counts
 
   // ---- workspace buffers (grown on demand, named) ----
-  phys::DevBuf ws[48];
+  phys::DevBuf ws[56];
 
   // ---- events for per-phase timings ----
   cudaEvent_t ev[12] = {};
@@ -178,7 +178,7 @@ enum WsSlot {
   WS_DIRECT_PART, WS_ADJ0, WS_ADJ1, WS_ADJ2, WS_ADJ3, WS_ADJ4,
   WS_ENS0, WS_ENS1, WS_ENS2, WS_ENS3, WS_ENS4, WS_ENS5, WS_ENS6, WS_ENS7,
   WS_GROUPS, WS_GROUP_OFF, WS_GROUP_CTR, WS_GROUP_POOL, WS_GROUP_ITEMS, WS_SHARE_PERM, WS_BODY_IN,
-  WS_COUNT_
+  WS_COM_SEG, WS_COM_TRAJ, WS_COUNT_
 };
 static_assert(WS_COUNT_ <= sizeof(phys_ctx::ws) / sizeof(DevBuf), "workspace slots");
 

@@ -629,10 +629,6 @@ gather_entries_kernel(int64_t total, const uint64_t* __restrict__ entries,
   }
 }
 
-// Cells with at least kLongChain bodies run on a warp each
-// (com_recurrence_long_kernel), the rest on a thread each.
-constexpr int kLongChain = 2048;
-
 // The reference recurrence over a cell's gathered bodies eb[e0, e1)
 // (gravity_tree.rs:113-118): M' = M + m, and when M' > 0,
 // c = (c M + x m) / M' per coordinate.  kFast divides through div_recip by
@@ -691,13 +687,14 @@ __device__ __forceinline__ bool com_chain(const double4* __restrict__ eb, int64_
 }
 
 // One thread per cell runs com_chain over the cell's gathered bodies.
-// Cells of kLongChain bodies or more are appended to `longs` (count in
-// longs[nnodes]) instead.
+// Cells of long_chain bodies or more are appended to `longs` (count in
+// longs[nnodes]) instead (com.cu).
 __global__ void __launch_bounds__(kBlock)
 com_recurrence_kernel(int64_t nnodes, const int32_t* __restrict__ eoff,
                       const double4* __restrict__ eb, double4* __restrict__ mc,
                       const int4* __restrict__ link, const TreeHeader* __restrict__ hdr,
-                      int skip_unused, int32_t* __restrict__ longs, const int32_t* status) {
+                      int skip_unused, int long_chain, int32_t* __restrict__ longs,
+                      const int32_t* status) {
   wait_for_previous();
   if (sort_failed(status)) return;
   // the bound holds when every centre of mass is a convex combination of
@@ -712,147 +709,13 @@ com_recurrence_kernel(int64_t nnodes, const int32_t* __restrict__ eoff,
       mc[k] = make_double4(nan, nan, nan, __longlong_as_double(0x7ff0000000000000ll));
       continue;
     }
-    if (e1 - e0 >= kLongChain) {
+    if (e1 - e0 >= long_chain) {
       longs[atomicAdd(&longs[nnodes], 1)] = (int32_t)k;
       continue;
     }
     double4 r;
     if (!com_chain<true>(eb, e0, e1, r)) com_chain<false>(eb, e0, e1, r);
     mc[k] = r;
-  }
-}
-
-// The same recurrence for the cells listed by com_recurrence_kernel, a warp
-// per cell: the warp stages 32 bodies at a time in shared memory (one
-// coalesced 1 KiB read, the next batch's in flight) while lanes 0, 1 and 2
-// run the x, y and z chains.
-constexpr int kLongWarps = 4;
-struct LongStage {
-  double4 rec[2][32];           // two batches of body records (x, y, z, m)
-  double nt[2][32], y[2][32];   // per body: running mass M + m, RN(1/(M + m))
-};
-
-// The reference's form (com_chain<false> per coordinate lane): the fallback.
-__device__ void com_chain_warp_ieee(const double4* __restrict__ eb, int64_t e0, int64_t e1,
-                                   LongStage& S, int lane, double4& out) {
-  const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
-  double M = 0.0, cc = 0.0;  // lane j < 3: coordinate j
-  double4 v = e0 + lane < e1 ? eb[e0 + lane] : zero;
-  for (int64_t e = e0; e < e1; e += 32) {
-    S.rec[0][lane] = v;
-    __syncwarp();
-    v = e + 32 + lane < e1 ? eb[e + 32 + lane] : zero;
-    const int cnt = (int)min((int64_t)32, e1 - e);
-    if (lane < 3) {
-      const double* q = reinterpret_cast<const double*>(&S.rec[0][0]);
-      for (int u = 0; u < cnt; ++u) {
-        const double p = q[4 * u + lane], mm = q[4 * u + 3];
-        const double nt = xadd(M, mm);
-        if (nt > 0.0) cc = xdiv(xadd(xmul(cc, M), xmul(p, mm)), nt);
-        M = nt;
-      }
-    }
-    __syncwarp();
-  }
-  const double cy = __shfl_sync(0xffffffffu, cc, 1), cz = __shfl_sync(0xffffffffu, cc, 2);
-  out = make_double4(cc, cy, cz, M);
-}
-
-// The fast form: per body a multiply, an add and div_recip's five
-// operations, with nothing else on the chain.  The running masses of a
-// batch (the reference's additions, in order) are summed by lane 0 while the
-// batch before it runs, and the whole warp then forms the batch's 32
-// reciprocals at once (__drcp_rn, correctly rounded, as div_recip requires),
-// so the chain's loop over a full batch has no branch and its shared-memory
-// loads can be issued ahead.  Returns false (warp-uniform) when a step left
-// div_recip's range or the running mass was not positive; the caller then
-// reruns the cell in the reference's form.
-__device__ bool com_chain_warp_fast(const double4* __restrict__ eb, int64_t e0, int64_t e1,
-                                    LongStage& S, int lane, double4& out) {
-  const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
-  const int64_t len = e1 - e0;
-  S.rec[0][lane] = lane < len ? eb[e0 + lane] : zero;
-  double4 v = 32 + lane < len ? eb[e0 + 32 + lane] : zero;
-  __syncwarp();
-  if (lane == 0) {  // running masses of batch 0
-    double M = 0.0;
-    const int c0 = (int)min((int64_t)32, len);
-    for (int u = 0; u < c0; ++u) {
-      M = xadd(M, S.rec[0][u].w);
-      S.nt[0][u] = M;
-    }
-  }
-  __syncwarp();
-  S.y[0][lane] = __drcp_rn(S.nt[0][lane]);  // lanes past the batch: unused
-  __syncwarp();
-  bool ok = true;
-  double cc = 0.0, M = 0.0;  // lane j < 3: coordinate j; M = mass before the body
-  for (int64_t base = e0; base < e1; base += 32) {
-    const int cur = (int)(((base - e0) >> 5) & 1), nxt = cur ^ 1;
-    const int cnt = (int)min((int64_t)32, e1 - base);
-    const int cntn = (int)max((int64_t)0, min((int64_t)32, e1 - base - 32));
-    if (cntn > 0) S.rec[nxt][lane] = v;
-    __syncwarp();
-    v = base + 64 + lane < e1 ? eb[base + 64 + lane] : zero;
-    if (lane < 3) {
-      const double* __restrict__ rc = reinterpret_cast<const double*>(&S.rec[cur][0]);
-      const double* __restrict__ rn = reinterpret_cast<const double*>(&S.rec[nxt][0]);
-      const double* __restrict__ ntc = S.nt[cur];
-      const double* __restrict__ yc = S.y[cur];
-      auto step = [&](int u) {
-        const double nt = ntc[u];
-        const double a = xadd(xmul(cc, M), xmul(rc[4 * u + lane], rc[4 * u + 3]));
-        ok &= div_recip_den_ok(nt) & div_recip_num_ok(a);
-        cc = div_recip(a, nt, yc[u]);
-        M = nt;
-      };
-      if (cnt == 32) {
-        // the next batch's running masses, in registers until the batch is
-        // done (a store into the arrays the loop reads would keep the
-        // loads behind it)
-        double Mn[32];
-        double acc = ntc[31];  // running mass before the next batch
-#pragma unroll
-        for (int u = 0; u < 32; ++u) {
-          step(u);
-          acc = xadd(acc, rn[4 * u + 3]);  // bodies past cntn: never stored
-          Mn[u] = acc;
-        }
-        if (lane == 0) {
-#pragma unroll
-          for (int u = 0; u < 32; ++u)
-            if (u < cntn) S.nt[nxt][u] = Mn[u];
-        }
-      } else {  // the last batch of the cell
-        for (int u = 0; u < cnt; ++u) step(u);
-      }
-    }
-    __syncwarp();
-    if (cntn > 0) S.y[nxt][lane] = __drcp_rn(S.nt[nxt][lane]);
-    __syncwarp();
-  }
-  const double cy = __shfl_sync(0xffffffffu, cc, 1), cz = __shfl_sync(0xffffffffu, cc, 2);
-  out = make_double4(cc, cy, cz, M);
-  return !__any_sync(0xffffffffu, !ok);
-}
-
-__global__ void __launch_bounds__(32 * kLongWarps)
-com_recurrence_long_kernel(int64_t nnodes, const int32_t* __restrict__ eoff,
-                           const double4* __restrict__ eb, double4* __restrict__ mc,
-                           const int32_t* __restrict__ longs, const int32_t* status) {
-  wait_for_previous();
-  if (sort_failed(status)) return;
-  __shared__ LongStage stage[kLongWarps];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int nlong = min(longs[nnodes], (int32_t)nnodes);
-  for (int i = blockIdx.x * kLongWarps + w; i < nlong; i += gridDim.x * kLongWarps) {
-    const int k = longs[i];
-    const int64_t e0 = eoff[k], e1 = eoff[k + 1];
-    double4 r;
-    if (!com_chain_warp_fast(eb, e0, e1, stage[w], lane, r))
-      com_chain_warp_ieee(eb, e0, e1, stage[w], lane, r);
-    if (lane == 0) mc[k] = r;
-    __syncwarp();
   }
 }
 
@@ -1263,9 +1126,8 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     int32_t* longs = ncnt;
     PHYS_CUDA(c, cudaMemsetAsync(longs + nnodes, 0, sizeof(int32_t), c->stream));
     PHYS_LAUNCH(c, com_recurrence_kernel, grid_for(nnodes, 128, 1 << 30), 128, 0, nnodes, eoff, eb,
-                mc, link, c->d_hdr, full_com ? 0 : 1, longs, c->d_status);
-    PHYS_LAUNCH(c, com_recurrence_long_kernel, 148 * 4, 32 * kLongWarps, 0, nnodes, eoff, eb, mc,
-                longs, c->d_status);
+                mc, link, c->d_hdr, full_com ? 0 : 1, com_long_chain(n), longs, c->d_status);
+    PHYS_TRY(com_long_cells(c, n, nnodes, total, eoff, eb, link, c->d_hdr, longs, mc));
   } else {
     PHYS_CUDA(c, cudaMemsetAsync(arrive, 0, sizeof(int32_t) * (nnodes + 1), c->stream));
     PHYS_LAUNCH(c, com_upward_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, parent, nchild,
