@@ -199,6 +199,16 @@ int direct_eval(phys_ctx* c, const phys_params* p, bool want_force, double* ox, 
 int direct_exact_tick(phys_ctx* c, const phys_params* p, double dt, bool to_scratch);
 int direct_targets(phys_ctx* c, const phys_params* p, int64_t nt, const int64_t* d_tidx,
                    double* ox, double* oy, double* oz);
+// The F64 sum's layout for n bodies, and its kernel: partial sums per slice
+// into part (3 n doubles each), or results when part is null (one slice).
+struct F64Plan {
+  int64_t slice_len, slices;
+};
+F64Plan f64_plan(int64_t n, int64_t most_slices);
+void direct_f64_launch(cudaStream_t s, const F64Plan& plan, int64_t n, int64_t t0, int64_t t1,
+                       const double* x, const double* y, const double* z, const double* m,
+                       double G, double eps2, int want_force, double* ox, double* oy, double* oz,
+                       double* part, int32_t* status);
 // Launches on stream s with caller-provided scratch; returns the launch error.
 cudaError_t direct_accel_launch_scratch(cudaStream_t s, int64_t n, const double* x,
                                         const double* y, const double* z, const double* m,
@@ -437,6 +447,16 @@ __device__ __forceinline__ double inv_cubed(double x) {
   const double h = fma(-xc, t, 1.0);
   const double y3 = t * y0;
   return fma(y3 * h, fma(h, 1.875, 1.5), y3);
+}
+
+// 1/sqrt(x) the same way: y0 (1 + h/2 + 3/8 h^2), within 1.01 u; for the VJP,
+// which needs the fifth power as well.
+__device__ __forceinline__ double inv_root(double x) {
+  const double xc = __hiloint2double(min(__double2hiint(x), 0x7fe00000), __double2loint(x));
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(xc));
+  const double h = fma(-xc, y0 * y0, 1.0);
+  return fma(y0 * h, fma(h, 0.375, 0.5), y0);
 }
 
 // sum_{s < nsl} p[s stride], added in slice order from 0.0 (the order the

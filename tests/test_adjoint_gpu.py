@@ -134,3 +134,43 @@ def test_adjoint_vs_full_difference_gradient(ctx):
     ctx.upload(pos, vel, m)
     assert np.linalg.norm(gx - fx) / np.linalg.norm(fx) < 1e-6
     assert np.linalg.norm(gv - fv) / np.linalg.norm(fv) < 1e-6
+
+
+def test_segments_beyond_the_kept_positions(ctx):
+    """2800 steps of 4096 bodies (262 MiB of positions, more than are kept):
+    checkpointed segments of any length, recomputed, give the gradient of one
+    segment over the whole run bit for bit."""
+    n, nsteps, dt = 4096, 2800, 1e-4
+    pos, vel, m = ics.plummer(n, seed=5)
+    p = make_params(1.0, 0.05, precision=F64)
+    ctx.upload(pos, vel, m)
+    targets = pos + 0.1
+    ref = ctx.adjoint(p, dt, nsteps, targets, checkpoint=nsteps)
+    for K in (700, 999):
+        out = ctx.adjoint(p, dt, nsteps, targets, checkpoint=K)
+        assert out[0] == ref[0]
+        for a, b in zip(out[1:], ref[1:]):
+            assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [2, 63, 64, 65, 127, 128, 129, 1000])
+def test_vjp_tiles(ctx, n):
+    """One-step gradients at the edges of the VJP's tiles and slices against
+    the analytic gradient in numpy (sums of at most 1000 terms: 1e-12)."""
+    pos, vel, m = ics.plummer(n, seed=40 + n)
+    eps, dt = 0.05, 1e-2
+    ctx.upload(pos, vel, m)
+    targets = pos + 0.3
+    _, gx, gv, gm = ctx.adjoint(make_params(1.0, eps, precision=F64), dt, 1, targets)
+    r = pos[None] - pos[:, None]
+    s2 = (r * r).sum(-1) + eps * eps
+    acc = (m[None, :, None] * r / s2[..., None] ** 1.5).sum(1)
+    w = 2.0 * (pos + vel * dt + acc * (0.5 * dt * dt) - targets)
+    wa = w * (0.5 * dt * dt)
+    q = m[None, :, None] * wa[:, None] - m[:, None, None] * wa[None]
+    k3 = s2 ** -1.5
+    rq = (r * q).sum(-1)
+    jx = (q * k3[..., None] - 3.0 * r * (rq * s2 ** -2.5)[..., None]).sum(0)
+    jm = ((r * wa[:, None]).sum(-1) * k3).sum(0)
+    for got, want in ((gx, w + jx), (gv, w * dt), (gm, jm)):
+        assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
