@@ -52,7 +52,10 @@ struct __align__(16) Rec32x2 {
 struct __align__(16) Body32x2 {
   float4 q0, q1, q2, q3;  // same layout, ropen2 slot unused
 };
-// Group-walk record, breadth-first order (children of a cell contiguous).
+// Group-walk record, breadth-first order (children of a cell contiguous): what
+// the list walk reads, 48 bytes; the f64 position and mass that only the
+// evaluation reads are an array of their own (BhTree::gsrc), one 32-byte
+// sector per entry.
 // l = {a, (b << 2) | type, first body, end body} (sorted positions; the
 // cell holds bodies [first, end)).  internal: a = first child, b = child
 // count; one-body leaf: a = the body it stands for (the last inserted one for
@@ -67,9 +70,8 @@ struct __align__(16) GNode {
   float4 hi;    // x_hi, y_hi, z_hi, mass (f32)
   float4 lo;    // x_lo, y_lo, z_lo, cell side squared (2h)^2 (f32)
   int4 l;
-  double4 c64;  // x, y, z, mass (f64)
 };
-static_assert(sizeof(GNode) == 80, "GNode layout");
+static_assert(sizeof(GNode) == 48, "GNode layout");
 struct __align__(16) Rec64 {
   double4 a;  // x, y, z, mass
   int4 l;
@@ -112,6 +114,7 @@ struct BhTree {
   const float4* body_lo = nullptr;
   const TreeHeader* hdr = nullptr;
   const GNode* gnode = nullptr;       // group-walk records (breadth-first)
+  const double4* gsrc = nullptr;      // and their x, y, z, mass
   const int2* groups = nullptr;       // group-walk target groups: body ranges [x, y),
                                       // room for n more (re-queued subgroups) after n
   const int32_t* ngroups = nullptr;   // device: number of groups

@@ -216,7 +216,7 @@ __device__ __forceinline__ Box group_box(double4 X0, double4 ta, double4 tb) {
 }
 
 // What one popped cell contributes: children to push, and list entries
-// (kind 1: the cell itself / the body of a one-body leaf, source c64 of
+// (kind 1: the cell itself / the body of a one-body leaf, source c64, that of
 // record a; kind 2: the bodies [a, a + nent) of a bucket leaf, skipping the
 // group's range [olo, ohi)).
 struct NodeOut {
@@ -228,7 +228,7 @@ struct NodeOut {
 template <bool kNeedC64>
 __device__ __forceinline__ void classify(int nd, int base, int gend, int nnodes, const Box& B,
                                          float theta2f, const GNode* __restrict__ gn,
-                                         NodeOut& o) {
+                                         const double4* __restrict__ gsrc, NodeOut& o) {
   o.npush = o.cfirst = o.nent = o.kind = o.a = o.olo = o.ohi = 0;
   o.malformed = false;
   o.c64 = make_double4(0.0, 0.0, 0.0, 0.0);
@@ -237,7 +237,7 @@ __device__ __forceinline__ void classify(int nd, int base, int gend, int nnodes,
   const GNode* g = gn + nd;
   const int4 l = __ldg(&g->l);
   const float4 h = __ldg(&g->hi), lo = __ldg(&g->lo);
-  if (kNeedC64) o.c64 = ldg_d4(&g->c64);
+  if (kNeedC64) o.c64 = ldg_d4(&gsrc[nd]);
   const int type = l.y & 3, cnt = l.y >> 2;
   const bool inside = l.z >= base && l.w <= gend;  // only group bodies
   if (type == kGSkip || inside) return;
@@ -296,7 +296,8 @@ __device__ __forceinline__ int bucket_body(int a, int olo, int ohi, int j) {
 template <bool kNeedC64, class Sink>
 __device__ __forceinline__ int traverse(int lane, int base, int gend, int nnodes, int limit,
                                         int* stk, const Box& B, float theta2f,
-                                        const GNode* __restrict__ gn, Sink& sink) {
+                                        const GNode* __restrict__ gn,
+                                        const double4* __restrict__ gsrc, Sink& sink) {
   int ssize = 1, listed = 0;
   long long pops = 0;
   if (lane == 0) stk[0] = 0;
@@ -309,11 +310,19 @@ __device__ __forceinline__ int traverse(int lane, int base, int gend, int nnodes
     pops += k;
     __syncwarp();
     NodeOut o;
-    classify<kNeedC64>(nd, base, gend, nnodes, B, theta2f, gn, o);
+    classify<kNeedC64>(nd, base, gend, nnodes, B, theta2f, gn, gsrc, o);
     if (pops > nnodes) o.malformed = true;
-    // both scans first (independent chains), then pushes, then entries
-    const int pin = warp_incl_scan(o.npush, lane);
-    const int ein = warp_incl_scan(o.nent, lane);
+    // both scans in one (pushes in the low half: at most 32 x 8), unless a
+    // leaf of very many bodies overflows the high half; then pushes, entries
+    int pin = o.npush | (o.nent << 16), ein;
+    if (__any_sync(kFull, o.nent > 1000)) {
+      pin = warp_incl_scan(o.npush, lane);
+      ein = warp_incl_scan(o.nent, lane);
+    } else {
+      pin = warp_incl_scan(pin, lane);
+      ein = pin >> 16;
+      pin &= 0xffff;
+    }
     const int ptot = __shfl_sync(kFull, pin, 31);
     const int etot = __shfl_sync(kFull, ein, 31);
     if (__any_sync(kFull, o.malformed) || ssize + ptot > kGStack) return -1;
@@ -761,7 +770,7 @@ struct Evaluator {
   // F32C-vs-F64 median stays at 5e-8); the rest go to the near list
   // (double-float).  F64: the staged records are the list.
   __device__ __forceinline__ void stream_eval(const uint32_t* __restrict__ codes, int len,
-                                              const GNode* __restrict__ gn,
+                                              const double4* __restrict__ gsrc,
                                               const double4* __restrict__ body64, const Box& B,
                                               float far2, double4* stage) {
     constexpr int kPer = kL / 32;
@@ -781,7 +790,7 @@ struct Evaluator {
       for (int j = 0; j < kPer; ++j) {
         if (pc[j] != ~0u) {
           const int id = (int)(pc[j] >> 1);
-          const double4* src = (pc[j] & 1u) ? body64 + id : &gn[id].c64;
+          const double4* src = ((pc[j] & 1u) ? body64 : gsrc) + id;
           double4* d = dst + lane + 32 * j;
           cp_async16(d, src);
           cp_async16(reinterpret_cast<char*>(d) + 16, reinterpret_cast<const char*>(src) + 16);
@@ -1016,7 +1025,7 @@ glist_kernel(int n, int q0, int q1, int nnodes, const GNode* __restrict__ gn,
       return true;
     };
     const int r = traverse<false>(lane, base, gend, nnodes, kGListLimit, stk, B, theta2f, gn,
-                                  sink);
+                                  nullptr, sink);
     if (r < 0) {
       bad = true;
       break;
@@ -1045,7 +1054,7 @@ glist_kernel(int n, int q0, int q1, int nnodes, const GNode* __restrict__ gn,
 // ---------------------------------------------------------------------------
 template <bool kF32>
 __global__ void __launch_bounds__(kGBlock, GEVAL_MIN_BLOCKS)
-geval_kernel(int n, const GNode* __restrict__ gn, const int4* __restrict__ items,
+geval_kernel(int n, const double4* __restrict__ gsrc, const int4* __restrict__ items,
              const int32_t* __restrict__ nitems_p, int32_t* __restrict__ ctr,
              const uint32_t* __restrict__ pool, const double4* __restrict__ body64,
              const uint32_t* __restrict__ perm, double G, double eps2, int want_force,
@@ -1071,7 +1080,7 @@ geval_kernel(int n, const GNode* __restrict__ gn, const int4* __restrict__ items
     const float far2 = (float)(GWALK_FAR * GWALK_FAR) * fmaf(B.bx, B.bx, fmaf(B.by, B.by, B.bz * B.bz));
     E.self_pass();
     ninter += (unsigned long long)E.nvalid * (unsigned long long)(E.nvalid - 1 + len);
-    E.stream_eval(codes, len, gn, body64, B, far2,
+    E.stream_eval(codes, len, gsrc, body64, B, far2,
                   reinterpret_cast<double4*>(lbase + kEListBytes));
     E.finish(body64, perm, G, want_force, ox, oy, oz, status);
   }
@@ -1086,7 +1095,8 @@ geval_kernel(int n, const GNode* __restrict__ gn, const int4* __restrict__ items
 // ---------------------------------------------------------------------------
 template <bool kF32>
 __global__ void __launch_bounds__(kGBlock, 4)
-gwalk_kernel(int n, int nnodes, const GNode* __restrict__ gn, const int2* __restrict__ groups,
+gwalk_kernel(int n, int nnodes, const GNode* __restrict__ gn,
+             const double4* __restrict__ gsrc, const int2* __restrict__ groups,
              const int32_t* __restrict__ ngroups_p, int32_t* __restrict__ ctr,
              const double4* __restrict__ body64, const uint32_t* __restrict__ perm, double G,
              double eps2, float theta2f, int want_force, double* __restrict__ ox,
@@ -1177,7 +1187,8 @@ gwalk_kernel(int n, int nnodes, const GNode* __restrict__ gn, const int2* __rest
       __syncwarp();
       return true;
     };
-    const int r = traverse<true>(lane, gr.x, gr.y, nnodes, INT_MAX, stk, B, theta2f, gn, sink);
+    const int r = traverse<true>(lane, gr.x, gr.y, nnodes, INT_MAX, stk, B, theta2f, gn, gsrc,
+                                 sink);
     if (r != 1) {
       bad = true;
       break;
@@ -1258,11 +1269,11 @@ int launch(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force, 
   PHYS_CUDA(c, cudaEventRecord(c->fork, c->stream));
   PHYS_CUDA(c, cudaStreamWaitEvent(c->side, c->fork, 0));
   PHYS_LAUNCH_ON(c, c->side, gwalk_kernel<kF32>, grid_fused, kGBlock, kGSmem, (int)n,
-                 (int)t.nnodes, t.gnode, retry, ctr + 1, ctr + 4, t.body64, t.perm, p->G, eps2,
+                 (int)t.nnodes, t.gnode, t.gsrc, retry, ctr + 1, ctr + 4, t.body64, t.perm, p->G, eps2,
                  theta2f, (int)want_force, ox, oy, oz, c->d_counter, c->d_status);
   PHYS_CUDA(c, cudaEventRecord(c->join, c->side));
   PHYS_CUDA(c, cudaEventRecord(c->ev[10], c->stream));
-  PHYS_LAUNCH(c, geval_kernel<kF32>, grid_eval, kGBlock, kESmem, (int)n, t.gnode, items, ctr + 2,
+  PHYS_LAUNCH(c, geval_kernel<kF32>, grid_eval, kGBlock, kESmem, (int)n, t.gsrc, items, ctr + 2,
               ctr + 3, pool, t.body64, t.perm, p->G, eps2, (int)want_force, ox, oy, oz,
               c->d_counter, c->d_status);  // adds to counter[0] and counter[1]
   PHYS_CUDA(c, cudaEventRecord(c->ev[11], c->stream));

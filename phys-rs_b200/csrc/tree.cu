@@ -867,7 +867,7 @@ gnode_kernel(int64_t nnodes, const uint32_t* __restrict__ bfs2pre,
              const int32_t* __restrict__ pre2bfs, const int4* __restrict__ link,
              const double4* __restrict__ mc, const int32_t* __restrict__ nchild, int leaf_cap,
              const double4* __restrict__ body64, const TreeHeader* __restrict__ hdr,
-             GNode* __restrict__ g, const int32_t* status) {
+             GNode* __restrict__ g, double4* __restrict__ gsrc, const int32_t* status) {
   wait_for_previous();
   if (sort_failed(status)) return;
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nnodes;
@@ -898,8 +898,8 @@ gnode_kernel(int64_t nnodes, const uint32_t* __restrict__ bfs2pre,
     o.hi.w = (float)r.w;
     o.lo.w = (float)hdr->s2[d];
     o.l = l;
-    o.c64 = r;
     g[j] = o;
+    gsrc[j] = r;
   }
 }
 
@@ -1178,12 +1178,14 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     uint32_t *dv = nullptr, *dv_alt = nullptr;
     int32_t* pre2bfs = nullptr;
     GNode* g = nullptr;
+    double4* gsrc = nullptr;
     PHYS_TRY(ws_alloc(c, WS_ENTRIES, nnodes, &dk));
     PHYS_TRY(ws_alloc(c, WS_ENTRIES_ALT, nnodes, &dk_alt));
     PHYS_TRY(ws_alloc(c, WS_KEEP, nnodes, &dv));
     PHYS_TRY(ws_alloc(c, WS_NEWID, nnodes, &dv_alt));
     PHYS_TRY(ws_alloc(c, WS_EOFF, nnodes + 1, &pre2bfs));
     PHYS_TRY(ws_alloc(c, WS_ENS5, nnodes, &g));
+    PHYS_TRY(ws_alloc(c, WS_NODE_LO, nnodes, &gsrc));
     PHYS_LAUNCH(c, depth_key_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, dk, dv);
     bool alt = false;
     PHYS_TRY(radix_sort_u64(c, dk, dv, dk_alt, dv_alt, nnodes, 0, 8, &alt));
@@ -1191,8 +1193,9 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     PHYS_LAUNCH(c, invert_kernel, grid_for(nnodes), kBlock, 0, nnodes, bfs2pre, pre2bfs,
                 c->d_status);
     PHYS_LAUNCH(c, gnode_kernel, grid_for(nnodes), kBlock, 0, nnodes, bfs2pre, pre2bfs, link, mc,
-                nchild, p->leaf_cap, body64, c->d_hdr, g, c->d_status);
+                nchild, p->leaf_cap, body64, c->d_hdr, g, gsrc, c->d_status);
     t->gnode = g;
+    t->gsrc = gsrc;
     int32_t *gcnt = nullptr, *goff = nullptr, *gctr = nullptr;
     int2* groups = nullptr;
     PHYS_TRY(ws_alloc(c, WS_NCOUNT, nnodes + 1, &gcnt));
