@@ -77,16 +77,20 @@ int ensure_pinned(phys_ctx* c, size_t bytes) {
   return PHYS_OK;
 }
 
+// Place of the status block in the pinned scalars (the tree build's counts
+// and the sector flag lie below).
+constexpr int kHostStatus = 64;
+
 int read_status(phys_ctx* c, int32_t* out) {
-  PHYS_CUDA(c, cudaMemcpyAsync(c->h_small, c->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost,
+  // status word and counters are 256 bytes apart in one block: one copy
+  PHYS_CUDA(c, cudaMemcpyAsync(c->h_small + kHostStatus, c->d_status,
+                               256 + 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                                c->stream));
-  PHYS_CUDA(c, cudaMemcpyAsync(c->h_small + 2, c->d_counter, 2 * sizeof(unsigned long long),
-                               cudaMemcpyDeviceToHost, c->stream));
   PHYS_CUDA(c, cudaStreamSynchronize(c->stream));
-  *out = c->h_small[0];
+  *out = c->h_small[kHostStatus];
   if (c->last_eval_bh) {
     unsigned long long v[2];
-    memcpy(v, c->h_small + 2, sizeof v);
+    memcpy(v, c->h_small + kHostStatus + 64, sizeof v);
     c->tm.interactions = v[0];
     c->tm.walk_eval_interactions = c->last_eval_group ? v[1] : 0;
   }
@@ -140,6 +144,57 @@ int h2d(phys_ctx* c, double* dst, const double* src, int64_t n) {
 int d2h(phys_ctx* c, double* dst, const double* src, int64_t n) {
   if (dst)
     PHYS_CUDA(c, cudaMemcpyAsync(dst, src, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+  return PHYS_OK;
+}
+
+// Host arrays of n 8-byte values into `rows` consecutive state arrays from
+// `first` on (the state is one allocation, cap apart; null: zeros).  Small
+// states are packed into the pinned staging buffer at `at` and go out in one
+// copy: a copy call costs 2 to 4 us whatever its size (100 bodies: 7 copies
+// and 9 memsets of a system call against 3 calls).
+constexpr int64_t kPackBytes = int64_t(4) << 20;
+
+bool packs(int64_t n, int rows) { return 8 * n * rows <= kPackBytes; }
+
+int copy_rows(phys_ctx* c, double* first, int rows, const void* const* src, int64_t n,
+              int64_t at) {
+  if (!packs(n, rows)) {
+    for (int k = 0; k < rows; ++k)
+      PHYS_TRY(h2d(c, first + k * c->cap, static_cast<const double*>(src[k]), n));
+    return PHYS_OK;
+  }
+  double* h = static_cast<double*>(c->h_stage) + at;
+  for (int k = 0; k < rows; ++k) {
+    if (src[k])
+      memcpy(h + k * n, src[k], 8 * n);
+    else
+      memset(h + k * n, 0, 8 * n);
+  }
+  PHYS_CUDA(c, cudaMemcpy2DAsync(first, 8 * c->cap, h, 8 * n, 8 * n, rows,
+                                 cudaMemcpyHostToDevice, c->stream));
+  return PHYS_OK;
+}
+
+// A strided call takes a pitch below 2^31 bytes.
+bool one_call(const phys_ctx* c) { return 8 * c->cap < (int64_t(1) << 31); }
+
+int zero_rows(phys_ctx* c, double* first, int rows, int64_t n) {
+  if (one_call(c)) {
+    PHYS_CUDA(c, cudaMemset2DAsync(first, 8 * c->cap, 0, 8 * n, rows, c->stream));
+    return PHYS_OK;
+  }
+  for (int k = 0; k < rows; ++k) PHYS_TRY(h2d(c, first + k * c->cap, nullptr, n));
+  return PHYS_OK;
+}
+
+// fx, fy, fz into h (3 n, pinned).
+int forces_to_host(phys_ctx* c, double* h, int64_t n) {
+  if (one_call(c)) {
+    PHYS_CUDA(c, cudaMemcpy2DAsync(h, 8 * n, c->fx, 8 * c->cap, 8 * n, 3, cudaMemcpyDeviceToHost,
+                                   c->stream));
+    return PHYS_OK;
+  }
+  for (int k = 0; k < 3; ++k) PHYS_TRY(d2h(c, h + k * n, c->fx + k * c->cap, n));
   return PHYS_OK;
 }
 
@@ -531,19 +586,10 @@ int phys_state_upload(phys_ctx* c, int64_t n, const double* x, const double* y, 
   c->sector_mode = false;
   c->accel_valid = false;
   if (n == 0) return PHYS_OK;
-  PHYS_TRY(h2d(c, c->x, x, n));
-  PHYS_TRY(h2d(c, c->y, y, n));
-  PHYS_TRY(h2d(c, c->z, z, n));
-  PHYS_TRY(h2d(c, c->vx, vx, n));
-  PHYS_TRY(h2d(c, c->vy, vy, n));
-  PHYS_TRY(h2d(c, c->vz, vz, n));
-  PHYS_TRY(h2d(c, c->m, m, n));
-  PHYS_TRY(h2d(c, c->ax, nullptr, n));
-  PHYS_TRY(h2d(c, c->ay, nullptr, n));
-  PHYS_TRY(h2d(c, c->az, nullptr, n));
-  PHYS_TRY(h2d(c, c->pax, nullptr, n));
-  PHYS_TRY(h2d(c, c->pay, nullptr, n));
-  PHYS_TRY(h2d(c, c->paz, nullptr, n));
+  const void* src[7] = {x, y, z, vx, vy, vz, m};
+  if (packs(n, 7)) PHYS_TRY(ensure_pinned(c, 8 * 7 * n));
+  PHYS_TRY(copy_rows(c, c->x, 7, src, n, 0));
+  PHYS_TRY(zero_rows(c, c->ax, 6, n));  // Acceleration, PreviousAcceleration
   PHYS_CUDA(c, cudaStreamSynchronize(c->stream));
   return PHYS_OK;
 }
@@ -565,26 +611,15 @@ int phys_state_upload_sectors(phys_ctx* c, int64_t n, const int64_t* sx, const i
   if (n == 0) return PHYS_OK;
   // Stage sectors in the force scratch arrays (same size as int64) and the
   // local positions in x/y/z, then flatten in place on the device.
-  int64_t* dsx = reinterpret_cast<int64_t*>(c->fx);
-  int64_t* dsy = reinterpret_cast<int64_t*>(c->fy);
-  int64_t* dsz = reinterpret_cast<int64_t*>(c->fz);
-  PHYS_CUDA(c, cudaMemcpyAsync(dsx, sx, 8 * n, cudaMemcpyHostToDevice, c->stream));
-  PHYS_CUDA(c, cudaMemcpyAsync(dsy, sy, 8 * n, cudaMemcpyHostToDevice, c->stream));
-  PHYS_CUDA(c, cudaMemcpyAsync(dsz, sz, 8 * n, cudaMemcpyHostToDevice, c->stream));
-  PHYS_TRY(h2d(c, c->x, lx, n));
-  PHYS_TRY(h2d(c, c->y, ly, n));
-  PHYS_TRY(h2d(c, c->z, lz, n));
-  PHYS_TRY(flatten_sectors(c, dsx, dsy, dsz, c->x, c->y, c->z, sector_size, bh_quirk));
-  PHYS_TRY(h2d(c, c->vx, vx, n));
-  PHYS_TRY(h2d(c, c->vy, vy, n));
-  PHYS_TRY(h2d(c, c->vz, vz, n));
-  PHYS_TRY(h2d(c, c->m, m, n));
-  PHYS_TRY(h2d(c, c->ax, nullptr, n));
-  PHYS_TRY(h2d(c, c->ay, nullptr, n));
-  PHYS_TRY(h2d(c, c->az, nullptr, n));
-  PHYS_TRY(h2d(c, c->pax, nullptr, n));
-  PHYS_TRY(h2d(c, c->pay, nullptr, n));
-  PHYS_TRY(h2d(c, c->paz, nullptr, n));
+  const void* sec[3] = {sx, sy, sz};
+  const void* src[7] = {lx, ly, lz, vx, vy, vz, m};
+  if (packs(n, 3)) PHYS_TRY(ensure_pinned(c, 8 * 10 * n));
+  PHYS_TRY(copy_rows(c, c->fx, 3, sec, n, 0));
+  PHYS_TRY(copy_rows(c, c->x, 7, src, n, 3 * n));
+  PHYS_TRY(flatten_sectors(c, reinterpret_cast<int64_t*>(c->fx), reinterpret_cast<int64_t*>(c->fy),
+                           reinterpret_cast<int64_t*>(c->fz), c->x, c->y, c->z, sector_size,
+                           bh_quirk));
+  PHYS_TRY(zero_rows(c, c->ax, 6, n));
   PHYS_CUDA(c, cudaStreamSynchronize(c->stream));
   return PHYS_OK;
 }
@@ -758,11 +793,8 @@ int phys_gravity_forces(phys_ctx* c, const phys_params* p, double* fx, double* f
   PHYS_CUDA(c, cudaEventRecord(c->ev[1], c->stream));
   PHYS_TRY(ensure_pinned(c, sizeof(double) * 3 * n));
   double* h = static_cast<double*>(c->h_stage);
-  PHYS_TRY(d2h(c, h, c->fx, n));
-  PHYS_TRY(d2h(c, h + n, c->fy, n));
-  PHYS_TRY(d2h(c, h + 2 * n, c->fz, n));
-  PHYS_CUDA(c, cudaStreamSynchronize(c->stream));
-  int st = finish_status(c);
+  PHYS_TRY(forces_to_host(c, h, n));
+  int st = finish_status(c);  // synchronises
   c->tm.total_ms = ev_ms(c->ev[0], c->ev[1]);
   if (st) return st;
   for (int64_t i = 0; i < n; ++i) {  // Force += computed (gravity.rs:71-73)
@@ -828,8 +860,7 @@ int phys_gravity_accel(phys_ctx* c, const phys_params* p, double* ax, double* ay
   PHYS_TRY(d2h(c, ax, c->ax, c->n));
   PHYS_TRY(d2h(c, ay, c->ay, c->n));
   PHYS_TRY(d2h(c, az, c->az, c->n));
-  PHYS_CUDA(c, cudaStreamSynchronize(c->stream));
-  int st = finish_status(c);
+  int st = finish_status(c);  // synchronises
   c->tm.total_ms = ev_ms(c->ev[0], c->ev[1]);
   return st;
 }
