@@ -434,6 +434,11 @@ int scan_exclusive_i32(phys_ctx* c, const int32_t* in, int32_t* out, int64_t n) 
   if (n <= 0) return PHYS_OK;
   const int64_t nb = ceil_div(n, kScanTile);
   int st = PHYS_OK;
+  if (nb <= 3) {  // one block and one launch: about 1 us per 4096 values, a launch costs 2
+    PHYS_LAUNCH(c, scan_single_kernel, 1, 1024, 0, reinterpret_cast<const uint32_t*>(in),
+                reinterpret_cast<uint32_t*>(out), n, (uint32_t*)nullptr);
+    return PHYS_OK;
+  }
   uint32_t* sums = (uint32_t*)ws_get(c, WS_SCAN_TMP, sizeof(uint32_t) * (nb + 1), &st);
   if (st) return st;
   PHYS_LAUNCH(c, scan_block_sums_kernel, (int)nb, kScanBlock, 0, in, n, sums);

@@ -128,26 +128,28 @@ __global__ void bbox_final_kernel(int nparts, const double* __restrict__ part, d
     amin = fmin(amin, __shfl_xor_sync(0xffffffffu, amin, o));
     amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   }
-  if (lane != 0) return;
-  hdr->min_mass = mmin;
-  hdr->min_abs = amin;
-  hdr->max_abs = amax;
   // extent = max - min; max_extent = x.max(y).max(z); half = max_extent*0.55 + 1
   const double ex = xsub(mx[0], mn[0]), ey = xsub(mx[1], mn[1]), ez = xsub(mx[2], mn[2]);
   const double max_extent = fmax(fmax(ex, ey), ez);
   const double half = xadd(xmul(max_extent, 0.55), 1.0);
+  // child half size h * 0.5 per level (gravity_tree.rs:137): exact, so lane d
+  // scales by 2^-d; the guard depth is the first with d >= 40 or h < 1e-8
+  int guard = INT_MAX;
+  for (int d = lane; d < kMaxLevels; d += 32) {
+    const double h = xmul(half, __hiloint2double((1023 - d) << 20, 0));
+    const double s = xmul(h, 2.0);  // full side length (gravity_tree.rs:192)
+    hdr->s2[d] = xmul(s, s);
+    if (d >= kMaxDepth || h < kMinNodeSize) guard = min(guard, d);
+  }
+  guard = __reduce_min_sync(0xffffffffu, guard);
+  if (lane != 0) return;
+  hdr->min_mass = mmin;
+  hdr->min_abs = amin;
+  hdr->max_abs = amax;
   for (int k = 0; k < 3; ++k) hdr->center[k] = xmul(xadd(mn[k], mx[k]), 0.5);
   hdr->half = half;
   hdr->theta2 = xmul(theta, theta);
-  double h = half;
-  int dstar = -1;
-  for (int d = 0; d < kMaxLevels; ++d) {
-    const double s = xmul(h, 2.0);  // full side length (gravity_tree.rs:192)
-    hdr->s2[d] = xmul(s, s);
-    if (dstar < 0 && (d >= kMaxDepth || h < kMinNodeSize)) dstar = d;
-    h = xmul(h, 0.5);  // child half size (gravity_tree.rs:137)
-  }
-  hdr->dstar = dstar;
+  hdr->dstar = guard;
   hdr->nonfinite = (*status & kStatNonfinite) ? 1 : 0;
 }
 
@@ -244,6 +246,19 @@ __global__ void run_fixup_kernel(int64_t n, const uint64_t* __restrict__ hs,
   }
 }
 
+// Double-float forms of a body: hi and lo parts, and the paired layout.
+__device__ __forceinline__ void split_body(double4 b, float4& h, float4& l, Body32x2& q) {
+  split_df(b.x, h.x, l.x);
+  split_df(b.y, h.y, l.y);
+  split_df(b.z, h.z, l.z);
+  h.w = (float)b.w;
+  l.w = 0.f;
+  q.q0 = make_float4(h.x, h.x, h.y, h.y);
+  q.q1 = make_float4(h.z, h.z, h.w, h.w);
+  q.q2 = make_float4(l.x, l.x, l.y, l.y);
+  q.q3 = make_float4(l.z, l.z, 0.f, 0.f);
+}
+
 __global__ void __launch_bounds__(kBlock)
 gather_sorted_kernel(int64_t n, const uint32_t* __restrict__ perm, const uint64_t* __restrict__ klo,
                      const double4* __restrict__ rec, uint64_t* __restrict__ lo_s,
@@ -260,23 +275,120 @@ gather_sorted_kernel(int64_t n, const uint32_t* __restrict__ perm, const uint64_
     body64[p] = b;
     if (body_hi) {
       float4 h, l;
-      split_df(b.x, h.x, l.x);
-      split_df(b.y, h.y, l.y);
-      split_df(b.z, h.z, l.z);
-      h.w = (float)b.w;
-      l.w = 0.f;
+      Body32x2 q;
+      split_body(b, h, l, q);
       body_hi[p] = h;
       body_lo[p] = l;
-      if (body2) {
-        Body32x2 q;
-        q.q0 = make_float4(h.x, h.x, h.y, h.y);
-        q.q1 = make_float4(h.z, h.z, h.w, h.w);
-        q.q2 = make_float4(l.x, l.x, l.y, l.y);
-        q.q3 = make_float4(l.z, l.z, 0.f, 0.f);
-        body2[p] = q;
-      }
+      if (body2) body2[p] = q;
     }
   }
+}
+
+// The sorted form of few bodies in one kernel: body i's place is the number of
+// bodies before it in (hi, lo, index), counted against every key.  A block
+// counts for 32 bodies, each of its warps over an eighth of the keys (shared
+// memory, broadcast); bodies that share a whole hi key (21 octants) compare
+// lo and index in a second look.  Quadratic, but one launch in place of the
+// radix sort's eleven: 8 against 50 us at 1000 bodies, 20.5 against 59.5 at
+// 5003, 57 against 65 at 12288, 96 against 64 at 16384 - hence the limit.
+constexpr int64_t kRankBodies = 12288;
+constexpr int kRankTile = 1024;
+
+__global__ void __launch_bounds__(kBlock)
+rank_kernel(int n, const uint64_t* __restrict__ khi, const uint64_t* __restrict__ klo,
+            const double4* __restrict__ rec, uint64_t* __restrict__ hs,
+            uint64_t* __restrict__ lo_s, uint32_t* __restrict__ perm,
+            double4* __restrict__ body64, float4* __restrict__ body_hi,
+            float4* __restrict__ body_lo, Body32x2* __restrict__ body2) {
+  wait_for_previous();
+  __shared__ __align__(16) uint64_t tile[kRankTile];
+  __shared__ int less[kBlock / 32][32], same[kBlock / 32][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  const uint64_t key = i < n ? khi[i] : 0;
+  constexpr int kPart = kRankTile / (kBlock / 32);
+  int lt = 0, eq = 0;
+  for (int base = 0; base < n; base += kRankTile) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < kRankTile; k += kBlock)
+      tile[k] = base + k < n ? khi[base + k] : ~0ull;  // above every key (63 bits)
+    __syncthreads();
+    const ulonglong2* t = reinterpret_cast<const ulonglong2*>(tile + w * kPart);
+#pragma unroll 8
+    for (int k = 0; k < kPart / 2; ++k) {
+      const ulonglong2 v = t[k];
+      lt += v.x < key;
+      eq += v.x == key;
+      lt += v.y < key;
+      eq += v.y == key;
+    }
+  }
+  less[w][lane] = lt;
+  same[w][lane] = eq;
+  __syncthreads();
+  if (w != 0 || i >= n) return;
+  int at = 0, twins = 0;
+  for (int k = 0; k < kBlock / 32; ++k) {
+    at += less[k][lane];
+    twins += same[k][lane];
+  }
+  const uint64_t lo = klo[i];
+  if (twins > 1)
+    for (int j = 0; j < n; ++j)
+      if (khi[j] == key) at += klo[j] < lo || (klo[j] == lo && j < i);
+  perm[at] = (uint32_t)i;
+  hs[at] = key;
+  lo_s[at] = lo;
+  const double4 b = rec[i];
+  body64[at] = b;
+  if (body_hi) {
+    float4 h, l;
+    Body32x2 q;
+    split_body(b, h, l, q);
+    body_hi[at] = h;
+    body_lo[at] = l;
+    if (body2) body2[at] = q;
+  }
+}
+
+// Breadth-first order of few nodes the same way: by (depth, pre-order id),
+// which are distinct.  In place of a key kernel, one radix pass and the
+// inversion: the tree phase takes 98 against 108 us at 2156 nodes, 122 against
+// 125 at 5256, 121 against 118 at 6874.
+constexpr int64_t kRankNodes = 6144;
+
+__global__ void __launch_bounds__(kBlock)
+depth_rank_kernel(int nnodes, const int4* __restrict__ link, uint32_t* __restrict__ bfs2pre,
+                  int32_t* __restrict__ pre2bfs) {
+  wait_for_previous();
+  __shared__ __align__(16) uint32_t tile[kRankTile];
+  __shared__ int less[kBlock / 32][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  auto key_of = [&](int k) { return (uint32_t)(link[k].w & kMetaDepth) << 16 | (uint32_t)k; };
+  static_assert(kRankNodes <= 65536, "16 bits of node id");
+  const uint32_t key = i < nnodes ? key_of(i) : 0;
+  constexpr int kPart = kRankTile / (kBlock / 32);
+  int lt = 0;
+  for (int base = 0; base < nnodes; base += kRankTile) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < kRankTile; k += kBlock)
+      tile[k] = base + k < nnodes ? key_of(base + k) : 0xffffffffu;
+    __syncthreads();
+    const uint4* t = reinterpret_cast<const uint4*>(tile + w * kPart);
+#pragma unroll 8
+    for (int k = 0; k < kPart / 4; ++k) {
+      const uint4 v = t[k];
+      lt += (v.x < key) + (v.y < key) + (v.z < key) + (v.w < key);
+    }
+  }
+  less[w][lane] = lt;
+  __syncthreads();
+  if (w != 0 || i >= nnodes) return;
+  int at = 0;
+  for (int k = 0; k < kBlock / 32; ++k) at += less[k][lane];
+  bfs2pre[at] = (uint32_t)i;
+  pre2bfs[i] = at;
 }
 
 __device__ __forceinline__ int lcp_octants(uint64_t ha, uint64_t la, uint64_t hb, uint64_t lb) {
@@ -470,10 +582,16 @@ emit_pruned_kernel(int64_t n, const uint64_t* __restrict__ hs, const uint64_t* _
   }
 }
 
-// parent / number of children, by walking each internal node's child chain.
+// parent / number / ids of the children, by walking each internal node's
+// child chain once: the kernels after this one read a node's children with
+// independent loads instead of hopping along the chain again.
+struct __align__(16) Kids {
+  int32_t id[8];
+};
+
 __global__ void __launch_bounds__(kBlock)
 children_kernel(int64_t nnodes, const int4* __restrict__ link, int32_t* __restrict__ parent,
-                int32_t* __restrict__ nchild, int32_t* status) {
+                int32_t* __restrict__ nchild, Kids* __restrict__ kids, int32_t* status) {
   wait_for_previous();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnodes;
        k += (int64_t)gridDim.x * blockDim.x) {
@@ -484,6 +602,7 @@ children_kernel(int64_t nnodes, const int4* __restrict__ link, int32_t* __restri
       int32_t ch = (int32_t)k + 1;
       while (ch < lk.x && cc < 8) {  // an octree cell has at most 8 children
         parent[ch] = (int32_t)k;
+        if (kids) kids[k].id[cc] = ch;
         const int32_t nx = link[ch].x;
         if (nx <= ch) break;
         ch = nx;
@@ -500,6 +619,10 @@ children_kernel(int64_t nnodes, const int4* __restrict__ link, int32_t* __restri
 // bodies in key order, internal cells over their children in octant order
 // (fixed order: deterministic), propagated bottom-up by the last-arriving
 // child.  Differs from the reference's insertion-order running mean by ulps.
+// Bound by the chain of levels, each an atomic and the loads of up to eight
+// children's sums; those go out together (ids from children_kernel): 27 us
+// against 35 at 5003 bodies, 58 against 72 at 2^20 when each child was found
+// from the one before it.
 // ---------------------------------------------------------------------------
 // arrive[] += 1 with acquire-release order at GPU scope; returns the old
 // count.  Orders the caller's earlier stores before it and later loads after
@@ -513,8 +636,8 @@ __device__ __forceinline__ int32_t arrive_acq_rel(int32_t* p) {
 __global__ void __launch_bounds__(kBlock)
 com_upward_kernel(int64_t nnodes, const int4* __restrict__ link,
                   const int32_t* __restrict__ parent, const int32_t* __restrict__ nchild,
-                  int32_t* __restrict__ arrive, const double4* __restrict__ body64,
-                  double4* __restrict__ sums, int32_t* status) {
+                  const Kids* __restrict__ kids, int32_t* __restrict__ arrive,
+                  const double4* __restrict__ body64, double4* __restrict__ sums, int32_t* status) {
   wait_for_previous();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnodes;
        k += (int64_t)gridDim.x * blockDim.x) {
@@ -538,17 +661,27 @@ com_upward_kernel(int64_t nnodes, const int4* __restrict__ link,
       }
       // release: this child's sums are visible to whoever arrives last;
       // acquire: the last arrival sees every sibling's sums
-      if (arrive_acq_rel(&arrive[par]) != nchild[par] - 1) break;
-      const int32_t stop = link[par].x;
+      const int nc = nchild[par];
+      const int4 ka = *reinterpret_cast<const int4*>(&kids[par].id[0]);
+      const int4 kb = *reinterpret_cast<const int4*>(&kids[par].id[4]);
+      if (arrive_acq_rel(&arrive[par]) != nc - 1) break;
+      const int32_t ids[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+      double2 v0[8], v1[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const double2* sp = reinterpret_cast<const double2*>(&sums[i < nc ? ids[i] : cur]);
+        v0[i] = __ldcg(sp);  // L2: written by other threads
+        v1[i] = __ldcg(sp + 1);
+      }
       double ax = 0.0, ay = 0.0, az = 0.0, am = 0.0;
-      int guard = 0;
-      for (int32_t ch = par + 1; ch < stop && guard < 8; ch = link[ch].x, ++guard) {
-        const double2* sp = reinterpret_cast<const double2*>(&sums[ch]);
-        const double2 v0 = __ldcg(sp), v1 = __ldcg(sp + 1);  // L2: written by other threads
-        ax += v0.x;
-        ay += v0.y;
-        az += v1.x;
-        am += v1.y;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (i < nc) {
+          ax += v0[i].x;
+          ay += v0[i].y;
+          az += v1[i].x;
+          am += v1[i].y;
+        }
       }
       sums[par] = make_double4(ax, ay, az, am);
       cur = par;
@@ -928,8 +1061,8 @@ static_assert(kGroupBuild >= 1 && kGroupBuild <= kGroupMax, "group size");
 template <bool kEmit>
 __global__ void group_kernel(int64_t nnodes, const uint32_t* __restrict__ bfs2pre,
                              const int4* __restrict__ link, const int32_t* __restrict__ nchild,
-                             const uint64_t* __restrict__ hs, const uint64_t* __restrict__ klo,
-                             const uint32_t* __restrict__ perm,
+                             const Kids* __restrict__ kids, const uint64_t* __restrict__ hs,
+                             const uint64_t* __restrict__ klo, const uint32_t* __restrict__ perm,
                              int32_t* __restrict__ cnt, const int32_t* __restrict__ off,
                              int2* __restrict__ out, int64_t cap, const int32_t* status) {
   wait_for_previous();
@@ -953,15 +1086,22 @@ __global__ void group_kernel(int64_t nnodes, const uint32_t* __restrict__ bfs2pr
     } else if (lk.w & kMetaLeaf) {
       for (int b = lk.y; b < lk.z; b += kGroupBuild) put(b, min(b + kGroupBuild, lk.z));
     } else {
-      int c = (int)k + 1, rb = -1, re = -1, ob = 0;
+      int rb = -1, re = -1, ob = 0;
       const int nc = nchild[k];
       const int d = lk.w & kMetaDepth;
-      for (int i = 0; i < nc && c < nnodes; ++i) {
-        const int4 lc = link[c];
-        const int cc = lc.z - lc.y;
-        // the child's octant: digit d of its first body's descent key
-        const int oc = d < 21 ? (int)((hs[lc.y] >> (60 - 3 * d)) & 7)
-                              : (int)((klo[perm[lc.y]] >> (54 - 3 * (d - 21))) & 7);
+      int4 ch[8];
+      int oct[8];  // the child's octant: digit d of its first body's descent key
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ch[i] = link[i < nc ? kids[k].id[i] : k];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        oct[i] = d < 21 ? (int)((hs[ch[i].y] >> (60 - 3 * d)) & 7)
+                        : (int)((klo[perm[ch[i].y]] >> (54 - 3 * (d - 21))) & 7);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (i >= nc) break;
+        const int4 lc = ch[i];
+        const int cc = lc.z - lc.y, oc = oct[i];
         if (cc > kGroupBuild) {
           if (rb >= 0) put(rb, re);
           rb = -1;
@@ -973,7 +1113,6 @@ __global__ void group_kernel(int64_t nnodes, const uint32_t* __restrict__ bfs2pr
           re = lc.z;
           ob = oc;
         }
-        c = lc.x;
       }
       if (rb >= 0) put(rb, re);
     }
@@ -1035,14 +1174,21 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
   PHYS_LAUNCH(c, keys_kernel, grid_for(n), kBlock, 0, n, c->x, c->y, c->z, c->m, c->d_hdr, khi,
               klo, idx, rec);
   PHYS_CUDA(c, cudaEventRecord(c->ev[4], c->stream));
-  bool in_alt = false;
-  PHYS_TRY(radix_sort_u64(c, khi, idx, khi_alt, idx_alt, n, 0, 64, &in_alt));
-  uint64_t* hs = in_alt ? khi_alt : khi;
-  uint32_t* perm = in_alt ? idx_alt : idx;
-  uint32_t* spare = in_alt ? idx : idx_alt;
-  PHYS_LAUNCH(c, run_fixup_kernel, grid_for(n), kBlock, 0, n, hs, perm, klo, spare, c->d_status);
-  PHYS_LAUNCH(c, gather_sorted_kernel, grid_for(n), kBlock, 0, n, perm, klo, rec, lo_s, body64,
-              body_hi, body_lo, body2, c->d_status);
+  uint64_t* hs = khi_alt;
+  uint32_t* perm = idx_alt;
+  if (n <= kRankBodies) {
+    PHYS_LAUNCH(c, rank_kernel, (int)ceil_div(n, 32), kBlock, 0, (int)n, khi, klo, rec, hs, lo_s,
+                perm, body64, body_hi, body_lo, body2);
+  } else {
+    bool in_alt = false;
+    PHYS_TRY(radix_sort_u64(c, khi, idx, khi_alt, idx_alt, n, 0, 64, &in_alt));
+    hs = in_alt ? khi_alt : khi;
+    perm = in_alt ? idx_alt : idx;
+    uint32_t* spare = in_alt ? idx : idx_alt;
+    PHYS_LAUNCH(c, run_fixup_kernel, grid_for(n), kBlock, 0, n, hs, perm, klo, spare, c->d_status);
+    PHYS_LAUNCH(c, gather_sorted_kernel, grid_for(n), kBlock, 0, n, perm, klo, rec, lo_s, body64,
+                body_hi, body_lo, body2, c->d_status);
+  }
   PHYS_CUDA(c, cudaEventRecord(c->ev[5], c->stream));
   PHYS_LAUNCH(c, lcp_count_kernel, grid_for(n + 1), kBlock, 0, n, hs, lo_s, c->d_hdr, L, cnt);
   // bucket leaves: count only the cells that survive (no full tree)
@@ -1086,7 +1232,17 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     PHYS_LAUNCH(c, emit_nodes_kernel, grid_for(n), kBlock, 0, n, hs, lo_s, L, cnt, first,
                 c->d_hdr, link);
   }
-  PHYS_LAUNCH(c, children_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, parent, nchild,
+  // child ids, read up to the group list; their slot then takes the records
+  // that finalize_kernel or gnode_kernel writes, and is sized for those
+  Kids* kids = nullptr;
+  if (!exact) {
+    const size_t later = need_f32 ? sizeof(Rec32x2) : need_group ? sizeof(double4) : sizeof(Rec64);
+    static_assert(sizeof(Kids) <= sizeof(double4), "shared slot");
+    char* slot = nullptr;
+    PHYS_TRY(ws_alloc(c, need_f32 ? WS_NODE_HI : WS_NODE_LO, nnodes * (int64_t)later, &slot));
+    kids = reinterpret_cast<Kids*>(slot);
+  }
+  PHYS_LAUNCH(c, children_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, parent, nchild, kids,
               c->d_status);
   double4* mc = nullptr;
   PHYS_TRY(ws_alloc(c, WS_NODE_S, nnodes, &mc));
@@ -1131,7 +1287,7 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
   } else {
     PHYS_CUDA(c, cudaMemsetAsync(arrive, 0, sizeof(int32_t) * (nnodes + 1), c->stream));
     PHYS_LAUNCH(c, com_upward_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, parent, nchild,
-                arrive, body64, mc, c->d_status);
+                kids, arrive, body64, mc, c->d_status);
   }
   double4* rec64 = nullptr;
   RecX* wx = nullptr;
@@ -1185,17 +1341,18 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     PHYS_TRY(ws_alloc(c, WS_NEWID, nnodes, &dv_alt));
     PHYS_TRY(ws_alloc(c, WS_EOFF, nnodes + 1, &pre2bfs));
     PHYS_TRY(ws_alloc(c, WS_ENS5, nnodes, &g));
-    PHYS_TRY(ws_alloc(c, WS_NODE_LO, nnodes, &gsrc));
-    PHYS_LAUNCH(c, depth_key_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, dk, dv);
-    bool alt = false;
-    PHYS_TRY(radix_sort_u64(c, dk, dv, dk_alt, dv_alt, nnodes, 0, 8, &alt));
-    const uint32_t* bfs2pre = alt ? dv_alt : dv;
-    PHYS_LAUNCH(c, invert_kernel, grid_for(nnodes), kBlock, 0, nnodes, bfs2pre, pre2bfs,
-                c->d_status);
-    PHYS_LAUNCH(c, gnode_kernel, grid_for(nnodes), kBlock, 0, nnodes, bfs2pre, pre2bfs, link, mc,
-                nchild, p->leaf_cap, body64, c->d_hdr, g, gsrc, c->d_status);
-    t->gnode = g;
-    t->gsrc = gsrc;
+    uint32_t* bfs2pre = dv;
+    if (nnodes <= kRankNodes) {
+      PHYS_LAUNCH(c, depth_rank_kernel, (int)ceil_div(nnodes, 32), kBlock, 0, (int)nnodes, link,
+                  bfs2pre, pre2bfs);
+    } else {
+      PHYS_LAUNCH(c, depth_key_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, dk, dv);
+      bool alt = false;
+      PHYS_TRY(radix_sort_u64(c, dk, dv, dk_alt, dv_alt, nnodes, 0, 8, &alt));
+      bfs2pre = alt ? dv_alt : dv;
+      PHYS_LAUNCH(c, invert_kernel, grid_for(nnodes), kBlock, 0, nnodes, bfs2pre, pre2bfs,
+                  c->d_status);
+    }
     int32_t *gcnt = nullptr, *goff = nullptr, *gctr = nullptr;
     int2* groups = nullptr;
     PHYS_TRY(ws_alloc(c, WS_NCOUNT, nnodes + 1, &gcnt));
@@ -1203,10 +1360,15 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     PHYS_TRY(ws_alloc(c, WS_GROUPS, 2 * n, &groups));  // groups, then re-queued subgroups
     PHYS_TRY(ws_alloc(c, WS_GROUP_CTR, 8, &gctr));
     PHYS_LAUNCH(c, group_kernel<false>, grid_for(nnodes + 1), kBlock, 0, nnodes, bfs2pre, link,
-                nchild, hs, klo, perm, gcnt, goff, groups, n, c->d_status);
+                nchild, kids, hs, klo, perm, gcnt, goff, groups, n, c->d_status);
     PHYS_TRY(scan_exclusive_i32(c, gcnt, goff, nnodes + 1));
     PHYS_LAUNCH(c, group_kernel<true>, grid_for(nnodes + 1), kBlock, 0, nnodes, bfs2pre, link,
-                nchild, hs, klo, perm, gcnt, goff, groups, n, c->d_status);
+                nchild, kids, hs, klo, perm, gcnt, goff, groups, n, c->d_status);
+    PHYS_TRY(ws_alloc(c, WS_NODE_LO, nnodes, &gsrc));  // the child ids end here
+    PHYS_LAUNCH(c, gnode_kernel, grid_for(nnodes), kBlock, 0, nnodes, bfs2pre, pre2bfs, link, mc,
+                nchild, p->leaf_cap, body64, c->d_hdr, g, gsrc, c->d_status);
+    t->gnode = g;
+    t->gsrc = gsrc;
     t->groups = groups;
     t->ngroups = goff + nnodes;
     t->group_ctr = gctr;
