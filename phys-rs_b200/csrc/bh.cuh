@@ -77,13 +77,9 @@ struct __align__(16) Rec64 {
   int4 l;
 };
 
-// Exact walk, traversal record: the node's position relative to the root
-// cube's centre in units of its half size (f32: decides almost every opening,
-// the f64 record the rest), the skip pointer (int bits in w), the depth and
-// flags of `link` and the stored body of a leaf.
-struct __align__(16) RecX {
-  float4 a;  // x, y, z, next
-  int4 b;    // meta, stored body (leaf), -, -
+// A cell's children in octant order, -1 beyond the last.
+struct __align__(16) Kids {
+  int32_t id[8];
 };
 // The exact walk's split over subtrees: the cells of more than `most` bodies
 // (upper cells) and their other children (tasks), in pre-order.
@@ -101,7 +97,12 @@ struct BhTree {
   int leaf_cap = 1;
   const int4* link = nullptr;
   const double4* rec64 = nullptr;     // exact walk: record per node (with `link`)
-  const RecX* wx = nullptr;           // exact walk: traversal record per node
+  // exact walk, traversal record per node: position relative to the root
+  // cube's centre in units of its half size (f32: decides almost every
+  // opening, the f64 record the rest), for a leaf the stored body in x; the
+  // depth and flags of `link` in w (int bits)
+  const float4* wx = nullptr;
+  const Kids* kids = nullptr;
   TopTree top;                        // exact walk split over subtrees (max_tasks > 0)
   const Rec32* w32 = nullptr;         // F32C walk records
   const Rec32x2* w32x2 = nullptr;     // F32C paired walk records

@@ -585,10 +585,6 @@ emit_pruned_kernel(int64_t n, const uint64_t* __restrict__ hs, const uint64_t* _
 // parent / number / ids of the children, by walking each internal node's
 // child chain once: the kernels after this one read a node's children with
 // independent loads instead of hopping along the chain again.
-struct __align__(16) Kids {
-  int32_t id[8];
-};
-
 __global__ void __launch_bounds__(kBlock)
 children_kernel(int64_t nnodes, const int4* __restrict__ link, int32_t* __restrict__ parent,
                 int32_t* __restrict__ nchild, Kids* __restrict__ kids, int32_t* status) {
@@ -602,13 +598,14 @@ children_kernel(int64_t nnodes, const int4* __restrict__ link, int32_t* __restri
       int32_t ch = (int32_t)k + 1;
       while (ch < lk.x && cc < 8) {  // an octree cell has at most 8 children
         parent[ch] = (int32_t)k;
-        if (kids) kids[k].id[cc] = ch;
+        kids[k].id[cc] = ch;
         const int32_t nx = link[ch].x;
         if (nx <= ch) break;
         ch = nx;
         ++cc;
       }
       if (ch < lk.x) atomicOr(status, kStatOverflow);
+      for (int i = cc; i < 8; ++i) kids[k].id[i] = -1;
     }
     nchild[k] = cc;
   }
@@ -872,7 +869,7 @@ debug_divide_kernel(int64_t n, const double* __restrict__ a, const double* __res
 __global__ void __launch_bounds__(kBlock)
 finalize_kernel(int64_t nnodes, int4* __restrict__ link, double4* __restrict__ mc, int sums,
                 int leaf_cap, const double4* __restrict__ body64, const TreeHeader* __restrict__ hdr,
-                double4* __restrict__ rec64, RecX* __restrict__ wx, Rec32* __restrict__ w32,
+                double4* __restrict__ rec64, float4* __restrict__ wx, Rec32* __restrict__ w32,
                 Rec64* __restrict__ w64, Rec32x2* __restrict__ w32x2) {
   wait_for_previous();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnodes;
@@ -903,14 +900,11 @@ finalize_kernel(int64_t nnodes, int4* __restrict__ link, double4* __restrict__ m
     if (self >= 0) r = body64[self];
     if (rec64) rec64[k] = r;
     if (wx) {
-      // the root's own position is left to the f64 test (it may be anything
-      // when the total mass is not positive)
       const double ih = 1.0 / hdr->half;
-      RecX o;
-      o.a = make_float4((float)((r.x - hdr->center[0]) * ih), (float)((r.y - hdr->center[1]) * ih),
-                        (float)((r.z - hdr->center[2]) * ih), __int_as_float(lk.x));
-      if (k == 0) o.a.x = __int_as_float(0x7fc00000);
-      o.b = make_int4(lk.w, leaf ? (cntb == 1 ? lk.y : lk.z - 1) : -1, 0, 0);
+      float4 o = make_float4((float)((r.x - hdr->center[0]) * ih),
+                             (float)((r.y - hdr->center[1]) * ih),
+                             (float)((r.z - hdr->center[2]) * ih), __int_as_float(lk.w));
+      if (leaf) o.x = __int_as_float(cntb == 1 ? lk.y : lk.z - 1);
       wx[k] = o;
     }
     int wmeta = (gate || k == 0) ? d : kWSkip;
@@ -1232,20 +1226,26 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     PHYS_LAUNCH(c, emit_nodes_kernel, grid_for(n), kBlock, 0, n, hs, lo_s, L, cnt, first,
                 c->d_hdr, link);
   }
-  // child ids, read up to the group list; their slot then takes the records
-  // that finalize_kernel or gnode_kernel writes, and is sized for those
+  // child ids.  Without the exact form they are read up to the group list;
+  // their slot then takes the records that finalize_kernel or gnode_kernel
+  // writes, and is sized for those.
   Kids* kids = nullptr;
+  auto children = [&]() {
+    PHYS_LAUNCH(c, children_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, parent, nchild,
+                kids, c->d_status);
+    return (int)PHYS_OK;
+  };
   if (!exact) {
     const size_t later = need_f32 ? sizeof(Rec32x2) : need_group ? sizeof(double4) : sizeof(Rec64);
     static_assert(sizeof(Kids) <= sizeof(double4), "shared slot");
     char* slot = nullptr;
     PHYS_TRY(ws_alloc(c, need_f32 ? WS_NODE_HI : WS_NODE_LO, nnodes * (int64_t)later, &slot));
     kids = reinterpret_cast<Kids*>(slot);
+    PHYS_TRY(children());
   }
-  PHYS_LAUNCH(c, children_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, parent, nchild, kids,
-              c->d_status);
   double4* mc = nullptr;
   PHYS_TRY(ws_alloc(c, WS_NODE_S, nnodes, &mc));
+  float4* wx = nullptr;
   if (exact) {
     int32_t* ncnt = nullptr;
     PHYS_TRY(ws_alloc(c, WS_KEEP, nnodes + 1, &ncnt));
@@ -1259,10 +1259,12 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     const int64_t total = (uint32_t)hsm[0];
     if (total <= 0 || total >= (int64_t(1) << 31))
       return fail(c, PHYS_ERR_ARG, "exact centre of mass needs < 2^31 (cell, body) pairs");
+    // the pairs' slots take the child ids and the walk's records afterwards
+    const int64_t room = std::max(total, nnodes * (int64_t)(sizeof(Kids) / sizeof(uint64_t)));
     uint64_t* ent = nullptr;
-    PHYS_TRY(ws_alloc(c, WS_ENTRIES, total, &ent));
+    PHYS_TRY(ws_alloc(c, WS_ENTRIES, room, &ent));
     uint64_t* ent_alt = nullptr;
-    PHYS_TRY(ws_alloc(c, WS_ENTRIES_ALT, total, &ent_alt));
+    PHYS_TRY(ws_alloc(c, WS_ENTRIES_ALT, room, &ent_alt));
     PHYS_LAUNCH(c, expand_kernel, grid_for(total), kBlock, 0, total, nnodes, eoff, link, perm, ent);
     int bits_b = 1, bits_n = 1;
     while ((int64_t(1) << bits_b) < n) ++bits_b;
@@ -1284,13 +1286,15 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     PHYS_LAUNCH(c, com_recurrence_kernel, grid_for(nnodes, 128, 1 << 30), 128, 0, nnodes, eoff, eb,
                 mc, link, c->d_hdr, full_com ? 0 : 1, com_long_chain(n), longs, c->d_status);
     PHYS_TRY(com_long_cells(c, n, nnodes, total, eoff, eb, link, c->d_hdr, longs, mc));
+    kids = reinterpret_cast<Kids*>(ent);
+    wx = reinterpret_cast<float4*>(ent_alt);
+    PHYS_TRY(children());
   } else {
     PHYS_CUDA(c, cudaMemsetAsync(arrive, 0, sizeof(int32_t) * (nnodes + 1), c->stream));
     PHYS_LAUNCH(c, com_upward_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, parent, nchild,
                 kids, arrive, body64, mc, c->d_status);
   }
   double4* rec64 = nullptr;
-  RecX* wx = nullptr;
   TopTree top;
   Rec32* w32 = nullptr;
   Rec64* w64 = nullptr;
@@ -1299,7 +1303,6 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     PHYS_TRY(ws_alloc(c, WS_NODE_PM, nnodes, &rec64));
     top.max_tasks = exact_walk_tasks(c, n);
     if (top.max_tasks > 0) {
-      PHYS_TRY(ws_alloc(c, WS_NODE_HI, nnodes, &wx));
       int32_t *cnt2 = nullptr, *off2 = nullptr, *lists = nullptr;
       top.max_top = 4096;
       PHYS_TRY(ws_alloc(c, WS_NCOUNT, nnodes + 1, &cnt2));
@@ -1379,6 +1382,7 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
   t->link = link;
   t->rec64 = rec64;
   t->wx = wx;
+  t->kids = kids;
   t->top = top;
   t->w32 = w32;
   t->w64 = w64;

@@ -21,6 +21,8 @@
 //   F32C       f32 pair terms on double-float relative coordinates
 //              r = (hi_j - hi_i) + (lo_j - lo_i); f32 partial sums folded
 //              into a (hi, lo) accumulator with two-sum every 16 nodes.
+#include <type_traits>
+
 #include "bh.cuh"
 
 #ifndef WALK_BRANCHY
@@ -375,17 +377,24 @@ walk2_kernel(int q64, int n, int nnodes, const Rec32x2* __restrict__ w, const Bo
 // ---------------------------------------------------------------------------
 // F64_EXACT walk (leaf capacity 1).
 //
-// The traversal only decides: a node that some lane takes (a monopole or a
-// stored body) becomes an entry of the warp's queue in shared memory, with
-// the mask of those lanes, the level that the open partial sums close to
-// before it and its own level.  A full queue is evaluated kXU entries at a
-// time: every lane forms the weights (exact_scale, independent chains, the
-// node's record read once for the warp), then the terms are added in order,
-// the masked lanes' only.  Levels are opened and closed by the warp's path
-// for all lanes at once: a lane that did not open a cell has +0 in its level,
-// and adding that changes nothing.  The deepest level's sum is in registers,
-// the ones around it in local memory; closing a level adds it to the one
-// above, as the reference's nested sums do.
+// A warp walks for its 32 targets together.  The traversal only decides: a
+// node that some target takes (a monopole or a stored body) becomes an entry
+// of the warp's queue in shared memory, in pre-order, with the mask of those
+// lanes and the levels that the open partial sums close to and open to before
+// it.  A full queue is evaluated kXU entries at a time: every lane forms the
+// weights (exact_scale, independent chains), then the terms are added in
+// order, 0 for the lanes outside the mask.  Levels are opened and closed by
+// the warp's path for all lanes at once: a lane that did not open a cell has
+// +0 in its level, and adding that changes nothing.  The deepest level's sum
+// is in registers, the ones around it in local memory; closing a level adds it
+// to the one above, as the reference's nested sums do.
+//
+// The traversal works on 32 cells at a time, a cell per lane: the children of
+// up to four opened cells of one depth.  Each is first tested against the box
+// of the warp's targets, nearest and farthest point; the f32 operations are
+// the ones of a single target's test and monotone, so a cell that all targets
+// take or all open is found without looking at them.  Only the others (one in
+// six) are tested per target.
 //
 // Opening is decided in f32 on coordinates relative to the root cube: each
 // coordinate is within 2^-25 of its value, their difference within 2^-23, so
@@ -395,15 +404,24 @@ walk2_kernel(int q64, int n, int nnodes, const Rec32x2* __restrict__ w, const Bo
 // may then lie outside the cube), the warp takes the reference's f64 test.
 //
 // Few targets would leave most of the chip idle behind the longest walk, so
-// the children of the cells of more than n/8 bodies become tasks of their own
-// (grid.y; n/16 to n/64 make more tasks than they save walking: 10 000 bodies
-// 0.44 ms against 0.45, 0.55 and 0.68), each leaving its cell's contribution to each target in `part`;
-// exact_combine_kernel walks the cells above and sums them with the
-// reference's nesting.  Bound by the issue of the traversal and of the terms,
-// about 125 instructions per visit and warp, 37 of them on the FP64 pipe.
+// up to 65536 of them are split: the children of the cells of more than n/8
+// bodies become tasks of their own (grid.y; n/16 to n/64 make more tasks than
+// they save walking), each leaving its cell's contribution to each target in
+// `part`; exact_combine_kernel walks the cells above and sums them with the
+// reference's nesting.  Split against whole walks: 0.32 / 0.96 ms at 10 000
+// bodies, 0.86 / 1.21 at 32768, 1.3 / 1.54 at 65536.
+//
+// Bound by the terms: 3300 entries a warp at 300 000 bodies (2100 per target),
+// 38 FP64 instructions and about as many others each, at 55 % of the FP64
+// pipe; without them the traversal takes 1.1 of 5.0 ms.  Two entries at a time
+// and 24 warps an SM do best on a full chip (four: 17.3 ms at 2^20), four with
+// 16 warps when the tasks' tails show (0.32 against 0.34 ms at 10 000).  One
+// walk per target, a node per step and its term evaluated in place, took 19.8
+// ms at 2^20 bodies against 15.5, and 0.44 against 0.32 at 10 000 (split, a
+// node per step).
 // ---------------------------------------------------------------------------
+constexpr unsigned kFull = 0xffffffffu;
 constexpr int kXQ = 32;  // queue entries per warp
-constexpr int kXU = 4;   // entries evaluated together
 constexpr float kXBand = 4e-7f;
 
 // Whether every pair of an evaluation is in exact_scale's range: masses of
@@ -429,9 +447,10 @@ __device__ __forceinline__ double exact_weight(const ExactTarget& t, double4 s, 
   return kFast ? exact_scale(a, s2) : exact_scale_ieee(a, s2);
 }
 
-// The nested sums of one target: the deepest level with a term in registers.
+// The nested sums of one target: the deepest level with a term in registers,
+// the levels around it in an array of the caller's (one struct with the array
+// inside would be written back to local memory after every term).
 struct NestedSum {
-  double st[kMaxLevels + 1][3];
   double x, y, z;
   int d;
   __device__ __forceinline__ void init(int depth) {
@@ -439,7 +458,8 @@ struct NestedSum {
     d = depth;
   }
   // close the levels below m
-  __device__ __forceinline__ void close_to(int m) {
+  __device__ __forceinline__ void close_to(int m, double (*st)[3]) {
+#pragma unroll 1
     while (d > m) {
       --d;
       x = xadd(st[d][0], x);
@@ -448,7 +468,8 @@ struct NestedSum {
     }
   }
   // open levels up to depth, at 0
-  __device__ __forceinline__ void open_to(int depth) {
+  __device__ __forceinline__ void open_to(int depth, double (*st)[3]) {
+#pragma unroll 1
     while (d < depth) {
       st[d][0] = x;
       st[d][1] = y;
@@ -484,17 +505,44 @@ __device__ __forceinline__ int top_tasks(const TopTree& top) {
   return nt <= top.max_tasks && (c & 0xffff) <= top.max_top ? nt : 1;
 }
 
-__global__ void __launch_bounds__(kWalkBlock, 4)
-walk_task_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const RecX* __restrict__ wx,
-                 const double4* __restrict__ rec64, const double4* __restrict__ body64,
-                 const TreeHeader* __restrict__ hdr, TopTree top, double G, double eps2,
-                 double* __restrict__ part, unsigned long long* counter, int32_t* status) {
+// Force -> output of one target (a = F / m unless the force is wanted).
+__device__ __forceinline__ void exact_store(double fx, double fy, double fz, double mi,
+                                            uint32_t i, int want_force, double* ox, double* oy,
+                                            double* oz, int32_t* status) {
+  if (!want_force) {  // a = F / m (integrators.rs:115)
+    fx = xdiv(fx, mi);
+    fy = xdiv(fy, mi);
+    fz = xdiv(fz, mi);
+  }
+  ox[i] = fx;
+  oy[i] = fy;
+  oz[i] = fz;
+  if (!isfinite(fx) || !isfinite(fy) || !isfinite(fz)) atomicOr(status, kStatNonfinite);
+}
+
+constexpr int kXWarps = 4;  // warps per block
+constexpr int kXTargets = 32 * kXWarps;
+
+template <bool kWhole>
+__global__ void __launch_bounds__(32 * kXWarps, kWhole ? 6 : 4)
+walk_exact_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const float4* __restrict__ wx,
+                  const Kids* __restrict__ kids, const double4* __restrict__ rec64,
+                  const double4* __restrict__ body64, const uint32_t* __restrict__ perm,
+                  const TreeHeader* __restrict__ hdr, TopTree top, double G, double eps2,
+                  int want_force, double* __restrict__ part, double* __restrict__ ox,
+                  double* __restrict__ oy, double* __restrict__ oz, unsigned long long* counter,
+                  int32_t* status) {
   wait_for_previous();
+  constexpr int kXU = kWhole ? 2 : 4;  // entries evaluated together
+  static_assert(kXQ % kXU == 0, "whole rounds");
   __shared__ double s2d[kMaxLevels];
   __shared__ float2 band[kMaxLevels];
-  __shared__ uint4 queue[kWalkBlock / 32][kXQ];  // node, lane mask, close to, level
-  const int task = (int)blockIdx.y;
-  const int ntask = top_tasks(top);
+  __shared__ __align__(16) double4 srec[kXWarps][kXQ];
+  __shared__ int qnode[kXWarps][kXQ];
+  __shared__ unsigned qmask[kXWarps][kXQ];    // lanes that take it
+  __shared__ unsigned qlevels[kXWarps][kXQ];  // 0: those of the entry before
+  const int task = kWhole ? 0 : (int)blockIdx.y;
+  const int ntask = kWhole ? 1 : top_tasks(top);
   if (task >= ntask) return;
   const int root = ntask == 1 ? 0 : top.task[task];
   const double theta2 = hdr->theta2, half = hdr->half;
@@ -507,120 +555,227 @@ walk_task_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const RecX* _
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t p = q0 + blockIdx.x * (int64_t)kWalkBlock + threadIdx.x;  // targets [q0, n)
+  const unsigned bit = 1u << lane;
+  const int64_t p = q0 + blockIdx.x * (int64_t)kXTargets + threadIdx.x;  // targets [q0, n)
   const bool valid = p < n;
+  const int p0 = (int)(p - lane);
   const ExactTarget t = exact_target(body64, p, valid, G);
-  const bool coarse = hdr->min_mass >= 0.0;
-  const bool fast =
-      !__any_sync(0xffffffffu, !scale_mass_ok(t.gm)) && walk_in_range(hdr, nbody, eps2);
+  const bool fast = __all_sync(kFull, scale_mass_ok(t.gm)) && walk_in_range(hdr, nbody, eps2);
   const double ih = 1.0 / half;
   const float fx = (float)((t.x - hdr->center[0]) * ih), fy = (float)((t.y - hdr->center[1]) * ih),
               fz = (float)((t.z - hdr->center[2]) * ih);
+  const bool coarse =
+      hdr->min_mass >= 0.0 &&
+      __all_sync(kFull, !valid || (isfinite(fx) && isfinite(fy) && isfinite(fz)));
+  // the box around the warp's targets
+  float bl[3] = {valid ? fx : INFINITY, valid ? fy : INFINITY, valid ? fz : INFINITY};
+  float bh[3] = {valid ? fx : -INFINITY, valid ? fy : -INFINITY, valid ? fz : -INFINITY};
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      bl[k] = fminf(bl[k], __shfl_xor_sync(kFull, bl[k], o));
+      bh[k] = fmaxf(bh[k], __shfl_xor_sync(kFull, bh[k], o));
+    }
+  }
 
   NestedSum sum;
+  double outer[kMaxLevels + 1][3];
   unsigned ninter = 0;
   int cnt = 0;
-  uint4* const q = queue[wid];
-  auto drain = [&]() {
-    __syncwarp();
+  unsigned* const qm = qmask[wid];
+  unsigned* const ql = qlevels[wid];
+  int* const qn = qnode[wid];
+  double4* const sr = srec[wid];
+  // add the queue's terms: bit k of `on`: entry k is the lane's, of `ev`: it
+  // changes levels
+  auto terms = [&](auto quick, unsigned on, unsigned ev) {
+    constexpr bool kQuick = decltype(quick)::value;
+#pragma unroll 1
     for (int k0 = 0; k0 < cnt; k0 += kXU) {
       double rx[kXU], ry[kXU], rz[kXU], w[kXU];
-      uint4 e[kXU];
-      if (fast) {
 #pragma unroll
-        for (int u = 0; u < kXU; ++u) {
-          e[u] = q[min(k0 + u, cnt - 1)];
-          w[u] = exact_weight<true>(t, rec64[e[u].x], eps2, rx[u], ry[u], rz[u]);
-        }
-      } else {
-#pragma unroll
-        for (int u = 0; u < kXU; ++u) {
-          e[u] = q[min(k0 + u, cnt - 1)];
-          w[u] = exact_weight<false>(t, rec64[e[u].x], eps2, rx[u], ry[u], rz[u]);
-        }
-      }
+      for (int u = 0; u < kXU; ++u)
+        w[u] = exact_weight<kQuick>(t, sr[k0 + u], eps2, rx[u], ry[u], rz[u]);
 #pragma unroll
       for (int u = 0; u < kXU; ++u) {
-        if (k0 + u < cnt) {
-          sum.close_to((int)e[u].z);
-          sum.open_to((int)e[u].w);
-          if ((e[u].y >> lane) & 1u) {
-            sum.add(xmul(rx[u], w[u]), xmul(ry[u], w[u]), xmul(rz[u], w[u]));
-            ++ninter;
-          }
+        if (ev >> u & 1) {
+          const unsigned l = ql[k0 + u];
+          sum.close_to((int)(l & 0xffff), outer);
+          sum.open_to((int)(l >> 17), outer);
         }
+        // a lane outside the mask adds 0, which changes no sum
+        const bool mine = on >> u & 1;
+        const double wu = mine ? w[u] : 0.0;
+        if (!kQuick && !mine) rx[u] = ry[u] = rz[u] = 0.0;  // may be infinite
+        sum.add(xmul(rx[u], wu), xmul(ry[u], wu), xmul(rz[u], wu));
       }
+      on >>= kXU;
+      ev >>= kXU;
     }
+  };
+  auto drain = [&]() {
+    __syncwarp();
+    unsigned on = lane < cnt ? qm[lane] : 0;
+    const unsigned ev = __ballot_sync(kFull, lane < cnt && ql[lane] != 0);
+    sr[lane] = rec64[qn[min(lane, cnt - 1)]];
+    // transpose: from a lane mask per entry to an entry mask per lane
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) {
+      const unsigned m = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu
+                                     : j == 2 ? 0x33333333u : 0x55555555u;
+      const unsigned y = __shfl_xor_sync(kFull, on, j);
+      on = lane & j ? (on & ~m) | (y >> j & m) : (on & m) | (y & m) << j;
+    }
+    __syncwarp();
+    if (fast)
+      terms(std::true_type{}, on, ev);
+    else
+      terms(std::false_type{}, on, ev);
     __syncwarp();
     cnt = 0;
   };
 
-  // open_to: opened levels on the current path (a lane is active at a node
-  // of depth d iff open_to == d); low: the least depth of the warp's path
-  // since its last entry
   // the task's cells above were all opened by the lane?
-  const int base = wx[root].b.x & kMetaDepth;
-  int open_to = -1;
-  if (valid) {
-    bool in = true;
+  const int base = __float_as_int(wx[root].w) & kMetaDepth;
+  bool in = valid;
+  if (!kWhole && valid) {
     for (int k = root, d = base - 1; d >= 0; --d) {
       k = top.parent[k];
-      in = in && (k == 0 || (wx[k].b.x & kMetaGate)) && exact_open(rec64[k], t, s2d[d], theta2);
+      in = in && (k == 0 || (__float_as_int(wx[k].w) & kMetaGate)) &&
+           exact_open(rec64[k], t, s2d[d], theta2);
     }
-    if (in) open_to = base;
   }
-  const bool counted = open_to >= 0;
+  const unsigned start = __ballot_sync(kFull, in);
   sum.init(base);
-  int low = base;
-  int node = root;
-  const int end = __float_as_int(wx[root].a.w);
-  auto ld_a = [&](int k) { return __ldg(&wx[k].a); };
-  auto ld_b = [&](int k) { return __ldg(reinterpret_cast<const int2*>(&wx[k].b)); };
-  float4 A = ld_a(node);
-  int2 B = ld_b(node);
-  while (node < end) {
-    const int next = __float_as_int(A.w);
-    if (next <= node || next > nnodes) {  // malformed tree: report, never spin
-      if (lane == 0) atomicOr(status, kStatOverflow);
-      break;
+  // A frame per depth: in lanes 8g..8g+7 the children of the g-th of up to
+  // four opened cells of the frame above (set `above`), with the targets that
+  // take (tk) and open (op) each.  The walk goes through a group of lanes
+  // [pos, end) at a time; the other groups wait until it comes to their cell.
+  int4 frame[kMaxLevels];     // cell, tk, op, pos | end << 8
+  unsigned above[kMaxLevels + 1];
+  int d = base, cn = lane == 0 ? root : -1, pos = 0, end = 8;
+  unsigned tk, op, act = start;
+  auto classify = [&]() {
+    tk = op = 0;
+    bool mixed = false;
+    float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2 bd = band[d];
+    if (cn >= 0) {
+      A = __ldg(&wx[cn]);
+      const int meta = __float_as_int(A.w);
+      if ((meta & kMetaGate) || cn == 0) {
+        if (meta & kMetaLeaf) {  // every target but the body itself
+          const unsigned self = (unsigned)(__float_as_int(A.x) - p0);
+          tk = self < 32 ? act & ~(1u << self) : act;
+        } else {
+          const float nx = fmaxf(fmaxf(bl[0] - A.x, A.x - bh[0]), 0.f),
+                      ny = fmaxf(fmaxf(bl[1] - A.y, A.y - bh[1]), 0.f),
+                      nz = fmaxf(fmaxf(bl[2] - A.z, A.z - bh[2]), 0.f);
+          const float mx = fmaxf(A.x - bl[0], bh[0] - A.x), my = fmaxf(A.y - bl[1], bh[1] - A.y),
+                      mz = fmaxf(A.z - bl[2], bh[2] - A.z);
+          const float near2 = fmaf(nx, nx, fmaf(ny, ny, nz * nz)),
+                      far2 = fmaf(mx, mx, fmaf(my, my, mz * mz));
+          if (coarse && cn != 0 && near2 > bd.y && far2 >= near2)
+            tk = act;
+          else if (coarse && cn != 0 && far2 < bd.x)
+            op = act;
+          else
+            mixed = true;
+        }
+      }
     }
-    // both nodes that may follow are read while this one is decided
-    const int k0 = min(node + 1, nnodes - 1), k1 = min(next, nnodes - 1);
-    const float4 A0 = ld_a(k0), A1 = ld_a(k1);
-    const int2 B0 = ld_b(k0), B1 = ld_b(k1);
-    const int d = B.x & kMetaDepth;
-    open_to = min(open_to, d);
-    low = min(low, d);
-    const bool act = open_to == d && ((B.x & kMetaGate) || node == 0);
-    bool take;
-    int go = next;
-    if (B.x & kMetaLeaf) {
-      take = act && B.y != (int)p;
-    } else {
-      const float rx = A.x - fx, ry = A.y - fy, rz = A.z - fz;
+#pragma unroll 1
+    for (unsigned mm = __ballot_sync(kFull, mixed); mm; mm &= mm - 1) {
+      const int j = __ffs(mm) - 1;
+      const float rx = __shfl_sync(kFull, A.x, j) - fx, ry = __shfl_sync(kFull, A.y, j) - fy,
+                  rz = __shfl_sync(kFull, A.z, j) - fz;
+      const unsigned a = __shfl_sync(kFull, act, j);
       const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-      const float2 bd = band[d];
-      bool open = act && d2 < bd.x;
-      if (__any_sync(0xffffffffu, act && !(coarse && (d2 < bd.x || d2 > bd.y))))
-        open = act && exact_open(rec64[node], t, s2d[d], theta2);
-      take = act && !open;
-      if (open) open_to = d + 1;
-      if (__any_sync(0xffffffffu, open)) go = node + 1;
+      bool open = d2 < bd.x;
+      if (__any_sync(kFull, (a & bit) && !(coarse && (d2 < bd.x || d2 > bd.y))))
+        open = exact_open(rec64[__shfl_sync(kFull, cn, j)], t, s2d[d], theta2);
+      const unsigned o = __ballot_sync(kFull, open) & a;
+      if (lane == j) {
+        op = o;
+        tk = a & ~o;
+      }
     }
-    const unsigned mask = __ballot_sync(0xffffffffu, take);
-    if (mask) {
-      if (lane == 0) q[cnt] = make_uint4((unsigned)node, mask, (unsigned)low, (unsigned)d);
+    frame[d] = make_int4(cn, (int)tk, (int)op, 0);
+    above[d + 1] = 0;
+  };
+  if (start) classify();
+  // low: the least depth of the path since the last entry
+  int low = base, steps = 0;
+  while (start) {
+    const unsigned group = (unsigned)((1ull << end) - (1ull << pos));
+    const unsigned all_op = __ballot_sync(kFull, op != 0);
+    const unsigned opens = all_op & group, takes = __ballot_sync(kFull, tk != 0) & group;
+    const unsigned put = opens ? takes & (opens ^ (opens - 1)) : takes;  // up to the first opened
+    low = min(low, d);
+    if (put) {
+      if (put & bit) {
+        const int r = __popc(put & (bit - 1));
+        qn[cnt + r] = cn;
+        // levels: the one the open sums close to, then the entry's own
+        qm[cnt + r] = tk;
+        ql[cnt + r] = r == 0 ? (unsigned)(low | 0x10000 | d << 17) : 0u;
+        ninter += __popc(tk);
+      }
       low = d;
-      if (++cnt == kXQ) drain();
+      cnt += __popc(put);
+      if (cnt > kXQ - 8) drain();
     }
-    A = go == next ? A1 : A0;
-    B = go == next ? B1 : B0;
-    node = go;
+    if (!opens) {  // group done: on with the frame above
+      if (d == base) break;
+      --d;
+      const int4 f = frame[d];
+      cn = f.x;
+      tk = (unsigned)f.y;
+      op = (unsigned)f.z;
+      pos = f.w & 0xff;
+      end = f.w >> 8;
+      continue;
+    }
+    const int j = __ffs(opens) - 1;
+    frame[d].w = (j + 1) | end << 8;
+    unsigned done = above[d + 1];
+    if (done >> j & 1) {  // its children are in the frame below already
+      pos = 8 * __popc(done & ((1u << j) - 1));
+      ++d;
+      const int4 f = frame[d];
+      cn = f.x;
+      tk = (unsigned)f.y;
+      op = (unsigned)f.z;
+    } else {  // the children of this and of the next opened cells, four at most
+      if (d + 1 >= kMaxLevels || ++steps > nnodes) {  // malformed tree: report, never spin
+        if (lane == 0) atomicOr(status, kStatOverflow);
+        break;
+      }
+      const unsigned s0 = all_op & ~((1u << j) - 1), s1 = s0 & (s0 - 1), s2 = s1 & (s1 - 1),
+                     s3 = s2 & (s2 - 1);
+      done = s0 & ~(s3 & (s3 - 1));
+      const unsigned mine = lane < 16 ? (lane < 8 ? s0 : s1) : (lane < 24 ? s2 : s3);
+      const int from = __ffs(mine) - 1;
+      const int cell = __shfl_sync(kFull, cn, from & 31);
+      act = __shfl_sync(kFull, op, from & 31);
+      cn = -1;
+      if (mine) cn = __ldg(&kids[cell].id[lane & 7]);
+      if (cn <= cell || cn >= nnodes) cn = -1;
+      above[d + 1] = done;
+      ++d;
+      classify();
+      pos = 0;
+    }
+    end = pos + 8;
   }
-  drain();
-  sum.close_to(base);
+  if (cnt) drain();
+  sum.close_to(base, outer);
   warp_count(ninter, counter);
-  if (counted) {
+  if (kWhole) {
+    if (valid)
+      exact_store(sum.x, sum.y, sum.z, body64[p].w, perm[p], want_force, ox, oy, oz, status);
+  } else if (in) {
     double* o = part + ((size_t)task * (size_t)(n - q0) + (size_t)(p - q0)) * 3;
     o[0] = sum.x;
     o[1] = sum.y;
@@ -630,8 +785,11 @@ walk_task_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const RecX* _
 
 // A target's force from its tasks' contributions: the walk over the upper
 // cells, nested as in compute_force (gravity_tree.rs:194-205).
-__global__ void __launch_bounds__(kWalkBlock)
-exact_combine_kernel(int64_t q0, int64_t n, const RecX* __restrict__ wx,
+constexpr int kStage = 64;  // top nodes in shared memory at a time
+constexpr int kAhead = 8;
+
+__global__ void __launch_bounds__(kStage)
+exact_combine_kernel(int64_t q0, int64_t n, const float4* __restrict__ wx,
                      const double4* __restrict__ rec64, const double4* __restrict__ body64,
                      const uint32_t* __restrict__ perm, const TreeHeader* __restrict__ hdr,
                      TopTree top, double G, double eps2, int want_force,
@@ -639,6 +797,8 @@ exact_combine_kernel(int64_t q0, int64_t n, const RecX* __restrict__ wx,
                      double* __restrict__ oy, double* __restrict__ oz,
                      unsigned long long* counter, int32_t* status) {
   wait_for_previous();
+  __shared__ int4 se[kStage];
+  __shared__ __align__(16) double4 sr[kStage];
   const int64_t p = q0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const bool valid = p < n;
   const ExactTarget t = exact_target(body64, valid ? p : q0, true, G);
@@ -646,150 +806,60 @@ exact_combine_kernel(int64_t q0, int64_t n, const RecX* __restrict__ wx,
   const int ntop = top_tasks(top) == 1 ? 1 : *top.counts & 0xffff;
   unsigned ninter = 0;
   NestedSum sum;
+  double outer[kMaxLevels + 1][3];
   sum.init(0);
   int open_to = 0;
-  for (int i = 0; i < ntop; ++i) {
-    const int4 e = ntop == 1 ? make_int4(0, 0, 0, 0) : top.top[i];
-    const int node = e.x, d = e.z;
-    open_to = min(open_to, d);
-    sum.close_to(d);
-    const bool act = open_to == d && (node == 0 || (wx[node].b.x & kMetaGate));
-    if (e.y >= 0) {
-      sum.open_to(d);
-      if (act && valid) {
-        const double* q = part + ((size_t)e.y * (size_t)(n - q0) + (size_t)(p - q0)) * 3;
-        sum.add(q[0], q[1], q[2]);
+  for (int i0 = 0; i0 < ntop; i0 += kStage) {
+    __syncthreads();
+    const int i = i0 + (int)threadIdx.x;
+    if (threadIdx.x < kStage) {
+      const int4 e = ntop == 1 ? make_int4(0, 0, 0, 0)
+                               : i < ntop ? top.top[i] : make_int4(0, -1, 0, 0);
+      const bool gate = e.x == 0 || (__float_as_int(wx[e.x].w) & kMetaGate);
+      se[threadIdx.x] = make_int4(e.x, e.y, e.z, gate);
+      sr[threadIdx.x] = rec64[e.x];
+    }
+    __syncthreads();
+    for (int k0 = 0; k0 < min(kStage, ntop - i0); k0 += kAhead) {
+      // the contributions of several tasks are read together
+      double v[kAhead][3];
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        const int task = se[k0 + k].y;
+        const double* q = part + ((size_t)max(task, 0) * (size_t)(n - q0) + (size_t)(p - q0)) * 3;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[k][c] = task >= 0 && valid ? q[c] : 0.0;
       }
-    } else {
-      const double4 r = rec64[node];
-      const bool open = act && exact_open(r, t, hdr->s2[d], theta2);
-      if (open) open_to = d + 1;
-      if (act && !open) {  // taken as a monopole
-        double rx, ry, rz;
-        const double w = exact_weight<false>(t, r, eps2, rx, ry, rz);
-        sum.open_to(d);
-        sum.add(xmul(rx, w), xmul(ry, w), xmul(rz, w));
-        ninter += valid;
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        if (i0 + k0 + k >= ntop) break;
+        const int4 e = se[k0 + k];
+        const int d = e.z;
+        open_to = min(open_to, d);
+        sum.close_to(d, outer);
+        const bool act = open_to == d && e.w;
+        if (e.y >= 0) {
+          sum.open_to(d, outer);
+          if (act && valid) sum.add(v[k][0], v[k][1], v[k][2]);
+        } else {
+          const double4 r = sr[k0 + k];
+          const bool open = act && exact_open(r, t, hdr->s2[d], theta2);
+          if (open) open_to = d + 1;
+          if (act && !open) {  // taken as a monopole
+            double rx, ry, rz;
+            const double w = exact_weight<false>(t, r, eps2, rx, ry, rz);
+            sum.open_to(d, outer);
+            sum.add(xmul(rx, w), xmul(ry, w), xmul(rz, w));
+            ninter += valid;
+          }
+        }
       }
     }
   }
-  sum.close_to(0);
+  sum.close_to(0, outer);
   warp_count(ninter, counter);
   if (!valid) return;
-  double f[3] = {sum.x, sum.y, sum.z};
-  const double mi = body64[p].w;
-  const uint32_t i = perm[p];
-  double* o[3] = {ox, oy, oz};
-  bool bad = false;
-  for (int k = 0; k < 3; ++k) {
-    if (!want_force) f[k] = xdiv(f[k], mi);  // a = F / m (integrators.rs:115)
-    o[k][i] = f[k];
-    bad |= !isfinite(f[k]);
-  }
-  if (bad) atomicOr(status, kStatNonfinite);
-}
-
-// One walk per target over the whole tree, terms evaluated as they are
-// taken: 48 registers and more warps per SM hide the latency of a visit, so
-// with enough targets to fill the SMs this is the faster form (2^20 bodies:
-// 19.8 ms against 28.7 for walk_task_kernel over the root, 100 000: 2.9
-// against 3.0; 65 536: 2.7 against 2.1, 10 000: 1.64 against 0.44).
-__global__ void __launch_bounds__(kWalkBlock)
-walk_exact_kernel(int64_t q0, int64_t n, int64_t nnodes, const int4* __restrict__ link,
-                  const double4* __restrict__ rec64, const double4* __restrict__ body64,
-                  const uint32_t* __restrict__ perm, const TreeHeader* __restrict__ hdr, double G,
-                  double eps2, int want_force, double* __restrict__ ox, double* __restrict__ oy,
-                  double* __restrict__ oz, unsigned long long* counter, int32_t* status) {
-  wait_for_previous();
-  __shared__ double s2d[kMaxLevels];
-  for (int d = threadIdx.x; d < kMaxLevels; d += blockDim.x) s2d[d] = hdr->s2[d];
-  __syncthreads();
-  const double theta2 = hdr->theta2;
-  const int64_t p = q0 + blockIdx.x * (int64_t)kWalkBlock + threadIdx.x;  // targets [q0, n)
-  const bool valid = p < n;
-  double tx = 0, ty = 0, tz = 0, mi = 0;
-  if (valid) {
-    const double4 b = body64[p];
-    tx = b.x;
-    ty = b.y;
-    tz = b.z;
-    mi = b.w;
-  }
-  const double gm = xmul(G, mi);
-  // acc[d] collects the terms of the nodes at depth d (children of the lane's
-  // opened node at depth d-1); acc[0] is the root's own term.
-  double acc[kMaxLevels + 1][3];
-  acc[0][0] = acc[0][1] = acc[0][2] = 0.0;
-  unsigned ninter = 0;
-  int open_to = 0;
-  int32_t node = 0;
-
-  // compute_gravity_pair (gravity_tree.rs:218-234)
-  auto pair = [&](double4 s, int slot) {
-    const double rx = xsub(s.x, tx), ry = xsub(s.y, ty), rz = xsub(s.z, tz);
-    const double r2 = xlen2(rx, ry, rz);
-    const double s2 = xadd(r2, eps2);
-    const double s3 = xmul(s2, xsqrt(s2));
-    const double sc = xdiv(xmul(gm, s.w), s3);
-    acc[slot][0] = xadd(acc[slot][0], xmul(rx, sc));
-    acc[slot][1] = xadd(acc[slot][1], xmul(ry, sc));
-    acc[slot][2] = xadd(acc[slot][2], xmul(rz, sc));
-  };
-  auto close_to = [&](int d) {  // finish the lane's opened cells at depths >= d
-    for (int k = open_to; k > d; --k) {
-      acc[k - 1][0] = xadd(acc[k - 1][0], acc[k][0]);
-      acc[k - 1][1] = xadd(acc[k - 1][1], acc[k][1]);
-      acc[k - 1][2] = xadd(acc[k - 1][2], acc[k][2]);
-    }
-    if (open_to > d) open_to = d;
-  };
-
-  while (node < nnodes) {
-    const int4 lk = link[node];
-    if (lk.x <= node || lk.x > nnodes) {  // malformed tree: report, never spin
-      if ((threadIdx.x & 31) == 0) atomicOr(status, kStatOverflow);
-      break;
-    }
-    const int d = lk.w & kMetaDepth;
-    close_to(d);
-    const bool act = valid && open_to == d && ((lk.w & kMetaGate) || node == 0);
-    if (lk.w & kMetaLeaf) {
-      const int sp = (lk.z - lk.y) == 1 ? lk.y : lk.z - 1;
-      if (act && sp != p) {
-        pair(rec64[node], d);
-        ++ninter;
-      }
-      node = lk.x;
-    } else {
-      const double4 s = rec64[node];
-      const double rx = xsub(s.x, tx), ry = xsub(s.y, ty), rz = xsub(s.z, tz);
-      const double d2 = xlen2(rx, ry, rz);
-      const bool open = act && !(s2d[d] < xmul(theta2, d2));
-      if (act && !open) {
-        pair(s, d);
-        ++ninter;
-      }
-      if (open) {
-        acc[d + 1][0] = acc[d + 1][1] = acc[d + 1][2] = 0.0;
-        open_to = d + 1;
-      }
-      node = __any_sync(0xffffffffu, open) ? node + 1 : lk.x;
-    }
-  }
-  close_to(0);
-  warp_count(ninter, counter);
-  if (!valid) return;
-  double fx = acc[0][0], fy = acc[0][1], fz = acc[0][2];
-  if (!want_force) {  // a = F / m (integrators.rs:115)
-    fx = xdiv(fx, mi);
-    fy = xdiv(fy, mi);
-    fz = xdiv(fz, mi);
-  }
-  const uint32_t i = perm[p];
-  ox[i] = fx;
-  oy[i] = fy;
-  oz[i] = fz;
-  if (!isfinite(fx) || !isfinite(fy) || !isfinite(fz)) atomicOr(status, kStatNonfinite);
+  exact_store(sum.x, sum.y, sum.z, body64[p].w, perm[p], want_force, ox, oy, oz, status);
 }
 
 }  // namespace
@@ -817,19 +887,20 @@ int bh_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force,
     PHYS_TRY(bh_group_walk(c, p, t, want_force, ox, oy, oz));
   } else if (p->precision == PHYS_F64_EXACT) {
     const int tasks = t.top.max_tasks;
+    const int xgrid = (int)ceil_div(nt > 0 ? nt : 1, kXTargets);
     if (tasks > 0) {
       double* part = nullptr;
       PHYS_TRY(ws_alloc(c, WS_DIRECT_PART, 3 * nt * tasks, &part));
-      PHYS_LAUNCH(c, walk_task_kernel, dim3(grid, tasks), kWalkBlock, 0, q0, q1, n, t.nnodes,
-                  t.wx, t.rec64, t.body64, t.hdr, t.top, p->G, eps2, part, c->d_counter,
-                  c->d_status);
-      PHYS_LAUNCH(c, exact_combine_kernel, (int)ceil_div(nt, 64), 64, 0, q0, q1, t.wx, t.rec64,
+      PHYS_LAUNCH(c, walk_exact_kernel<false>, dim3(xgrid, tasks), 32 * kXWarps, 0, q0, q1, n,
+                  (int)t.nnodes, t.wx, t.kids, t.rec64, t.body64, t.perm, t.hdr, t.top, p->G, eps2,
+                  (int)want_force, part, ox, oy, oz, c->d_counter, c->d_status);
+      PHYS_LAUNCH(c, exact_combine_kernel, (int)ceil_div(nt > 0 ? nt : 1, kStage), kStage, 0, q0, q1, t.wx, t.rec64,
                   t.body64, t.perm, t.hdr, t.top, p->G, eps2, want_force, part, ox, oy, oz,
                   c->d_counter, c->d_status);
     } else {
-      PHYS_LAUNCH(c, walk_exact_kernel, grid, kWalkBlock, 0, q0, q1, t.nnodes, t.link, t.rec64,
-                  t.body64, t.perm, t.hdr, p->G, eps2, want_force, ox, oy, oz, c->d_counter,
-                  c->d_status);
+      PHYS_LAUNCH(c, walk_exact_kernel<true>, xgrid, 32 * kXWarps, 0, q0, q1, n, (int)t.nnodes, t.wx,
+                  t.kids, t.rec64, t.body64, t.perm, t.hdr, t.top, p->G, eps2, (int)want_force,
+                  (double*)nullptr, ox, oy, oz, c->d_counter, c->d_status);
     }
   } else if (p->precision == PHYS_F64) {
     PHYS_LAUNCH(c, walk_kernel<false>, grid, kWalkBlock, 0, (int)q0, (int)q1, (int)t.nnodes, t.w32, t.w64,

@@ -54,3 +54,23 @@ def test_ranges(ctx, kind):
     ctx.upload(pos, None, m)
     f = ctx.gravity_forces(exact(0.5, eps))
     assert np.array_equal(f, oracle.bh_forces(pos, m, 1.0, eps, 0.5))
+
+
+@pytest.mark.parametrize("kind,theta", [("negative", 0.7), ("clumps", 1.1), ("unsoftened", 0.9)])
+def test_whole_walk_ranges(ctx, kind, theta):
+    """More targets than are split: the f64 test for every cell, deep chains
+    with the cells of several depths waiting, and the library's weights."""
+    n = 65_700
+    rng = np.random.default_rng(5)
+    pos, _, m = ics.plummer(n, seed=8)
+    eps = 0.02
+    if kind == "negative":
+        m *= rng.choice([-1.0, 1.0], n, p=[0.3, 0.7])
+    elif kind == "clumps":
+        pos[200:230] = pos[200]
+        pos[900:1100] = pos[900] + rng.normal(scale=1e-7, size=(200, 3))
+    else:
+        eps = 0.0
+    ctx.upload(pos, None, m)
+    f = ctx.gravity_forces(exact(theta, eps))
+    assert np.array_equal(f, oracle.bh_forces(pos, m, 1.0, eps, theta))
