@@ -5,8 +5,9 @@
 // One persistent kernel runs a chunk of steps for every system: a group of G
 // lanes (G = 8, 16 or 32; several groups per warp when G < 32) takes the next
 // system from a global queue (systems in descending N, longest first), keeps
-// the system's f64 state in shared memory for the whole chunk and returns it
-// to HBM at the end.  Pair terms are F32C (double-float relative coordinates,
+// the system's f64 state on chip for the whole chunk (F32C with 32 lanes or
+// lanes by size: in registers; otherwise in shared memory) and returns it to
+// HBM at the end.  Pair terms are F32C (double-float relative coordinates,
 // two-sum accumulation) or F64_EXACT (reference op order, bit-identical).
 // The host captures the chunk launches of a run in a CUDA graph; an
 // autotuner picks G by timing a few steps of each candidate.
@@ -40,6 +41,16 @@ struct GroupSmemT {
   float lx[MAXN], ly[MAXN], lz[MAXN];            // lo parts
 };
 using GroupSmem = GroupSmemT<kMaxSys>;
+// The F32C staging alone: the bodies' f64 state is in their lanes' registers.
+template <int MAXN>
+struct SourceSmemT {
+  float hx[MAXN], hy[MAXN], hz[MAXN], hm[MAXN];
+  float lx[MAXN], ly[MAXN], lz[MAXN];
+};
+using SourceSmem = SourceSmemT<kMaxSys>;
+static_assert(sizeof(SourceSmemT<8>) % 16 == 0 && 2 * sizeof(SourceSmemT<16>) <= sizeof(SourceSmem) &&
+                  4 * sizeof(SourceSmemT<8>) <= sizeof(SourceSmem),
+              "sub-warp groups fit in a warp's share, 16-byte aligned");
 // With lanes per system chosen by size, a warp's shared memory holds one
 // 64-body group, two 16-body groups or four 8-body groups in turn.
 // quads of sources are read with 16-byte loads
@@ -133,19 +144,52 @@ __device__ __forceinline__ TargetNeg target_neg(const S_t* S, int i) {
   return TargetNeg{n(S->hx[i]), n(S->hy[i]), n(S->hz[i]), n(S->lx[i]), n(S->ly[i]), n(S->lz[i])};
 }
 
-// F32C accelerations of the group's own targets, TC targets per pass.  The
-// sources come four at a time (two packed f32x2 pairs: sources j, j+1 and
-// j+2, j+3); with one target per lane the two pairs go to separate partial
-// sums, so two dependency chains interleave.  Partial sums of kFold sources are
-// folded into a (hi, lo) accumulator by two-sum.
-template <int G, int TC, bool kSkip, class S_t>
-__device__ void group_forces_f32c(S_t* S, int N, int gl, double Gc, float eps2f) {
+// F32C acceleration of body i.  The sources come four at a time (two packed
+// f32x2 pairs: sources j, j+1 and j+2, j+3); the two pairs go to separate
+// partial sums, so two dependency chains interleave.  Partial sums of kFold
+// sources are folded into a (hi, lo) accumulator by two-sum.
+template <bool kSkip, class S_t>
+__device__ __forceinline__ void one_target(const S_t* S, int N, int i, double Gc, float eps2f,
+                                           double (&f)[3]) {
   const float2 e2 = make_float2(eps2f, eps2f);
-  constexpr int kSets = TC == 1 ? 2 : 1;
+  const int n4 = (N + 3) & ~3;
+  const TargetNeg a = target_neg(S, i);
+  const float2 z2 = make_float2(0.f, 0.f);
+  float2 px0 = z2, py0 = z2, pz0 = z2, px1 = z2, py1 = z2, pz1 = z2;
+  float hx = 0.f, hy = 0.f, hz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
+  for (int j0 = 0; j0 < n4; j0 += kFold) {
+    const int j1 = min(n4, j0 + kFold);
+    for (int j = j0; j < j1; j += 4) {
+      const QuadSrc q = load_quad(S, j);
+      pair_term<kSkip>(lo2(q.sx), lo2(q.sy), lo2(q.sz), lo2(q.sm), lo2(q.tx), lo2(q.ty),
+                       lo2(q.tz), a.hx, a.hy, a.hz, a.lx, a.ly, a.lz, e2, j == i, j + 1 == i, px0,
+                       py0, pz0);
+      pair_term<kSkip>(hi2(q.sx), hi2(q.sy), hi2(q.sz), hi2(q.sm), hi2(q.tx), hi2(q.ty),
+                       hi2(q.tz), a.hx, a.hy, a.hz, a.lx, a.ly, a.lz, e2, j + 2 == i, j + 3 == i,
+                       px1, py1, pz1);
+    }
+    fold(px0, hx, lx);
+    fold(py0, hy, ly);
+    fold(pz0, hz, lz);
+    fold(px1, hx, lx);
+    fold(py1, hy, ly);
+    fold(pz1, hz, lz);
+  }
+  f[0] = Gc * ((double)hx + (double)lx);
+  f[1] = Gc * ((double)hy + (double)ly);
+  f[2] = Gc * ((double)hz + (double)lz);
+}
+
+// Accelerations of the group's own targets, two per pass (a fixed 8 or 16
+// lanes and more bodies than those; each target one chain of partial sums).
+template <int G, bool kSkip, class S_t>
+__device__ void two_targets(S_t* S, int N, int gl, double Gc, float eps2f) {
+  constexpr int TC = 2;
+  const float2 e2 = make_float2(eps2f, eps2f);
   const int n4 = (N + 3) & ~3;
   for (int i0 = gl; i0 < N; i0 += G * TC) {
     TargetNeg tn[TC];
-    float2 px[kSets][TC], py[kSets][TC], pz[kSets][TC];
+    float2 px[TC], py[TC], pz[TC];
     float hx[TC], hy[TC], hz[TC], lx[TC], ly[TC], lz[TC];
     int idx[TC];
 #pragma unroll
@@ -153,8 +197,7 @@ __device__ void group_forces_f32c(S_t* S, int N, int gl, double Gc, float eps2f)
       idx[t] = i0 + t * G;
       tn[t] = target_neg(S, idx[t] < N ? idx[t] : i0);
       hx[t] = hy[t] = hz[t] = lx[t] = ly[t] = lz[t] = 0.f;
-#pragma unroll
-      for (int k = 0; k < kSets; ++k) px[k][t] = py[k][t] = pz[k][t] = make_float2(0.f, 0.f);
+      px[t] = py[t] = pz[t] = make_float2(0.f, 0.f);
     }
     for (int j0 = 0; j0 < n4; j0 += kFold) {
       const int j1 = min(n4, j0 + kFold);
@@ -165,21 +208,17 @@ __device__ void group_forces_f32c(S_t* S, int N, int gl, double Gc, float eps2f)
           const TargetNeg& a = tn[t];
           pair_term<kSkip>(lo2(q.sx), lo2(q.sy), lo2(q.sz), lo2(q.sm), lo2(q.tx), lo2(q.ty),
                            lo2(q.tz), a.hx, a.hy, a.hz, a.lx, a.ly, a.lz, e2, j == idx[t],
-                           j + 1 == idx[t], px[0][t], py[0][t], pz[0][t]);
+                           j + 1 == idx[t], px[t], py[t], pz[t]);
           pair_term<kSkip>(hi2(q.sx), hi2(q.sy), hi2(q.sz), hi2(q.sm), hi2(q.tx), hi2(q.ty),
                            hi2(q.tz), a.hx, a.hy, a.hz, a.lx, a.ly, a.lz, e2, j + 2 == idx[t],
-                           j + 3 == idx[t], px[kSets - 1][t], py[kSets - 1][t],
-                           pz[kSets - 1][t]);
+                           j + 3 == idx[t], px[t], py[t], pz[t]);
         }
       }
 #pragma unroll
       for (int t = 0; t < TC; ++t) {
-#pragma unroll
-        for (int k = 0; k < kSets; ++k) {
-          fold(px[k][t], hx[t], lx[t]);
-          fold(py[k][t], hy[t], ly[t]);
-          fold(pz[k][t], hz[t], lz[t]);
-        }
+        fold(px[t], hx[t], lx[t]);
+        fold(py[t], hy[t], ly[t]);
+        fold(pz[t], hz[t], lz[t]);
       }
     }
 #pragma unroll
@@ -211,7 +250,8 @@ __device__ __forceinline__ int next_pow2(int v) {
 // compile time, so b's quad is a's and is loaded once; kR = 0 derives the
 // streams from N.
 template <bool kSkip, int kR, class S_t>
-__device__ void group_forces_f32c_split(S_t* S, int N, int gl, double Gc, float eps2f) {
+__device__ __forceinline__ void split_targets(const S_t* S, int N, int gl, double Gc, float eps2f,
+                                              double (&fa_)[3], double (&fb_)[3]) {
   const float2 e2 = make_float2(eps2f, eps2f);
   const int nb = N - 32;
   const int lps = kR ? 32 / kR : next_pow2(nb), r = kR ? kR : 32 / lps;
@@ -273,9 +313,9 @@ __device__ void group_forces_f32c_split(S_t* S, int N, int gl, double Gc, float 
   fold(pbx, hbx, lbx);
   fold(pby, hby, lby);
   fold(pbz, hbz, lbz);
-  S->ax[ta] = Gc * ((double)hax + (double)lax);
-  S->ay[ta] = Gc * ((double)hay + (double)lay);
-  S->az[ta] = Gc * ((double)haz + (double)laz);
+  fa_[0] = Gc * ((double)hax + (double)lax);
+  fa_[1] = Gc * ((double)hay + (double)lay);
+  fa_[2] = Gc * ((double)haz + (double)laz);
   double bx = (double)hbx + (double)lbx, by = (double)hby + (double)lby,
          bz = (double)hbz + (double)lbz;
   for (int o = lps; o < 32; o <<= 1) {  // the streams' sums of the same b
@@ -283,34 +323,47 @@ __device__ void group_forces_f32c_split(S_t* S, int N, int gl, double Gc, float 
     by += __shfl_xor_sync(0xffffffffu, by, o);
     bz += __shfl_xor_sync(0xffffffffu, bz, o);
   }
-  if (st == 0 && tb < N) {
-    S->ax[tb] = Gc * bx;
-    S->ay[tb] = Gc * by;
-    S->az[tb] = Gc * bz;
+  fb_[0] = Gc * bx;
+  fb_[1] = Gc * by;
+  fb_[2] = Gc * bz;
+}
+
+// A lane's own bodies: gl, and with 32 lanes gl + 32.
+struct Body {
+  double x, y, z, vx, vy, vz, a[3];
+};
+
+// F32C accelerations of the lane's own bodies into registers.
+template <int G, bool kSkip, int kBodies, class S_t>
+__device__ __forceinline__ void own_forces(const S_t* S, int N, int gl, double Gc, float eps2f,
+                                           Body (&own)[kBodies]) {
+  if constexpr (kBodies == 2) {
+    if (N > 48)
+      split_targets<kSkip, 1>(S, N, gl, Gc, eps2f, own[0].a, own[1].a);
+    else
+      split_targets<kSkip, 0>(S, N, gl, Gc, eps2f, own[0].a, own[1].a);
+  } else if (gl < N) {
+    one_target<kSkip>(S, N, gl, Gc, eps2f, own[0].a);
   }
 }
 
-// Targets per lane for this system: one, or passes of kMaxTC (two) when
-// the system has more bodies than the group has lanes (8 or 16 lanes only:
-// 32 lanes take 33..64 bodies in the split layout).
-template <int G, int kMaxTC, bool kSkip, class S_t>
-__device__ __forceinline__ void group_forces_f32c_any(S_t* S, int N, int gl, double Gc,
-                                                      float eps2f) {
-  if (G == 32 && N > 32) {
-    if (N > 48)
-      group_forces_f32c_split<kSkip, 1>(S, N, gl, Gc, eps2f);
-    else
-      group_forces_f32c_split<kSkip, 0>(S, N, gl, Gc, eps2f);
-    return;
+// Accelerations of a system on a fixed 8 or 16 lanes: one target per lane, or
+// passes of two when it has more bodies.
+template <int G, bool kSkip, class S_t>
+__device__ __forceinline__ void group_forces_f32c(S_t* S, int N, int gl, double Gc, float eps2f) {
+  if (N > G) {
+    two_targets<G, kSkip>(S, N, gl, Gc, eps2f);
+  } else if (gl < N) {
+    double f[3];
+    one_target<kSkip>(S, N, gl, Gc, eps2f, f);
+    S->ax[gl] = f[0];
+    S->ay[gl] = f[1];
+    S->az[gl] = f[2];
   }
-  if (kMaxTC == 1 || N <= G)
-    group_forces_f32c<G, 1, kSkip>(S, N, gl, Gc, eps2f);
-  else
-    group_forces_f32c<G, (kMaxTC > 1 ? 2 : 1), kSkip>(S, N, gl, Gc, eps2f);
 }
 
 // Accelerations of the group's own targets (i = gl, gl+G, ...) into S->a.
-template <int G, bool kExact, int kMaxTC, class S_t>
+template <int G, bool kExact, class S_t>
 __device__ void group_forces(S_t* S, int N, int gl, double Gc, double eps2) {
   if (kExact) {
     for (int i = gl; i < N; i += G) {
@@ -334,9 +387,9 @@ __device__ void group_forces(S_t* S, int N, int gl, double Gc, double eps2) {
   }
   const float eps2f = (float)eps2;
   if (eps2f > 0.f)
-    group_forces_f32c_any<G, kMaxTC, false>(S, N, gl, Gc, eps2f);
+    group_forces_f32c<G, false>(S, N, gl, Gc, eps2f);
   else  // eps = 0: the self pair must be skipped by index
-    group_forces_f32c_any<G, kMaxTC, true>(S, N, gl, Gc, eps2f);
+    group_forces_f32c<G, true>(S, N, gl, Gc, eps2f);
 }
 
 struct EnsArgs {
@@ -354,7 +407,7 @@ struct EnsArgs {
 
 // A group of G lanes takes systems s in [lo, hi) from the counter and runs
 // `nsteps` reference ticks on each with its state in shared memory.
-template <int G, bool kExact, int kMaxTC, class S_t>
+template <int G, bool kExact, class S_t>
 __device__ void drain(S_t* S, const EnsArgs& a, int lo, int hi, int* ctr, int maxn) {
   const int gl = (threadIdx.x & 31) % G;
   const unsigned gm = group_mask<G>();
@@ -389,7 +442,7 @@ __device__ void drain(S_t* S, const EnsArgs& a, int lo, int hi, int* ctr, int ma
     // slots N .. N rounded up to 4 are massless pads (the quads of sources)
     for (int i = N + gl; i < ((N + 3) & ~3); i += G) set_pad(S, i);
     __syncwarp(gm);
-    if (a.need_accel && N >= 2) group_forces<G, kExact, kMaxTC>(S, N, gl, a.Gc, a.eps2);
+    if (a.need_accel && N >= 2) group_forces<G, kExact>(S, N, gl, a.Gc, a.eps2);
     if (a.need_accel && N < 2)
       for (int i = gl; i < N; i += G) S->ax[i] = S->ay[i] = S->az[i] = 0.0;
     __syncwarp(gm);
@@ -406,7 +459,7 @@ __device__ void drain(S_t* S, const EnsArgs& a, int lo, int hi, int* ctr, int ma
         split_into(S, i);
       }
       __syncwarp(gm);
-      if (N >= 2) group_forces<G, kExact, kMaxTC>(S, N, gl, a.Gc, a.eps2);
+      if (N >= 2) group_forces<G, kExact>(S, N, gl, a.Gc, a.eps2);
       __syncwarp(gm);
       // velocity_verlet_velocity_system: v += (prev + a) dt/2
       for (int i = gl; i < N; i += G) {
@@ -434,6 +487,132 @@ __device__ void drain(S_t* S, const EnsArgs& a, int lo, int hi, int* ctr, int ma
   }
 }
 
+// The same for F32C systems of at most kBodies bodies per lane, with their
+// state in the lanes' registers: shared memory holds the sources only, and a
+// step reads and writes no f64 array (30 of the 60 shared-memory accesses per
+// body and step that are not pair sources).  kBodies = 2: systems of 33..64
+// bodies.  Bound by the packed pair terms, about 64 % of their rate on 12
+// warps an SM (150 registers; 16 warps at 128 registers do the same at 16384
+// systems and worse at 2000, 20 warps worse at both).  200 steps of 16384
+// systems of 3..64 bodies 5.74 -> 5.46 ms, 4096 of 3..32 0.88 -> 0.76, 16384
+// of 3..24 1.90 -> 1.65.
+template <int G, int kBodies, class S_t>
+__device__ __forceinline__ void run_system(S_t* S, const EnsArgs& a, int64_t b, int N) {
+  const int gl = (threadIdx.x & 31) % G;
+  const unsigned gm = group_mask<G>();
+  const double dt = a.dt;
+  const double h2 = xmul(xmul(0.5, dt), dt), hdt = xmul(0.5, dt);
+  const float eps2f = (float)a.eps2;
+  Body own[kBodies];
+  bool on[kBodies];
+  auto stage = [&](int i, const Body& o) {
+    split_df(o.x, S->hx[i], S->lx[i]);
+    split_df(o.y, S->hy[i], S->ly[i]);
+    split_df(o.z, S->hz[i], S->lz[i]);
+  };
+#pragma unroll
+  for (int t = 0; t < kBodies; ++t) {
+    const int i = gl + t * G;
+    on[t] = i < N;
+    own[t] = Body{};
+    if (on[t]) {
+      own[t] = Body{a.x[b + i],  a.y[b + i],  a.z[b + i],
+                    a.vx[b + i], a.vy[b + i], a.vz[b + i],
+                    {a.ax[b + i], a.ay[b + i], a.az[b + i]}};
+      S->hm[i] = (float)a.m[b + i];
+      stage(i, own[t]);
+    }
+  }
+  // slots N .. N rounded up to 4 are massless pads (the quads of sources)
+  for (int i = N + gl; i < ((N + 3) & ~3); i += G) set_pad(S, i);
+  __syncwarp(gm);
+  auto forces = [&]() {
+    if (eps2f > 0.f)
+      own_forces<G, false>(S, N, gl, a.Gc, eps2f, own);
+    else  // eps = 0: the self pair must be skipped by index
+      own_forces<G, true>(S, N, gl, a.Gc, eps2f, own);
+  };
+  if (a.need_accel) {
+    if (N >= 2)
+      forces();
+    else
+      own[0].a[0] = own[0].a[1] = own[0].a[2] = 0.0;
+  }
+  for (int st = 0; st < a.nsteps; ++st) {
+    double prev[kBodies][3];
+    __syncwarp(gm);  // the sources are no longer read
+#pragma unroll
+    for (int t = 0; t < kBodies; ++t) {
+      // velocity_verlet_position_system: prev = a; x += v dt + a dt^2/2
+      Body& o = own[t];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) prev[t][k] = o.a[k];
+      o.x = xadd(o.x, xadd(xmul(o.vx, dt), xmul(o.a[0], h2)));
+      o.y = xadd(o.y, xadd(xmul(o.vy, dt), xmul(o.a[1], h2)));
+      o.z = xadd(o.z, xadd(xmul(o.vz, dt), xmul(o.a[2], h2)));
+      if (on[t]) stage(gl + t * G, o);
+    }
+    __syncwarp(gm);
+    if (N >= 2) forces();
+#pragma unroll
+    for (int t = 0; t < kBodies; ++t) {
+      // velocity_verlet_velocity_system: v += (prev + a) dt/2
+      Body& o = own[t];
+      o.vx = xadd(o.vx, xmul(xadd(prev[t][0], o.a[0]), hdt));
+      o.vy = xadd(o.vy, xmul(xadd(prev[t][1], o.a[1]), hdt));
+      o.vz = xadd(o.vz, xmul(xadd(prev[t][2], o.a[2]), hdt));
+    }
+  }
+  bool bad = false;
+#pragma unroll
+  for (int t = 0; t < kBodies; ++t) {
+    const int i = gl + t * G;
+    const Body& o = own[t];
+    if (!on[t]) continue;
+    a.x[b + i] = o.x;
+    a.y[b + i] = o.y;
+    a.z[b + i] = o.z;
+    a.vx[b + i] = o.vx;
+    a.vy[b + i] = o.vy;
+    a.vz[b + i] = o.vz;
+    a.ax[b + i] = o.a[0];
+    a.ay[b + i] = o.a[1];
+    a.az[b + i] = o.a[2];
+    bad |= !isfinite(o.x) || !isfinite(o.vx) || !isfinite(o.a[0]);
+  }
+  if (bad) atomicOr(a.status, kStatNonfinite);
+  __syncwarp(gm);
+}
+
+template <int G, class S_t>
+__device__ void drain_f32c(S_t* S, const EnsArgs& a, int lo, int hi, int* ctr, int maxn) {
+  const int gl = (threadIdx.x & 31) % G;
+  const unsigned gm = group_mask<G>();
+  for (;;) {
+    int s = 0;
+    if (gl == 0) s = lo + atomicAdd(ctr, 1);
+    s = __shfl_sync(gm, s, 0, G);
+    if (s >= hi) break;
+    const int sys = a.order[s];
+    const int64_t b = a.off[sys];
+    const int N = (int)(a.off[sys + 1] - b);
+    if (N < 0 || N > maxn) {
+      if (gl == 0) atomicOr(a.status, kStatOverflow);
+      continue;
+    }
+    if constexpr (G == 32) {
+      if (N > 32) {
+        run_system<32, 2>(S, a, b, N);
+        continue;
+      }
+    }
+    run_system<G, 1>(S, a, b, N);
+  }
+}
+
+// F32C with 32 lanes or lanes by size keeps the state in registers.
+constexpr bool in_registers(int G, bool exact) { return !exact && (G == 0 || G == 32); }
+
 // One persistent launch of BW warps per block.  G = 8, 16, 32: every system
 // gets G lanes (32 / G systems per warp at a time).  G = 0: lanes by size —
 // a warp takes the systems of more than 16 bodies one at a time, then two of
@@ -444,15 +623,25 @@ ensemble_kernel(EnsArgs a) {
   wait_for_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if constexpr (G != 0) {
+  if constexpr (in_registers(G, kExact)) {
+    unsigned char* base = smem_raw + warp * sizeof(SourceSmem);
+    drain_f32c<32>(reinterpret_cast<SourceSmem*>(base), a, 0, G == 32 ? a.nsys : a.n32, a.queue,
+                   kMaxSys);
+    if constexpr (G == 0) {
+      drain_f32c<16>(reinterpret_cast<SourceSmemT<16>*>(base) + (lane >> 4), a, a.n32, a.n16,
+                     a.queue + 1, 16);
+      drain_f32c<8>(reinterpret_cast<SourceSmemT<8>*>(base) + (lane >> 3), a, a.n16, a.nsys,
+                    a.queue + 2, 8);
+    }
+  } else if constexpr (G != 0) {
     GroupSmem* S = reinterpret_cast<GroupSmem*>(smem_raw) + warp * (32 / G) + lane / G;
-    drain<G, kExact, (G == 32 ? 1 : 2)>(S, a, 0, a.nsys, a.queue, kMaxSys);
+    drain<G, kExact>(S, a, 0, a.nsys, a.queue, kMaxSys);
   } else {
     unsigned char* base = smem_raw + warp * sizeof(GroupSmem);
-    drain<32, kExact, 1>(reinterpret_cast<GroupSmem*>(base), a, 0, a.n32, a.queue, kMaxSys);
-    drain<16, kExact, 1>(reinterpret_cast<GroupSmemT<16>*>(base) + (lane >> 4), a, a.n32, a.n16,
+    drain<32, kExact>(reinterpret_cast<GroupSmem*>(base), a, 0, a.n32, a.queue, kMaxSys);
+    drain<16, kExact>(reinterpret_cast<GroupSmemT<16>*>(base) + (lane >> 4), a, a.n32, a.n16,
                       a.queue + 1, 16);
-    drain<8, kExact, 1>(reinterpret_cast<GroupSmemT<8>*>(base) + (lane >> 3), a, a.n16, a.nsys,
+    drain<8, kExact>(reinterpret_cast<GroupSmemT<8>*>(base) + (lane >> 3), a, a.n16, a.nsys,
                      a.queue + 2, 8);
   }
 }
@@ -511,7 +700,8 @@ int prepare(phys_ctx* c, const phys_params* p, int code, LaunchCfg* cfg) {
   cfg->k = pick(G, bw, exact);
   cfg->block = 32 * bw;
   const int groups_per_warp = G == 0 ? 1 : 32 / G;
-  cfg->smem = sizeof(GroupSmem) * groups_per_warp * bw;
+  cfg->smem = (in_registers(G, exact) ? sizeof(SourceSmem) : sizeof(GroupSmem)) *
+              groups_per_warp * bw;
   PHYS_CUDA(c, cudaFuncSetAttribute(cfg->k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)cfg->smem));
   int per_sm = 0;
