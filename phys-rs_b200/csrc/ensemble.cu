@@ -491,11 +491,10 @@ __device__ void drain(S_t* S, const EnsArgs& a, int lo, int hi, int* ctr, int ma
 // state in the lanes' registers: shared memory holds the sources only, and a
 // step reads and writes no f64 array (30 of the 60 shared-memory accesses per
 // body and step that are not pair sources).  kBodies = 2: systems of 33..64
-// bodies.  Bound by the packed pair terms, about 64 % of their rate on 12
-// warps an SM (150 registers; 16 warps at 128 registers do the same at 16384
-// systems and worse at 2000, 20 warps worse at both).  200 steps of 16384
-// systems of 3..64 bodies 5.74 -> 5.46 ms, 4096 of 3..32 0.88 -> 0.76, 16384
-// of 3..24 1.90 -> 1.65.
+// bodies.  Bound by the packed pair terms, about 64 % of their rate on 16
+// warps an SM (128 registers; 12 warps at 150 take 2 to 8 % longer, 20 warps
+// 3 %).  300 steps of 16384 systems of 3..64 bodies 8.13 -> 7.61 ms, of 3..32
+// 3.30 -> 2.80, of 3..24 2.59 -> 2.08; 2000 systems of 3..64 2.66 -> 1.98.
 template <int G, int kBodies, class S_t>
 __device__ __forceinline__ void run_system(S_t* S, const EnsArgs& a, int64_t b, int N) {
   const int gl = (threadIdx.x & 31) % G;
@@ -618,7 +617,7 @@ constexpr bool in_registers(int G, bool exact) { return !exact && (G == 0 || G =
 // a warp takes the systems of more than 16 bodies one at a time, then two of
 // 9..16 bodies at a time (16 lanes each), then four of at most 8.
 template <int G, int BW, bool kExact>
-__global__ void __launch_bounds__(32 * BW)
+__global__ void __launch_bounds__(32 * BW, in_registers(G, kExact) ? 16 / BW : 1)
 ensemble_kernel(EnsArgs a) {
   wait_for_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -709,6 +708,11 @@ int prepare(phys_ctx* c, const phys_params* p, int code, LaunchCfg* cfg) {
                                                              cfg->smem));
   int sms = 148;
   PHYS_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  // more than 12 warps an SM only when every one gets a system: a fourth block
+  // on some SMs alone makes the longest systems there the last to finish (300
+  // steps of 2000 systems of 3..64 bodies: 2.55 ms against 1.98)
+  if (in_registers(G, exact))
+    while (per_sm * bw > 12 && c->ens_nsys < (int64_t)per_sm * bw * sms) --per_sm;
   const int64_t groups_per_block = (int64_t)groups_per_warp * bw;
   cfg->grid = std::min<int64_t>((int64_t)std::max(per_sm, 1) * sms,
                                 ceil_div(c->ens_nsys, groups_per_block));
