@@ -151,8 +151,11 @@ int d2h(phys_ctx* c, double* dst, const double* src, int64_t n) {
 // `first` on (the state is one allocation, cap apart; null: zeros).  Small
 // states are packed into the pinned staging buffer at `at` and go out in one
 // copy: a copy call costs 2 to 4 us whatever its size (100 bodies: 7 copies
-// and 9 memsets of a system call against 3 calls).
-constexpr int64_t kPackBytes = int64_t(4) << 20;
+// and 9 memsets of a system call against 3 calls; a host tick of 300 bodies
+// 153 -> 137 us).  Beyond a quarter MB the packing costs what it saves, and
+// page-locked arrays go out faster in place (a host tick of 20000 bodies 770
+// us against 830 packed, of 60000 995 against 1228).
+constexpr int64_t kPackBytes = int64_t(256) << 10;
 
 bool packs(int64_t n, int rows) { return 8 * n * rows <= kPackBytes; }
 
