@@ -412,7 +412,7 @@ walk2_kernel(int q64, int n, int nnodes, const Rec32x2* __restrict__ w, const Bo
 // bodies, 0.86 / 1.21 at 32768, 1.3 / 1.54 at 65536.
 //
 // Bound by the terms: 3300 entries a warp at 300 000 bodies (2100 per target),
-// 38 FP64 instructions and about as many others each, at 55 % of the FP64
+// 38 FP64 instructions and about as many others each, at 47 % of the FP64
 // pipe; without them the traversal takes 1.1 of 5.0 ms.  Two entries at a time
 // and 24 warps an SM do best on a full chip (four: 17.3 ms at 2^20), four with
 // 16 warps when the tasks' tails show (0.32 against 0.34 ms at 10 000).  One
