@@ -89,6 +89,8 @@ struct TopTree {
   int32_t* task = nullptr;           // node of each task
   int4* top = nullptr;               // node, task (-1: upper cell), depth, -
   const int32_t* parent = nullptr;   // of every node
+  int32_t* order = nullptr;          // tasks by falling size
+  int32_t* queue = nullptr;          // next (place in order, 32 targets) to be taken
 };
 
 struct BhTree {

@@ -968,6 +968,27 @@ top_tree_kernel(int64_t nnodes, const int4* __restrict__ link, const int32_t* __
   }
 }
 
+// The tasks by falling number of bodies: the walk takes the long ones first.
+__global__ void __launch_bounds__(512)
+task_order_kernel(int max_tasks, int max_top, const int32_t* __restrict__ counts,
+                  const int4* __restrict__ link, const int32_t* __restrict__ task,
+                  int32_t* __restrict__ order, int32_t* __restrict__ queue) {
+  wait_for_previous();
+  __shared__ int bodies[512];
+  const int i = threadIdx.x, c = *counts, nt = c >> 16;
+  if (i == 0) *queue = 0;
+  if (nt > max_tasks || (c & 0xffff) > max_top) return;  // walked as one task
+  if (i < nt) {
+    const int4 l = link[task[i]];
+    bodies[i] = l.z - l.y;
+  }
+  __syncthreads();
+  if (i >= nt) return;
+  int at = 0;
+  for (int k = 0; k < nt; ++k) at += bodies[k] > bodies[i] || (bodies[k] == bodies[i] && k < i);
+  order[at] = i;
+}
+
 // Breadth-first order: node ids stably sorted by depth (one radix pass on
 // pre-order input); inverse map.
 __global__ void depth_key_kernel(int64_t nnodes, const int4* __restrict__ link,
@@ -1307,17 +1328,27 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
       top.max_top = 4096;
       PHYS_TRY(ws_alloc(c, WS_NCOUNT, nnodes + 1, &cnt2));
       PHYS_TRY(ws_alloc(c, WS_GROUP_OFF, nnodes + 1, &off2));
-      PHYS_TRY(ws_alloc(c, WS_GROUPS, 4 * top.max_top + top.max_tasks, &lists));
+      PHYS_TRY(ws_alloc(c, WS_GROUPS, 4 * top.max_top + 2 * top.max_tasks + 1, &lists));
       top.top = reinterpret_cast<int4*>(lists);
       top.task = lists + 4 * top.max_top;
+      top.order = top.task + top.max_tasks;
+      top.queue = top.order + top.max_tasks;
       top.counts = off2 + nnodes;
       top.parent = parent;
-      const int most = (int)(n / 8);
+      // finer tasks balance better and cost more walking and adding: 20000
+      // bodies 0.41 / 0.44 / 0.48 ms with n/16 / n/12 / n/8, 32768 0.62 / 0.58
+      // with n/16 / n/8, 65536 1.10 / 1.05 with n/8 / n/5; and they must fit
+      // (nested cells make up to ten tasks and more per n/16 of a disk; with
+      // too many the tree is walked as one task, 24000 bodies 0.96 ms for 0.49)
+      const int room = top.max_tasks;
+      const int most = (int)(n / (room >= 256 ? 16 : room >= 160 ? 12 : room >= 80 ? 8 : 5));
       PHYS_LAUNCH(c, top_tree_kernel<false>, grid_for(nnodes + 1), kBlock, 0, nnodes, link, parent,
                   most, cnt2, off2, top.max_tasks, top.max_top, top.task, top.top);
       PHYS_TRY(scan_exclusive_i32(c, cnt2, off2, nnodes + 1));
       PHYS_LAUNCH(c, top_tree_kernel<true>, grid_for(nnodes + 1), kBlock, 0, nnodes, link, parent,
                   most, cnt2, off2, top.max_tasks, top.max_top, top.task, top.top);
+      PHYS_LAUNCH(c, task_order_kernel, 1, 512, 0, top.max_tasks, top.max_top, top.counts, link,
+                  top.task, top.order, top.queue);
     }
   }
 #ifndef WALK_PAIRED

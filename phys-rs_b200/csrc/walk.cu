@@ -21,6 +21,7 @@
 //   F32C       f32 pair terms on double-float relative coordinates
 //              r = (hi_j - hi_i) + (lo_j - lo_i); f32 partial sums folded
 //              into a (hi, lo) accumulator with two-sum every 16 nodes.
+#include <algorithm>
 #include <type_traits>
 
 #include "bh.cuh"
@@ -404,21 +405,24 @@ walk2_kernel(int q64, int n, int nnodes, const Rec32x2* __restrict__ w, const Bo
 // may then lie outside the cube), the warp takes the reference's f64 test.
 //
 // Few targets would leave most of the chip idle behind the longest walk, so
-// up to 65536 of them are split: the children of the cells of more than n/8
-// bodies become tasks of their own (grid.y; n/16 to n/64 make more tasks than
-// they save walking), each leaving its cell's contribution to each target in
-// `part`; exact_combine_kernel walks the cells above and sums them with the
-// reference's nesting.  Split against whole walks: 0.32 / 0.96 ms at 10 000
-// bodies, 0.86 / 1.21 at 32768, 1.3 / 1.54 at 65536.
+// up to 131072 of them are split: the children of the cells of more than a
+// 16th to a 5th of the bodies become tasks of their own, each leaving its
+// cell's contribution to each target in `part`; exact_combine_kernel walks
+// the cells above and sums them with the reference's nesting.  Warps take
+// pairs of a task and 32 targets from a queue, large tasks first: the longest
+// pair (halo targets, spread out, against a dense cell) takes 0.27 ms at
+// 10 000 bodies and n/8, so it must not start last.  Split against whole
+// walks: 0.29 / 0.96 ms at 10 000 bodies, 0.58 / 1.21 at 32768, 1.05 / 1.54 at
+// 65536, 1.57 / 1.89 at 100 000, 4.8 / 4.9 at 300 000 (and a block per pair in
+// grid order: 0.32 at 10 000, 0.86 at 32768, 1.27 at 65536).
 //
 // Bound by the terms: 3300 entries a warp at 300 000 bodies (2100 per target),
 // 38 FP64 instructions and about as many others each, at 47 % of the FP64
 // pipe; without them the traversal takes 1.1 of 5.0 ms.  Two entries at a time
 // and 24 warps an SM do best on a full chip (four: 17.3 ms at 2^20), four with
-// 16 warps when the tasks' tails show (0.32 against 0.34 ms at 10 000).  One
+// 16 warps when the tasks' tails show (0.32 against 0.34 ms at 10 000, in grid order).  One
 // walk per target, a node per step and its term evaluated in place, took 19.8
-// ms at 2^20 bodies against 15.5, and 0.44 against 0.32 at 10 000 (split, a
-// node per step).
+// ms at 2^20 bodies against 15.5; split, a node per step, 0.44 at 10 000.
 // ---------------------------------------------------------------------------
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kXQ = 32;  // queue entries per warp
@@ -541,10 +545,7 @@ walk_exact_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const float4
   __shared__ int qnode[kXWarps][kXQ];
   __shared__ unsigned qmask[kXWarps][kXQ];    // lanes that take it
   __shared__ unsigned qlevels[kXWarps][kXQ];  // 0: those of the entry before
-  const int task = kWhole ? 0 : (int)blockIdx.y;
   const int ntask = kWhole ? 1 : top_tasks(top);
-  if (task >= ntask) return;
-  const int root = ntask == 1 ? 0 : top.task[task];
   const double theta2 = hdr->theta2, half = hdr->half;
   for (int d = threadIdx.x; d < kMaxLevels; d += blockDim.x) {
     s2d[d] = hdr->s2[d];
@@ -556,231 +557,247 @@ walk_exact_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const float4
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned bit = 1u << lane;
-  const int64_t p = q0 + blockIdx.x * (int64_t)kXTargets + threadIdx.x;  // targets [q0, n)
-  const bool valid = p < n;
-  const int p0 = (int)(p - lane);
-  const ExactTarget t = exact_target(body64, p, valid, G);
-  const bool fast = __all_sync(kFull, scale_mass_ok(t.gm)) && walk_in_range(hdr, nbody, eps2);
-  const double ih = 1.0 / half;
-  const float fx = (float)((t.x - hdr->center[0]) * ih), fy = (float)((t.y - hdr->center[1]) * ih),
-              fz = (float)((t.z - hdr->center[2]) * ih);
-  const bool coarse =
-      hdr->min_mass >= 0.0 &&
-      __all_sync(kFull, !valid || (isfinite(fx) && isfinite(fy) && isfinite(fz)));
-  // the box around the warp's targets
-  float bl[3] = {valid ? fx : INFINITY, valid ? fy : INFINITY, valid ? fz : INFINITY};
-  float bh[3] = {valid ? fx : -INFINITY, valid ? fy : -INFINITY, valid ? fz : -INFINITY};
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      bl[k] = fminf(bl[k], __shfl_xor_sync(kFull, bl[k], o));
-      bh[k] = fmaxf(bh[k], __shfl_xor_sync(kFull, bh[k], o));
-    }
-  }
-
-  NestedSum sum;
-  double outer[kMaxLevels + 1][3];
   unsigned ninter = 0;
-  int cnt = 0;
-  unsigned* const qm = qmask[wid];
-  unsigned* const ql = qlevels[wid];
-  int* const qn = qnode[wid];
-  double4* const sr = srec[wid];
-  // add the queue's terms: bit k of `on`: entry k is the lane's, of `ev`: it
-  // changes levels
-  auto terms = [&](auto quick, unsigned on, unsigned ev) {
-    constexpr bool kQuick = decltype(quick)::value;
-#pragma unroll 1
-    for (int k0 = 0; k0 < cnt; k0 += kXU) {
-      double rx[kXU], ry[kXU], rz[kXU], w[kXU];
+  // a warp's work: one task for 32 of the targets [q0, n)
+  const int nrun = (int)((n - q0 + 31) / 32);
+  for (;;) {
+    int task = 0, run = blockIdx.x * kXWarps + wid;
+    if (!kWhole) {
+      int it = 0;
+      if (lane == 0) it = atomicAdd(top.queue, 1);
+      it = __shfl_sync(kFull, it, 0);
+      task = it / nrun;
+      run = it - task * nrun;
+    }
+    if (run >= nrun || task >= ntask) break;
+    if (!kWhole && ntask > 1) task = top.order[task];
+    const int root = ntask == 1 ? 0 : top.task[task];
+    const int64_t p = q0 + run * 32 + lane;
+    const bool valid = p < n;
+    const int p0 = (int)(p - lane);
+    const ExactTarget t = exact_target(body64, p, valid, G);
+    const bool fast = __all_sync(kFull, scale_mass_ok(t.gm)) && walk_in_range(hdr, nbody, eps2);
+    const double ih = 1.0 / half;
+    const float fx = (float)((t.x - hdr->center[0]) * ih), fy = (float)((t.y - hdr->center[1]) * ih),
+                fz = (float)((t.z - hdr->center[2]) * ih);
+    const bool coarse =
+        hdr->min_mass >= 0.0 &&
+        __all_sync(kFull, !valid || (isfinite(fx) && isfinite(fy) && isfinite(fz)));
+    // the box around the warp's targets
+    float bl[3] = {valid ? fx : INFINITY, valid ? fy : INFINITY, valid ? fz : INFINITY};
+    float bh[3] = {valid ? fx : -INFINITY, valid ? fy : -INFINITY, valid ? fz : -INFINITY};
 #pragma unroll
-      for (int u = 0; u < kXU; ++u)
-        w[u] = exact_weight<kQuick>(t, sr[k0 + u], eps2, rx[u], ry[u], rz[u]);
+    for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-      for (int u = 0; u < kXU; ++u) {
-        if (ev >> u & 1) {
-          const unsigned l = ql[k0 + u];
-          sum.close_to((int)(l & 0xffff), outer);
-          sum.open_to((int)(l >> 17), outer);
-        }
-        // a lane outside the mask adds 0, which changes no sum
-        const bool mine = on >> u & 1;
-        const double wu = mine ? w[u] : 0.0;
-        if (!kQuick && !mine) rx[u] = ry[u] = rz[u] = 0.0;  // may be infinite
-        sum.add(xmul(rx[u], wu), xmul(ry[u], wu), xmul(rz[u], wu));
+      for (int k = 0; k < 3; ++k) {
+        bl[k] = fminf(bl[k], __shfl_xor_sync(kFull, bl[k], o));
+        bh[k] = fmaxf(bh[k], __shfl_xor_sync(kFull, bh[k], o));
       }
-      on >>= kXU;
-      ev >>= kXU;
     }
-  };
-  auto drain = [&]() {
-    __syncwarp();
-    unsigned on = lane < cnt ? qm[lane] : 0;
-    const unsigned ev = __ballot_sync(kFull, lane < cnt && ql[lane] != 0);
-    sr[lane] = rec64[qn[min(lane, cnt - 1)]];
-    // transpose: from a lane mask per entry to an entry mask per lane
-#pragma unroll
-    for (int j = 16; j > 0; j >>= 1) {
-      const unsigned m = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu
-                                     : j == 2 ? 0x33333333u : 0x55555555u;
-      const unsigned y = __shfl_xor_sync(kFull, on, j);
-      on = lane & j ? (on & ~m) | (y >> j & m) : (on & m) | (y & m) << j;
-    }
-    __syncwarp();
-    if (fast)
-      terms(std::true_type{}, on, ev);
-    else
-      terms(std::false_type{}, on, ev);
-    __syncwarp();
-    cnt = 0;
-  };
 
-  // the task's cells above were all opened by the lane?
-  const int base = __float_as_int(wx[root].w) & kMetaDepth;
-  bool in = valid;
-  if (!kWhole && valid) {
-    for (int k = root, d = base - 1; d >= 0; --d) {
-      k = top.parent[k];
-      in = in && (k == 0 || (__float_as_int(wx[k].w) & kMetaGate)) &&
-           exact_open(rec64[k], t, s2d[d], theta2);
+    NestedSum sum;
+    double outer[kMaxLevels + 1][3];
+    int cnt = 0;
+    unsigned* const qm = qmask[wid];
+    unsigned* const ql = qlevels[wid];
+    int* const qn = qnode[wid];
+    double4* const sr = srec[wid];
+    // add the queue's terms: bit k of `on`: entry k is the lane's, of `ev`: it
+    // changes levels
+    auto terms = [&](auto quick, unsigned on, unsigned ev) {
+      constexpr bool kQuick = decltype(quick)::value;
+#pragma unroll 1
+      for (int k0 = 0; k0 < cnt; k0 += kXU) {
+        double rx[kXU], ry[kXU], rz[kXU], w[kXU];
+#pragma unroll
+        for (int u = 0; u < kXU; ++u)
+          w[u] = exact_weight<kQuick>(t, sr[k0 + u], eps2, rx[u], ry[u], rz[u]);
+#pragma unroll
+        for (int u = 0; u < kXU; ++u) {
+          if (ev >> u & 1) {
+            const unsigned l = ql[k0 + u];
+            sum.close_to((int)(l & 0xffff), outer);
+            sum.open_to((int)(l >> 17), outer);
+          }
+          // a lane outside the mask adds 0, which changes no sum
+          const bool mine = on >> u & 1;
+          const double wu = mine ? w[u] : 0.0;
+          if (!kQuick && !mine) rx[u] = ry[u] = rz[u] = 0.0;  // may be infinite
+          sum.add(xmul(rx[u], wu), xmul(ry[u], wu), xmul(rz[u], wu));
+        }
+        on >>= kXU;
+        ev >>= kXU;
+      }
+    };
+    auto drain = [&]() {
+      __syncwarp();
+      unsigned on = lane < cnt ? qm[lane] : 0;
+      const unsigned ev = __ballot_sync(kFull, lane < cnt && ql[lane] != 0);
+      sr[lane] = rec64[qn[min(lane, cnt - 1)]];
+      // transpose: from a lane mask per entry to an entry mask per lane
+#pragma unroll
+      for (int j = 16; j > 0; j >>= 1) {
+        const unsigned m = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu
+                                       : j == 2 ? 0x33333333u : 0x55555555u;
+        const unsigned y = __shfl_xor_sync(kFull, on, j);
+        on = lane & j ? (on & ~m) | (y >> j & m) : (on & m) | (y & m) << j;
+      }
+      __syncwarp();
+      if (fast)
+        terms(std::true_type{}, on, ev);
+      else
+        terms(std::false_type{}, on, ev);
+      __syncwarp();
+      cnt = 0;
+    };
+
+    // the task's cells above were all opened by the lane?
+    const int base = __float_as_int(wx[root].w) & kMetaDepth;
+    bool in = valid;
+    if (!kWhole && valid) {
+      for (int k = root, d = base - 1; d >= 0; --d) {
+        k = top.parent[k];
+        in = in && (k == 0 || (__float_as_int(wx[k].w) & kMetaGate)) &&
+             exact_open(rec64[k], t, s2d[d], theta2);
+      }
     }
-  }
-  const unsigned start = __ballot_sync(kFull, in);
-  sum.init(base);
-  // A frame per depth: in lanes 8g..8g+7 the children of the g-th of up to
-  // four opened cells of the frame above (set `above`), with the targets that
-  // take (tk) and open (op) each.  The walk goes through a group of lanes
-  // [pos, end) at a time; the other groups wait until it comes to their cell.
-  int4 frame[kMaxLevels];     // cell, tk, op, pos | end << 8
-  unsigned above[kMaxLevels + 1];
-  int d = base, cn = lane == 0 ? root : -1, pos = 0, end = 8;
-  unsigned tk, op, act = start;
-  auto classify = [&]() {
-    tk = op = 0;
-    bool mixed = false;
-    float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2 bd = band[d];
-    if (cn >= 0) {
-      A = __ldg(&wx[cn]);
-      const int meta = __float_as_int(A.w);
-      if ((meta & kMetaGate) || cn == 0) {
-        if (meta & kMetaLeaf) {  // every target but the body itself
-          const unsigned self = (unsigned)(__float_as_int(A.x) - p0);
-          tk = self < 32 ? act & ~(1u << self) : act;
-        } else {
-          const float nx = fmaxf(fmaxf(bl[0] - A.x, A.x - bh[0]), 0.f),
-                      ny = fmaxf(fmaxf(bl[1] - A.y, A.y - bh[1]), 0.f),
-                      nz = fmaxf(fmaxf(bl[2] - A.z, A.z - bh[2]), 0.f);
-          const float mx = fmaxf(A.x - bl[0], bh[0] - A.x), my = fmaxf(A.y - bl[1], bh[1] - A.y),
-                      mz = fmaxf(A.z - bl[2], bh[2] - A.z);
-          const float near2 = fmaf(nx, nx, fmaf(ny, ny, nz * nz)),
-                      far2 = fmaf(mx, mx, fmaf(my, my, mz * mz));
-          if (coarse && cn != 0 && near2 > bd.y && far2 >= near2)
-            tk = act;
-          else if (coarse && cn != 0 && far2 < bd.x)
-            op = act;
-          else
-            mixed = true;
+    const unsigned start = __ballot_sync(kFull, in);
+    sum.init(base);
+    // A frame per depth: in lanes 8g..8g+7 the children of the g-th of up to
+    // four opened cells of the frame above (set `above`), with the targets that
+    // take (tk) and open (op) each.  The walk goes through a group of lanes
+    // [pos, end) at a time; the other groups wait until it comes to their cell.
+    int4 frame[kMaxLevels];     // cell, tk, op, pos | end << 8
+    unsigned above[kMaxLevels + 1];
+    int d = base, cn = lane == 0 ? root : -1, pos = 0, end = 8;
+    unsigned tk, op, act = start;
+    auto classify = [&]() {
+      tk = op = 0;
+      bool mixed = false;
+      float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float2 bd = band[d];
+      if (cn >= 0) {
+        A = __ldg(&wx[cn]);
+        const int meta = __float_as_int(A.w);
+        if ((meta & kMetaGate) || cn == 0) {
+          if (meta & kMetaLeaf) {  // every target but the body itself
+            const unsigned self = (unsigned)(__float_as_int(A.x) - p0);
+            tk = self < 32 ? act & ~(1u << self) : act;
+          } else {
+            const float nx = fmaxf(fmaxf(bl[0] - A.x, A.x - bh[0]), 0.f),
+                        ny = fmaxf(fmaxf(bl[1] - A.y, A.y - bh[1]), 0.f),
+                        nz = fmaxf(fmaxf(bl[2] - A.z, A.z - bh[2]), 0.f);
+            const float mx = fmaxf(A.x - bl[0], bh[0] - A.x), my = fmaxf(A.y - bl[1], bh[1] - A.y),
+                        mz = fmaxf(A.z - bl[2], bh[2] - A.z);
+            const float near2 = fmaf(nx, nx, fmaf(ny, ny, nz * nz)),
+                        far2 = fmaf(mx, mx, fmaf(my, my, mz * mz));
+            if (coarse && cn != 0 && near2 > bd.y && far2 >= near2)
+              tk = act;
+            else if (coarse && cn != 0 && far2 < bd.x)
+              op = act;
+            else
+              mixed = true;
+          }
         }
       }
-    }
 #pragma unroll 1
-    for (unsigned mm = __ballot_sync(kFull, mixed); mm; mm &= mm - 1) {
-      const int j = __ffs(mm) - 1;
-      const float rx = __shfl_sync(kFull, A.x, j) - fx, ry = __shfl_sync(kFull, A.y, j) - fy,
-                  rz = __shfl_sync(kFull, A.z, j) - fz;
-      const unsigned a = __shfl_sync(kFull, act, j);
-      const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-      bool open = d2 < bd.x;
-      if (__any_sync(kFull, (a & bit) && !(coarse && (d2 < bd.x || d2 > bd.y))))
-        open = exact_open(rec64[__shfl_sync(kFull, cn, j)], t, s2d[d], theta2);
-      const unsigned o = __ballot_sync(kFull, open) & a;
-      if (lane == j) {
-        op = o;
-        tk = a & ~o;
+      for (unsigned mm = __ballot_sync(kFull, mixed); mm; mm &= mm - 1) {
+        const int j = __ffs(mm) - 1;
+        const float rx = __shfl_sync(kFull, A.x, j) - fx, ry = __shfl_sync(kFull, A.y, j) - fy,
+                    rz = __shfl_sync(kFull, A.z, j) - fz;
+        const unsigned a = __shfl_sync(kFull, act, j);
+        const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+        bool open = d2 < bd.x;
+        if (__any_sync(kFull, (a & bit) && !(coarse && (d2 < bd.x || d2 > bd.y))))
+          open = exact_open(rec64[__shfl_sync(kFull, cn, j)], t, s2d[d], theta2);
+        const unsigned o = __ballot_sync(kFull, open) & a;
+        if (lane == j) {
+          op = o;
+          tk = a & ~o;
+        }
       }
-    }
-    frame[d] = make_int4(cn, (int)tk, (int)op, 0);
-    above[d + 1] = 0;
-  };
-  if (start) classify();
-  // low: the least depth of the path since the last entry
-  int low = base, steps = 0;
-  while (start) {
-    const unsigned group = (unsigned)((1ull << end) - (1ull << pos));
-    const unsigned all_op = __ballot_sync(kFull, op != 0);
-    const unsigned opens = all_op & group, takes = __ballot_sync(kFull, tk != 0) & group;
-    const unsigned put = opens ? takes & (opens ^ (opens - 1)) : takes;  // up to the first opened
-    low = min(low, d);
-    if (put) {
-      if (put & bit) {
-        const int r = __popc(put & (bit - 1));
-        qn[cnt + r] = cn;
-        // levels: the one the open sums close to, then the entry's own
-        qm[cnt + r] = tk;
-        ql[cnt + r] = r == 0 ? (unsigned)(low | 0x10000 | d << 17) : 0u;
-        ninter += __popc(tk);
+      frame[d] = make_int4(cn, (int)tk, (int)op, 0);
+      above[d + 1] = 0;
+    };
+    if (start) classify();
+    // low: the least depth of the path since the last entry
+    int low = base, steps = 0;
+    while (start) {
+      const unsigned group = (unsigned)((1ull << end) - (1ull << pos));
+      const unsigned all_op = __ballot_sync(kFull, op != 0);
+      const unsigned opens = all_op & group, takes = __ballot_sync(kFull, tk != 0) & group;
+      const unsigned put = opens ? takes & (opens ^ (opens - 1)) : takes;  // up to the first opened
+      low = min(low, d);
+      if (put) {
+        if (put & bit) {
+          const int r = __popc(put & (bit - 1));
+          qn[cnt + r] = cn;
+          // levels: the one the open sums close to, then the entry's own
+          qm[cnt + r] = tk;
+          ql[cnt + r] = r == 0 ? (unsigned)(low | 0x10000 | d << 17) : 0u;
+          ninter += __popc(tk);
+        }
+        low = d;
+        cnt += __popc(put);
+        if (cnt > kXQ - 8) drain();
       }
-      low = d;
-      cnt += __popc(put);
-      if (cnt > kXQ - 8) drain();
-    }
-    if (!opens) {  // group done: on with the frame above
-      if (d == base) break;
-      --d;
-      const int4 f = frame[d];
-      cn = f.x;
-      tk = (unsigned)f.y;
-      op = (unsigned)f.z;
-      pos = f.w & 0xff;
-      end = f.w >> 8;
-      continue;
-    }
-    const int j = __ffs(opens) - 1;
-    frame[d].w = (j + 1) | end << 8;
-    unsigned done = above[d + 1];
-    if (done >> j & 1) {  // its children are in the frame below already
-      pos = 8 * __popc(done & ((1u << j) - 1));
-      ++d;
-      const int4 f = frame[d];
-      cn = f.x;
-      tk = (unsigned)f.y;
-      op = (unsigned)f.z;
-    } else {  // the children of this and of the next opened cells, four at most
-      if (d + 1 >= kMaxLevels || ++steps > nnodes) {  // malformed tree: report, never spin
-        if (lane == 0) atomicOr(status, kStatOverflow);
-        break;
+      if (!opens) {  // group done: on with the frame above
+        if (d == base) break;
+        --d;
+        const int4 f = frame[d];
+        cn = f.x;
+        tk = (unsigned)f.y;
+        op = (unsigned)f.z;
+        pos = f.w & 0xff;
+        end = f.w >> 8;
+        continue;
       }
-      const unsigned s0 = all_op & ~((1u << j) - 1), s1 = s0 & (s0 - 1), s2 = s1 & (s1 - 1),
-                     s3 = s2 & (s2 - 1);
-      done = s0 & ~(s3 & (s3 - 1));
-      const unsigned mine = lane < 16 ? (lane < 8 ? s0 : s1) : (lane < 24 ? s2 : s3);
-      const int from = __ffs(mine) - 1;
-      const int cell = __shfl_sync(kFull, cn, from & 31);
-      act = __shfl_sync(kFull, op, from & 31);
-      cn = -1;
-      if (mine) cn = __ldg(&kids[cell].id[lane & 7]);
-      if (cn <= cell || cn >= nnodes) cn = -1;
-      above[d + 1] = done;
-      ++d;
-      classify();
-      pos = 0;
+      const int j = __ffs(opens) - 1;
+      frame[d].w = (j + 1) | end << 8;
+      unsigned done = above[d + 1];
+      if (done >> j & 1) {  // its children are in the frame below already
+        pos = 8 * __popc(done & ((1u << j) - 1));
+        ++d;
+        const int4 f = frame[d];
+        cn = f.x;
+        tk = (unsigned)f.y;
+        op = (unsigned)f.z;
+      } else {  // the children of this and of the next opened cells, four at most
+        if (d + 1 >= kMaxLevels || ++steps > nnodes) {  // malformed tree: report, never spin
+          if (lane == 0) atomicOr(status, kStatOverflow);
+          break;
+        }
+        const unsigned s0 = all_op & ~((1u << j) - 1), s1 = s0 & (s0 - 1), s2 = s1 & (s1 - 1),
+                       s3 = s2 & (s2 - 1);
+        done = s0 & ~(s3 & (s3 - 1));
+        const unsigned mine = lane < 16 ? (lane < 8 ? s0 : s1) : (lane < 24 ? s2 : s3);
+        const int from = __ffs(mine) - 1;
+        const int cell = __shfl_sync(kFull, cn, from & 31);
+        act = __shfl_sync(kFull, op, from & 31);
+        cn = -1;
+        if (mine) cn = __ldg(&kids[cell].id[lane & 7]);
+        if (cn <= cell || cn >= nnodes) cn = -1;
+        above[d + 1] = done;
+        ++d;
+        classify();
+        pos = 0;
+      }
+      end = pos + 8;
     }
-    end = pos + 8;
+    if (cnt) drain();
+    sum.close_to(base, outer);
+    if (kWhole) {
+      if (valid)
+        exact_store(sum.x, sum.y, sum.z, body64[p].w, perm[p], want_force, ox, oy, oz, status);
+    } else if (in) {
+      double* o = part + ((size_t)task * (size_t)(n - q0) + (size_t)(p - q0)) * 3;
+      o[0] = sum.x;
+      o[1] = sum.y;
+      o[2] = sum.z;
+    }
+    if (kWhole) break;
   }
-  if (cnt) drain();
-  sum.close_to(base, outer);
   warp_count(ninter, counter);
-  if (kWhole) {
-    if (valid)
-      exact_store(sum.x, sum.y, sum.z, body64[p].w, perm[p], want_force, ox, oy, oz, status);
-  } else if (in) {
-    double* o = part + ((size_t)task * (size_t)(n - q0) + (size_t)(p - q0)) * 3;
-    o[0] = sum.x;
-    o[1] = sum.y;
-    o[2] = sum.z;
-  }
 }
 
 // A target's force from its tasks' contributions: the walk over the upper
@@ -868,8 +885,10 @@ int exact_walk_tasks(const phys_ctx* c, int64_t n) {
   int64_t q0 = 0, q1 = n;
   target_range(c, n, q0, q1);
   const int64_t nt = q1 - q0;
-  // `part` holds 24 bytes per task and target: at most 100 MB
-  return nt > 0 && nt <= 65536 ? (int)min64(512, (int64_t(1) << 22) / nt) : 0;
+  // `part` holds 24 bytes per task and target: at most 100 MB, 200 MB for
+  // more than 65536 targets (64 tasks)
+  if (nt <= 0 || nt > 131072) return 0;
+  return (int)std::max<int64_t>(64, min64(512, (int64_t(1) << 22) / nt));
 }
 
 int bh_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force, double* ox,
@@ -891,7 +910,8 @@ int bh_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force,
     if (tasks > 0) {
       double* part = nullptr;
       PHYS_TRY(ws_alloc(c, WS_DIRECT_PART, 3 * nt * tasks, &part));
-      PHYS_LAUNCH(c, walk_exact_kernel<false>, dim3(xgrid, tasks), 32 * kXWarps, 0, q0, q1, n,
+      PHYS_LAUNCH(c, walk_exact_kernel<false>, (int)min64(148 * 4, (int64_t)xgrid * tasks),
+                  32 * kXWarps, 0, q0, q1, n,
                   (int)t.nnodes, t.wx, t.kids, t.rec64, t.body64, t.perm, t.hdr, t.top, p->G, eps2,
                   (int)want_force, part, ox, oy, oz, c->d_counter, c->d_status);
       PHYS_LAUNCH(c, exact_combine_kernel, (int)ceil_div(nt > 0 ? nt : 1, kStage), kStage, 0, q0, q1, t.wx, t.rec64,

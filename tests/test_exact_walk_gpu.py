@@ -74,3 +74,24 @@ def test_whole_walk_ranges(ctx, kind, theta):
     ctx.upload(pos, None, m)
     f = ctx.gravity_forces(exact(theta, eps))
     assert np.array_equal(f, oracle.bh_forces(pos, m, 1.0, eps, theta))
+
+
+@pytest.mark.parametrize("n,ic", [(30_000, "galaxy"), (60_000, "plummer"), (90_000, "plummer"),
+                                  (131_072, "galaxy"), (131_073, "plummer")])
+def test_task_sizes(ctx, n, ic):
+    """One size for each share of the bodies that the tasks are made from, and
+    both sides of the last split."""
+    pos, _, m = getattr(ics, ic)(n, seed=2)
+    ctx.upload(pos, None, m)
+    f = ctx.gravity_forces(exact(0.6, 0.02))
+    assert np.array_equal(f, oracle.bh_forces(pos, m, 1.0, 0.02, 0.6))
+
+
+def test_whole_walk_far_masses(ctx):
+    """Beyond the split: masses of both signs and unsoftened pairs."""
+    n = 131_500
+    pos, _, m = ics.plummer(n, seed=8)
+    m *= np.random.default_rng(5).choice([-1.0, 1.0], n, p=[0.3, 0.7])
+    ctx.upload(pos, None, m)
+    f = ctx.gravity_forces(exact(0.8, 0.0))
+    assert np.array_equal(f, oracle.bh_forces(pos, m, 1.0, 0.0, 0.8))
