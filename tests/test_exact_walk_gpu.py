@@ -1,4 +1,4 @@
-"""The exact Barnes-Hut walk split over subtrees (up to 65 536 targets) and
+"""The exact Barnes-Hut walk split over subtrees (up to 131 072 targets) and
 the one walk per target beyond: bit-identical to the oracle's recursive walk
 at the edges of the split, for trees without upper cells, deep chains, masses
 that rule out the f32 opening test or the branch-free weight, and shares."""
@@ -57,8 +57,8 @@ def test_ranges(ctx, kind):
 
 
 @pytest.mark.parametrize("kind,theta", [("negative", 0.7), ("clumps", 1.1), ("unsoftened", 0.9)])
-def test_whole_walk_ranges(ctx, kind, theta):
-    """More targets than are split: the f64 test for every cell, deep chains
+def test_many_targets_ranges(ctx, kind, theta):
+    """Many targets: the f64 test for every cell, deep chains
     with the cells of several depths waiting, and the library's weights."""
     n = 65_700
     rng = np.random.default_rng(5)
