@@ -185,7 +185,8 @@ vjp_kernel(int64_t n, int64_t slice_len, const double* __restrict__ x,
     const double4 zero = make_double4(0, 0, 0, 0);
     xj[q] = j < n ? make_double4(x[j], y[j], z[j], m[j]) : zero;
     wj[q] = j < n ? make_double4(wx[j], wy[j], wz[j], 0.0) : zero;
-    u[q] = zero;
+    const double s = sum_start(eps2);
+    u[q] = make_double4(s, s, s, s);
   }
   const int64_t lo = blockIdx.y * slice_len;
   const int64_t hi = min64(n, lo + slice_len);

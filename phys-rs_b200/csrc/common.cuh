@@ -438,7 +438,9 @@ __device__ __forceinline__ float rsqrt_sfu(float x) {
 // which the library function's range test prevents.  An infinite x (an
 // overflowed square) is read as 2^1023, so its term is 0 as the limit is; x
 // = 0 gives NaN where the cube of rsqrt gives infinity, and the caller's sum
-// is not finite either way.
+// is not finite either way.  A NaN is read as a large number too: a NaN
+// separation makes the term NaN by itself, and a NaN softening is carried by
+// the sums' first value (sum_start).
 __device__ __forceinline__ double inv_cubed(double x) {
   const double xc = __hiloint2double(min(__double2hiint(x), 0x7fe00000), __double2loint(x));
   double y0;
@@ -448,6 +450,12 @@ __device__ __forceinline__ double inv_cubed(double x) {
   const double y3 = t * y0;
   return fma(y3 * h, fma(h, 1.875, 1.5), y3);
 }
+
+// Where a sum over these terms starts: 0, or NaN for a NaN softening, so that
+// the result is reported as not finite.  (Keeping the NaN inside the term
+// takes an instruction a pair or a register: 65 536 bodies 4.59 or 4.75 ms
+// against 4.53.)
+__device__ __forceinline__ double sum_start(double eps2) { return eps2 == eps2 ? 0.0 : eps2; }
 
 // 1/sqrt(x) the same way: y0 (1 + h/2 + 3/8 h^2), within 1.01 u; for the VJP,
 // which needs the fifth power as well.

@@ -265,7 +265,7 @@ direct_f64_kernel(int64_t n, int64_t t0, int64_t t1, int64_t slice_len,
     xi[q] = valid ? x[i] : 0.0;
     yi[q] = valid ? y[i] : 0.0;
     zi[q] = valid ? z[i] : 0.0;
-    ax[q] = ay[q] = az[q] = 0.0;
+    ax[q] = ay[q] = az[q] = sum_start(eps2);
   }
   const int64_t lo = blockIdx.y * slice_len;
   const int64_t hi = min64(n, lo + slice_len);
@@ -496,7 +496,7 @@ direct_targets_kernel(int64_t n, int64_t nt, const int64_t* __restrict__ tidx, i
   const double gm = xmul(G, mi);
   const int64_t lo = blockIdx.y * slice_len;
   const int64_t hi = min64(n, lo + slice_len);
-  double ax = 0.0, ay = 0.0, az = 0.0;
+  double ax = exact ? 0.0 : sum_start(eps2), ay = ax, az = ax;
   for (int64_t base = lo; base < hi; base += kTile) {
     const int64_t j = base + threadIdx.x;
     __syncthreads();

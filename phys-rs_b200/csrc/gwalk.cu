@@ -413,7 +413,7 @@ struct Evaluator {
     const float2 z = make_float2(0.f, 0.f);
     pxa = pya = pza = pxb = pyb = pzb = z;
     Hx = Hy = Hz = Lx = Ly = Lz = z;
-    ax = ay = az = bx = by = bz = 0.0;
+    ax = ay = az = bx = by = bz = sum_start(eps2);
     pend = 0;
   }
 

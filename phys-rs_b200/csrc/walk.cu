@@ -80,7 +80,7 @@ walk_kernel(int q0, int n, int nnodes, const Rec32* __restrict__ w32, const Rec6
       tx = b.x; ty = b.y; tz = b.z;
     }
   }
-  double ax = 0, ay = 0, az = 0;            // F64 sums
+  double ax = sum_start(eps2), ay = ax, az = ax;  // F64 sums
   float hx = 0, hy = 0, hz = 0;             // F32C compensated sums (hi)
   float lx = 0, ly = 0, lz = 0;             //                      (lo)
   float px = 0, py = 0, pz = 0;             // F32C partial since last flush
