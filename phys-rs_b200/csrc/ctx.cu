@@ -157,11 +157,17 @@ int d2h(phys_ctx* c, double* dst, const double* src, int64_t n) {
 // us against 830 packed, of 60000 995 against 1228).
 constexpr int64_t kPackBytes = int64_t(256) << 10;
 
-bool packs(int64_t n, int rows) { return 8 * n * rows <= kPackBytes; }
+// A strided call takes a pitch below 2^31 bytes (the state's rows are as far
+// apart as the largest upload so far made them).
+bool one_call(const phys_ctx* c) { return 8 * c->cap < (int64_t(1) << 31); }
+
+bool packs(const phys_ctx* c, int64_t n, int rows) {
+  return 8 * n * rows <= kPackBytes && one_call(c);
+}
 
 int copy_rows(phys_ctx* c, double* first, int rows, const void* const* src, int64_t n,
               int64_t at) {
-  if (!packs(n, rows)) {
+  if (!packs(c, n, rows)) {
     for (int k = 0; k < rows; ++k)
       PHYS_TRY(h2d(c, first + k * c->cap, static_cast<const double*>(src[k]), n));
     return PHYS_OK;
@@ -177,9 +183,6 @@ int copy_rows(phys_ctx* c, double* first, int rows, const void* const* src, int6
                                  cudaMemcpyHostToDevice, c->stream));
   return PHYS_OK;
 }
-
-// A strided call takes a pitch below 2^31 bytes.
-bool one_call(const phys_ctx* c) { return 8 * c->cap < (int64_t(1) << 31); }
 
 int zero_rows(phys_ctx* c, double* first, int rows, int64_t n) {
   if (one_call(c)) {
@@ -590,7 +593,7 @@ int phys_state_upload(phys_ctx* c, int64_t n, const double* x, const double* y, 
   c->accel_valid = false;
   if (n == 0) return PHYS_OK;
   const void* src[7] = {x, y, z, vx, vy, vz, m};
-  if (packs(n, 7)) PHYS_TRY(ensure_pinned(c, 8 * 7 * n));
+  if (packs(c, n, 7)) PHYS_TRY(ensure_pinned(c, 8 * 7 * n));
   PHYS_TRY(copy_rows(c, c->x, 7, src, n, 0));
   PHYS_TRY(zero_rows(c, c->ax, 6, n));  // Acceleration, PreviousAcceleration
   PHYS_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -616,7 +619,7 @@ int phys_state_upload_sectors(phys_ctx* c, int64_t n, const int64_t* sx, const i
   // local positions in x/y/z, then flatten in place on the device.
   const void* sec[3] = {sx, sy, sz};
   const void* src[7] = {lx, ly, lz, vx, vy, vz, m};
-  if (packs(n, 3)) PHYS_TRY(ensure_pinned(c, 8 * 10 * n));
+  if (packs(c, n, 3)) PHYS_TRY(ensure_pinned(c, 8 * 10 * n));
   PHYS_TRY(copy_rows(c, c->fx, 3, sec, n, 0));
   PHYS_TRY(copy_rows(c, c->x, 7, src, n, 3 * n));
   PHYS_TRY(flatten_sectors(c, reinterpret_cast<int64_t*>(c->fx), reinterpret_cast<int64_t*>(c->fy),
