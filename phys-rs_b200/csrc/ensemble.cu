@@ -492,9 +492,10 @@ __device__ void drain(S_t* S, const EnsArgs& a, int lo, int hi, int* ctr, int ma
 // step reads and writes no f64 array (30 of the 60 shared-memory accesses per
 // body and step that are not pair sources).  kBodies = 2: systems of 33..64
 // bodies.  Bound by the packed pair terms, about 64 % of their rate on 16
-// warps an SM (128 registers; 12 warps at 150 take 2 to 8 % longer, 20 warps
-// 3 %).  300 steps of 16384 systems of 3..64 bodies 8.13 -> 7.61 ms, of 3..32
-// 3.30 -> 2.80, of 3..24 2.59 -> 2.08; 2000 systems of 3..64 2.66 -> 1.98.
+// warps an SM, with few systems by the latency of a step of the largest one.
+// 200 steps, against the state in shared memory: 16384 systems of 3..64 bodies
+// 4.98 -> 4.66 ms, of 3..32 1.97 -> 1.62, of 3..16 0.95 -> 0.75; 4000 of 3..64
+// 1.95 -> 1.56; 400 of 3..64 0.98 -> 0.94.
 template <int G, int kBodies, class S_t>
 __device__ __forceinline__ void run_system(S_t* S, const EnsArgs& a, int64_t b, int N) {
   const int gl = (threadIdx.x & 31) % G;
@@ -609,15 +610,28 @@ __device__ void drain_f32c(S_t* S, const EnsArgs& a, int lo, int hi, int* ctr, i
   }
 }
 
-// F32C with 32 lanes or lanes by size keeps the state in registers.
+// F32C with 32 lanes or lanes by size keeps the state in registers, on 16 warps
+// an SM (128 registers) when there are systems enough to fill them several
+// times over, else on 12 (162 registers): a step of one system is 18 % slower
+// with 128 (200 steps of 400 systems of 3..64 bodies 1.11 against 0.94 ms, of
+// 4800 1.78 against 1.54), which the four more warps make good from three
+// systems a warp on (7200: 2.22 against 2.19 of 3..64 bodies, 0.88 against 0.90
+// of 3..32; 16384: 4.66 against 4.73 and 1.62 against 1.74; 6400: 2.07 against
+// 1.99 and 0.80 against 0.82; 20 warps 3 % behind 16).
 constexpr bool in_registers(int G, bool exact) { return !exact && (G == 0 || G == 32); }
+constexpr int kDenseWarps = 16, kWideWarps = 12;
+constexpr int kDenseSystems = 3;  // per warp
+
+constexpr int warps_per_sm(int G, int BW, bool exact, bool dense) {
+  return !in_registers(G, exact) ? BW : dense ? kDenseWarps : kWideWarps;
+}
 
 // One persistent launch of BW warps per block.  G = 8, 16, 32: every system
 // gets G lanes (32 / G systems per warp at a time).  G = 0: lanes by size —
 // a warp takes the systems of more than 16 bodies one at a time, then two of
 // 9..16 bodies at a time (16 lanes each), then four of at most 8.
-template <int G, int BW, bool kExact>
-__global__ void __launch_bounds__(32 * BW, in_registers(G, kExact) ? 16 / BW : 1)
+template <int G, int BW, bool kExact, bool kDense>
+__global__ void __launch_bounds__(32 * BW, warps_per_sm(G, BW, kExact, kDense) / BW)
 ensemble_kernel(EnsArgs a) {
   wait_for_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -647,18 +661,26 @@ ensemble_kernel(EnsArgs a) {
 
 using EnsKernel = void (*)(EnsArgs);
 
+template <int G, int BW>
+EnsKernel pick_form(bool exact, bool dense) {
+  if (exact) return ensemble_kernel<G, BW, true, false>;
+  if constexpr (in_registers(G, false))
+    if (dense) return ensemble_kernel<G, BW, false, true>;
+  return ensemble_kernel<G, BW, false, false>;
+}
+
 template <int BW>
-EnsKernel pick_bw(int G, bool exact) {
+EnsKernel pick_bw(int G, bool exact, bool dense) {
   switch (G) {
-    case 8: return exact ? ensemble_kernel<8, BW, true> : ensemble_kernel<8, BW, false>;
-    case 16: return exact ? ensemble_kernel<16, BW, true> : ensemble_kernel<16, BW, false>;
-    case 32: return exact ? ensemble_kernel<32, BW, true> : ensemble_kernel<32, BW, false>;
-    default: return exact ? ensemble_kernel<0, BW, true> : ensemble_kernel<0, BW, false>;
+    case 8: return pick_form<8, BW>(exact, dense);
+    case 16: return pick_form<16, BW>(exact, dense);
+    case 32: return pick_form<32, BW>(exact, dense);
+    default: return pick_form<0, BW>(exact, dense);
   }
 }
 
-EnsKernel pick(int G, int bw, bool exact) {
-  return bw == 4 ? pick_bw<4>(G, exact) : pick_bw<2>(G, exact);
+EnsKernel pick(int G, int bw, bool exact, bool dense) {
+  return bw == 4 ? pick_bw<4>(G, exact, dense) : pick_bw<2>(G, exact, dense);
 }
 
 struct EnsView {
@@ -696,7 +718,9 @@ int prepare(phys_ctx* c, const phys_params* p, int code, LaunchCfg* cfg) {
   int G = 0, bw = 2;
   if (!decode(code, &G, &bw)) return fail(c, PHYS_ERR_ARG, "ensemble configuration 0x%x", code);
   const bool exact = p->precision == PHYS_F64_EXACT;
-  cfg->k = pick(G, bw, exact);
+  int sms = 148;
+  PHYS_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  cfg->k = pick(G, bw, exact, c->ens_nsys >= (int64_t)kDenseSystems * kDenseWarps * sms);
   cfg->block = 32 * bw;
   const int groups_per_warp = G == 0 ? 1 : 32 / G;
   cfg->smem = (in_registers(G, exact) ? sizeof(SourceSmem) : sizeof(GroupSmem)) *
@@ -706,13 +730,6 @@ int prepare(phys_ctx* c, const phys_params* p, int code, LaunchCfg* cfg) {
   int per_sm = 0;
   PHYS_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cfg->k, cfg->block,
                                                              cfg->smem));
-  int sms = 148;
-  PHYS_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  // more than 12 warps an SM only when every one gets a system: a fourth block
-  // on some SMs alone makes the longest systems there the last to finish (300
-  // steps of 2000 systems of 3..64 bodies: 2.55 ms against 1.98)
-  if (in_registers(G, exact))
-    while (per_sm * bw > 12 && c->ens_nsys < (int64_t)per_sm * bw * sms) --per_sm;
   const int64_t groups_per_block = (int64_t)groups_per_warp * bw;
   cfg->grid = std::min<int64_t>((int64_t)std::max(per_sm, 1) * sms,
                                 ceil_div(c->ens_nsys, groups_per_block));
