@@ -135,8 +135,7 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
 // (count in longs[nnodes]; those of at least com_long_chain(n) bodies).
 int com_long_chain(int64_t n);
 int com_long_cells(phys_ctx* c, int64_t n, int64_t nnodes, int64_t total, const int32_t* eoff,
-                   const double4* eb, const int4* link, const TreeHeader* hdr,
-                   const int32_t* longs, double4* mc);
+                   const double4* eb, const TreeHeader* hdr, const int32_t* longs, double4* mc);
 // walk.cu
 // Tasks that the exact walk of this evaluation may be split into (0: one walk
 // per target).

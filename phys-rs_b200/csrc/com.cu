@@ -29,8 +29,12 @@
 // around where it passed them (twice, for the longest chains); what is left
 // then is run from the true value in turn.
 //
-// The division is by a precomputed reciprocal (div_recip); a cell that leaves
-// its range, or with masses of both signs, runs whole with the IEEE division.
+// The division is by a precomputed reciprocal (div_recip).  A candidate that
+// leaves its range ends as NaN and counts as unknown: in a plane the centre of
+// mass is 0, in range, and its neighbours are not.  Only a segment whose
+// running masses, or whose true value, leave the range is run with the IEEE
+// division, by itself.  Masses of both signs have the same steps wherever the
+// running mass is positive; their running masses are summed in turn.
 //
 // Tree phase of the exact form, one chain per cell before against segments
 // (Plummer spheres): 10 000 bodies 0.59 -> 0.32 ms, 100 000 4.8 -> 1.26 ms,
@@ -58,7 +62,6 @@ struct LongCells {
   int len;               // bodies per segment
   const int32_t* eoff;   // node -> first (cell, body) pair
   const double4* eb;     // bodies in pair order (x, y, z, m)
-  const int4* link;
   const TreeHeader* hdr;
   const int32_t* longs;  // nodes of the long cells, count in longs[nnodes]
   double4* mc;           // result per node
@@ -70,10 +73,12 @@ struct LongCells {
                          // (first the sums before it, then the mean, then the
                          // prediction)
   double2* mass_end;     // per segment: masses at its end from the two starts
-  int32_t* bad;          // per segment: left div_recip's range
+  int32_t* bad;          // per segment: its masses (for a cell's first segment, its
+                         // steps) leave div_recip's range
   int32_t* redo;         // per segment: coordinates to run again (bits 0-2)
   double4* pass;         // per segment: com at its end from the mean
-  double* end;           // per candidate slot: com at the segment's end, [3][kCand]
+  double* end;           // per candidate slot: com at the segment's end, [3][kCand]; NaN
+                         // where the candidate left div_recip's range
   const int32_t* status;
 };
 
@@ -85,13 +90,14 @@ __device__ __forceinline__ double next_up(double v) {  // v >= 0
 }
 
 // The candidates at the start of a cell's segment s: consecutive doubles
-// around its prediction (which is the true value for s = 1).
+// around its prediction (few where that is the true value, s = 1, or 0: then
+// the bodies lie in a plane, and its neighbours are out of range).
 struct Window {
   double mid, ulp;
   int n;
   __device__ __forceinline__ Window(double m, int s, int64_t len)
       : mid(m), ulp(xsub(next_up(fabs(m)), fabs(m))),
-        n(s == 1             ? 32
+        n(s == 1 || m == 0.0 ? 32
           : s * len < 8192   ? kCand / 4
           : s * len < 100000 ? kCand / 2
                              : kCand) {}
@@ -227,7 +233,7 @@ __global__ void __launch_bounds__(32) mass_stitch_kernel(LongCells a) {
       __syncwarp();
       if (lane < 4) {  // the prefix sums become the means and the true mass
         double* st = reinterpret_cast<double*>(&a.start[base + s]);
-        st[lane] = lane == 3 ? M : s ? st[lane] / M : 0.0;
+        st[lane] = lane == 3 ? M : M > 0.0 ? st[lane] / M : 0.0;
       }
       const bool odd = ((__double_as_longlong(M) ^ __double_as_longlong(from)) & 1) != 0;
       const double f = odd ? next_up(from) : from, e = odd ? en.y : en.x;
@@ -280,7 +286,7 @@ __device__ __forceinline__ bool fill_batch(Batch<kN>& B, int at, double4 body, i
   return lane >= cnt || div_recip_den_ok(after);
 }
 
-// cnt steps of kQ chains.
+// cnt steps of kQ chains; ok: they stayed in div_recip's range.
 template <int kQ, int kN>
 __device__ __forceinline__ void chain_steps(const Batch<kN>& B, const double* __restrict__ p,
                                             int cnt, double (&c)[kQ], bool& ok) {
@@ -302,23 +308,27 @@ __device__ __forceinline__ void chain_steps(const Batch<kN>& B, const double* __
 }
 
 // The steps of segment eb[f0, f0 + len) from mass M and com c, lane j < 3
-// coordinate j (warp-collective).
+// coordinate j (warp-collective).  masses_ok: of the lane's own bodies.
 __device__ __forceinline__ void run_warp(const double4* __restrict__ eb, int64_t f0, int len,
-                                         double M, double& c, Batch<32>& B, int lane, bool& ok) {
+                                         double M, double& c, Batch<32>& B, int lane,
+                                         bool& masses_ok, bool& steps_ok) {
   const int j = lane < 3 ? lane : 0;
   const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
   double cc[1] = {c};
+  masses_ok = true;
+  bool ok = true;
   double4 body = lane < len ? eb[f0 + lane] : zero;
   for (int b = 0; b < len; b += 32) {
     const int cnt = min(32, len - b);
     const double4 next = b + 32 + lane < len ? eb[f0 + b + 32 + lane] : zero;
-    ok &= fill_batch(B, 0, body, cnt, lane, M);
+    masses_ok &= fill_batch(B, 0, body, cnt, lane, M);
     __syncwarp();
     chain_steps<1>(B, B.p[j], cnt, cc, ok);
     __syncwarp();
     body = next;
   }
   c = cc[0];
+  steps_ok = ok;
 }
 
 // Every segment from the mean at its start (the first one of a cell from 0,
@@ -335,10 +345,11 @@ __global__ void __launch_bounds__(32) first_pass_kernel(LongCells a) {
     const int len = (int)min64(a.len, a.eoff[k + 1] - f0);
     const double4 st = a.start[g];
     double c = lane == 0 ? st.x : lane == 1 ? st.y : st.z;
-    bool ok = true;
-    run_warp(a.eb, f0, len, st.w, c, B, lane, ok);
+    bool masses_ok, steps_ok;
+    run_warp(a.eb, f0, len, st.w, c, B, lane, masses_ok, steps_ok);
     if (lane < 3) reinterpret_cast<double*>(&a.pass[g])[lane] = c;
-    if (__any_sync(kFull, !ok) && lane == 0) a.bad[g] = 1;
+    // beyond the first segment the steps are a mean's and only predict
+    if (__any_sync(kFull, !masses_ok || (sg.y == 0 && !steps_ok)) && lane == 0) a.bad[g] = 1;
   }
 }
 
@@ -358,8 +369,9 @@ __global__ void __launch_bounds__(32) predict_kernel(LongCells a) {
       for (int s = 1; s < ns; ++s) {
         double* st = reinterpret_cast<double*>(&a.start[base + s]);
         const double mean = st[lane], Ms = st[3];
-        const double at = reinterpret_cast<const double*>(&a.pass[base + s - 1])[lane] +
-                          diff * (M / Ms);
+        double at = reinterpret_cast<const double*>(&a.pass[base + s - 1])[lane] +
+                    diff * (M / Ms);
+        if (!isfinite(at)) at = mean;  // no mass yet, or out of range
         diff = at - mean;
         M = Ms;
         st[lane] = at;
@@ -368,18 +380,24 @@ __global__ void __launch_bounds__(32) predict_kernel(LongCells a) {
   }
 }
 
-// kQ chains per lane of the places [g, g + 32 kQ) of val[0, live).
+// kQ chains per lane of the places [g, g + 32 kQ) of val[0, live).  A candidate
+// that leaves the range, or has, ends as the one NaN; which of a lane's it is
+// shows only with one per lane: of several, false and nothing written.
 template <int kQ>
-__device__ __forceinline__ void run_places(const Batch<kRound>& B, const double* p, int cnt,
-                                           double* val, int g, int live, int lane, bool& ok) {
+__device__ __forceinline__ bool run_places(const Batch<kRound>& B, const double* p, int cnt,
+                                           double* val, int g, int live, int lane) {
   double c[kQ];
 #pragma unroll
   for (int q = 0; q < kQ; ++q) c[q] = val[min(g + 32 * q + lane, live - 1)];
+  bool ok = true;
   chain_steps<kQ>(B, p, cnt, c, ok);
+  if (kQ > 1 && __any_sync(kFull, !ok)) return false;
+  if (!ok) c[0] = __longlong_as_double(0x7ff8000000000000ll);
   __syncwarp();
 #pragma unroll
   for (int q = 0; q < kQ; ++q)
     if (g + 32 * q + lane < live) val[g + 32 * q + lane] = c[q];
+  return true;
 }
 
 // A block per segment: warps 0-2 run the candidates of x, y and z, warp 3
@@ -396,13 +414,12 @@ __global__ void __launch_bounds__(128) segment_kernel(LongCells a, int again) {
     const int2 sg = a.seg[g];
     if (sg.y == 0) continue;  // the first pass started at the true value
     const int redo = again ? a.redo[g] : 7;
-    if (!redo) continue;
+    if (!redo || a.bad[g]) continue;
     const int k = a.longs[sg.x];
     const int64_t f0 = a.eoff[k] + (int64_t)sg.y * a.len;
     const int len = (int)min64(a.len, a.eoff[k + 1] - f0);
     const double4 st = a.start[g];
     const int rounds = (len + kRound - 1) / kRound;
-    bool ok = true;
     double M = st.w;
     auto fill = [&](int r) {  // round r's bodies into its buffer
       const int cnt = min(kRound, len - r * kRound);
@@ -411,7 +428,7 @@ __global__ void __launch_bounds__(128) segment_kernel(LongCells a, int again) {
       double4 body = lane < cnt ? eb[lane] : zero;
       for (int j = 0; j < cnt; j += 32) {
         const double4 next = j + 32 + lane < cnt ? eb[j + 32 + lane] : zero;
-        ok &= fill_batch(B[r & 1], j, body, min(32, cnt - j), lane, M);
+        fill_batch(B[r & 1], j, body, min(32, cnt - j), lane, M);
         body = next;
       }
     };
@@ -433,31 +450,35 @@ __global__ void __launch_bounds__(128) segment_kernel(LongCells a, int again) {
         const Batch<kRound>& C = B[r & 1];
         const int cnt = min(kRound, len - r * kRound);
         double* val = vals[w];
+        int apart = 0;  // places before this one go one per lane
         for (int g0 = 0; g0 < live;) {
-          if (live - g0 > 64) {
-            run_places<4>(C, C.p[w], cnt, val, g0, live, lane, ok);
-            g0 += 128;
-          } else if (live - g0 > 32) {
-            run_places<2>(C, C.p[w], cnt, val, g0, live, lane, ok);
-            g0 += 64;
+          if (live - g0 > 64 && g0 >= apart) {
+            if (run_places<4>(C, C.p[w], cnt, val, g0, live, lane))
+              g0 += 128;
+            else
+              apart = g0 + 128;
+          } else if (live - g0 > 32 && g0 >= apart) {
+            if (run_places<2>(C, C.p[w], cnt, val, g0, live, lane))
+              g0 += 64;
+            else
+              apart = g0 + 64;
           } else {
-            run_places<1>(C, C.p[w], cnt, val, g0, live, lane, ok);
+            run_places<1>(C, C.p[w], cnt, val, g0, live, lane);
             g0 += 32;
           }
         }
         __syncwarp();
         if (live > 32) {  // keep one place of each run of equal values
           int kept = 0;
-          double last = 0.0;
+          long long last = 0;
           for (int g0 = 0; g0 < live; g0 += 32) {
             const int i = g0 + lane;
             const double v = val[min(i, live - 1)];
-            const double up = __shfl_up_sync(kFull, v, 1);
-            const double before = lane ? up : last;
-            const bool first = i < live && (i == 0 || v != before);
+            const long long bits = __double_as_longlong(v), up = __shfl_up_sync(kFull, bits, 1);
+            const bool first = i < live && (i == 0 || bits != (lane ? up : last));
             const unsigned m = __ballot_sync(kFull, first);
             const int place = kept + __popc(m & (0xffffffffu >> (31 - lane))) - 1;
-            last = __shfl_sync(kFull, v, 31);
+            last = __shfl_sync(kFull, bits, 31);
             if (i < live) moved[w][i] = (uint16_t)place;
             if (first) val[place] = v;
             kept += __popc(m);
@@ -476,32 +497,38 @@ __global__ void __launch_bounds__(128) segment_kernel(LongCells a, int again) {
       double* out = a.end + ((size_t)(a.first[sg.x].y + sg.y - 1) * 3 + w) * kCand;
       for (int i = lane; i < win.n; i += 32) out[i] = vals[w][map[w][i]];
     }
-    if (__any_sync(kFull, !ok) && lane == 0) a.bad[g] = 1;
     __syncthreads();
   }
 }
 
-// The reference's form over a whole cell: the fallback.  Lane j < 3:
-// coordinate j.
-__device__ double cell_ieee(const double4* __restrict__ eb, int64_t e0, int64_t e1, double4* rec,
-                            int lane) {
-  double M = 0.0, cc = 0.0;
-  for (int64_t e = e0; e < e1; e += 32) {
+// The reference's form over a segment, from mass M and com c: the fallback.
+// Lane j < 3: coordinate j; the others return lane 0's.
+__device__ double segment_ieee(const double4* __restrict__ eb, int64_t f0, int len, double M,
+                               double c, double4* rec, int lane) {
+  for (int b = 0; b < len; b += 32) {
     __syncwarp();
-    if (e + lane < e1) rec[lane] = eb[e + lane];
+    if (b + lane < len) rec[lane] = eb[f0 + b + lane];
     __syncwarp();
-    const int cnt = (int)min64(32, e1 - e);
+    const int cnt = min(32, len - b);
     if (lane < 3) {
       const double* q = reinterpret_cast<const double*>(rec);
       for (int u = 0; u < cnt; ++u) {
         const double p = q[4 * u + lane], mm = q[4 * u + 3];
         const double nt = xadd(M, mm);
-        if (nt > 0.0) cc = xdiv(xadd(xmul(cc, M), xmul(p, mm)), nt);
+        if (nt > 0.0) c = xdiv(xadd(xmul(c, M), xmul(p, mm)), nt);
         M = nt;
       }
     }
   }
-  return cc;
+  __syncwarp();
+  return __shfl_sync(kFull, c, lane < 3 ? lane : 0);
+}
+
+// Whether one of the segments [g0, g0 + ns) is marked (warp-collective).
+__device__ __forceinline__ bool any_segment_bad(const LongCells& a, int g0, int ns, int lane) {
+  int bad = 0;
+  for (int g = lane; g < ns; g += 32) bad |= a.bad[g0 + g];
+  return __any_sync(kFull, bad != 0);
 }
 
 // A warp per long cell follows the true value through the segments, or past
@@ -516,9 +543,16 @@ __global__ void __launch_bounds__(32) refine_kernel(LongCells a) {
     const int k = a.longs[i];
     const int2 first = a.first[i];
     const int ns = (a.eoff[k + 1] - a.eoff[k] + a.len - 1) / a.len;
+    const bool any_bad = any_segment_bad(a, first.x, ns, lane);
     double c = reinterpret_cast<const double*>(&a.pass[first.x])[j];
     for (int s = 1; s < ns; ++s) {
       double* st = reinterpret_cast<double*>(&a.start[first.x + s]);
+      auto predicted = [&]() { return s + 1 < ns ? st[4 + j] : 0.0; };  // at its end
+      if (any_bad && a.bad[first.x + s]) {
+        if (lane == 0) a.redo[first.x + s] = 0;
+        c = predicted();
+        continue;
+      }
       const Window win(st[j], s, a.len);
       const int lo = win.find(c);
       const double* en = a.end + ((size_t)(first.y + s - 1) * 3 + j) * kCand + lo;
@@ -529,6 +563,7 @@ __global__ void __launch_bounds__(32) refine_kernel(LongCells a) {
       if (lane == 0) a.redo[first.x + s] = (int)out;
       // outside the window: the nearer end, shifted
       c = in ? (c == ch ? eh : el) : c < cl ? el + (c - cl) : eh + (c - ch);
+      if (!isfinite(c)) c = predicted();  // left the range
     }
   }
 }
@@ -546,26 +581,34 @@ __global__ void __launch_bounds__(32) stitch_kernel(LongCells a) {
     const int64_t e0 = a.eoff[k], e1 = a.eoff[k + 1];
     const int2 first = a.first[i];
     const int ns = (int)((e1 - e0 + a.len - 1) / a.len);
-    int bad = 0;
-    for (int g = lane; g < ns; g += 32) bad |= a.bad[first.x + g];
-    bool ok = !__any_sync(kFull, bad != 0) && a.hdr->min_mass >= 0.0;
+    const bool any_bad = any_segment_bad(a, first.x, ns, lane);
+    auto run_again = [&](int s, double4 st, bool in_range, double c) {  // from the true value
+      const int64_t f0 = e0 + (int64_t)s * a.len;
+      const int len = (int)min64(a.len, e1 - f0);
+      double to = c;
+      bool masses_ok = false, steps_ok = false;
+      if (in_range) run_warp(a.eb, f0, len, st.w, to, B, lane, masses_ok, steps_ok);
+      if (__any_sync(kFull, !masses_ok || !steps_ok))
+        to = segment_ieee(a.eb, f0, len, st.w, c, rec, lane);
+      return to;
+    };
     double c = reinterpret_cast<const double*>(&a.pass[first.x])[j];
-    for (int s = 1; s < ns && ok; ++s) {
+    if (any_bad && a.bad[first.x]) c = run_again(0, a.start[first.x], false, 0.0);
+    for (int s = 1; s < ns; ++s) {
       const double4 st = a.start[first.x + s];
+      if (any_bad && a.bad[first.x + s]) {
+        c = run_again(s, st, false, c);
+        continue;
+      }
       const Window win(j == 0 ? st.x : j == 1 ? st.y : st.z, s, a.len);
       const int lo = win.find(c);
       const double* en = a.end + ((size_t)(first.y + s - 1) * 3 + j) * kCand + lo;
       const double cl = win.at(lo), ch = win.at(lo + 1), el = en[0], eh = en[1];
-      const bool known = c == cl || c == ch || (cl < c && c < ch && el == eh);
-      if (__any_sync(kFull, !known)) {  // the segment again, from the true value
-        const int64_t f0 = e0 + (int64_t)s * a.len;
-        run_warp(a.eb, f0, (int)min64(a.len, e1 - f0), st.w, c, B, lane, ok);
-        ok = !__any_sync(kFull, !ok);
-      } else {
-        c = c == ch ? eh : el;
-      }
+      const double to = c == ch ? eh : el;
+      const bool known =
+          (c == cl || c == ch || (cl < c && c < ch && el == eh)) && to == to;
+      c = __all_sync(kFull, known) ? to : run_again(s, st, true, c);
     }
-    if (!ok) c = cell_ieee(a.eb, e0, e1, rec, lane);
     if (lane < 3) reinterpret_cast<double*>(&a.mc[k])[lane] = c;
     __syncwarp();
   }
@@ -581,14 +624,12 @@ int com_long_chain(int64_t n) {
 }
 
 int com_long_cells(phys_ctx* c, int64_t n, int64_t nnodes, int64_t total, const int32_t* eoff,
-                   const double4* eb, const int4* link, const TreeHeader* hdr,
-                   const int32_t* longs, double4* mc) {
+                   const double4* eb, const TreeHeader* hdr, const int32_t* longs, double4* mc) {
   LongCells a{};
   a.nnodes = nnodes;
   a.len = segment_len(n);
   a.eoff = eoff;
   a.eb = eb;
-  a.link = link;
   a.hdr = hdr;
   a.longs = longs;
   a.mc = mc;

@@ -1306,7 +1306,7 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     PHYS_CUDA(c, cudaMemsetAsync(longs + nnodes, 0, sizeof(int32_t), c->stream));
     PHYS_LAUNCH(c, com_recurrence_kernel, grid_for(nnodes, 128, 1 << 30), 128, 0, nnodes, eoff, eb,
                 mc, link, c->d_hdr, full_com ? 0 : 1, com_long_chain(n), longs, c->d_status);
-    PHYS_TRY(com_long_cells(c, n, nnodes, total, eoff, eb, link, c->d_hdr, longs, mc));
+    PHYS_TRY(com_long_cells(c, n, nnodes, total, eoff, eb, c->d_hdr, longs, mc));
     kids = reinterpret_cast<Kids*>(ent);
     wx = reinterpret_cast<float4*>(ent_alt);
     PHYS_TRY(children());
