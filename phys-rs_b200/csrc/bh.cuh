@@ -101,10 +101,11 @@ struct BhTree {
   const double4* rec64 = nullptr;     // exact walk: record per node (with `link`)
   // exact walk, traversal record per node: position relative to the root
   // cube's centre in units of its half size (f32: decides almost every
-  // opening, the f64 record the rest), for a leaf the stored body in x; the
-  // depth and flags of `link` in w (int bits)
+  // opening, the f64 record the rest; NaN outside the cube), for a leaf the
+  // stored body in x; the depth and flags of `link` in w (int bits)
   const float4* wx = nullptr;
   const Kids* kids = nullptr;
+  bool signs = false;                 // some mass is negative
   TopTree top;                        // exact walk split over subtrees (max_tasks > 0)
   const Rec32* w32 = nullptr;         // F32C walk records
   const Rec32x2* w32x2 = nullptr;     // F32C paired walk records

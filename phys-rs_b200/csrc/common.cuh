@@ -141,7 +141,7 @@ struct phys_ctx {
   // ---- host staging (pinned) ----
   void* h_stage = nullptr;
   size_t h_stage_bytes = 0;
-  int32_t* h_small = nullptr;                // pinned scalars for status / counts
+  int32_t* h_small = nullptr;                // pinned scalars for status / counts (4 KB)
 
   // ---- workspace buffers (grown on demand, named) ----
   phys::DevBuf ws[56];
@@ -180,6 +180,9 @@ enum WsSlot {
   WS_GROUPS, WS_GROUP_OFF, WS_GROUP_CTR, WS_GROUP_POOL, WS_GROUP_ITEMS, WS_SHARE_PERM, WS_BODY_IN,
   WS_COM_SEG, WS_COM_TRAJ, WS_COUNT_
 };
+// Place in h_small of what is read back of the small device block (status word,
+// counters, tree header); the tree build's counts and the sector flag lie below.
+constexpr int kHostStatus = 64;
 static_assert(WS_COUNT_ <= sizeof(phys_ctx::ws) / sizeof(DevBuf), "workspace slots");
 
 // ---- kernels' host launchers (per .cu file) ----

@@ -77,10 +77,6 @@ int ensure_pinned(phys_ctx* c, size_t bytes) {
   return PHYS_OK;
 }
 
-// Place of the status block in the pinned scalars (the tree build's counts
-// and the sector flag lie below).
-constexpr int kHostStatus = 64;
-
 int read_status(phys_ctx* c, int32_t* out) {
   // status word and counters are 256 bytes apart in one block: one copy
   PHYS_CUDA(c, cudaMemcpyAsync(c->h_small + kHostStatus, c->d_status,

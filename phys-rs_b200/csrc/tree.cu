@@ -19,6 +19,7 @@
 //                             leaf at max(L[p-1], L[p]) + 1
 // Pre-order = order of (start, depth), so node ids are a prefix sum.
 #include <climits>
+#include <cstring>
 #include <vector>
 
 #include "bh.cuh"
@@ -904,6 +905,8 @@ finalize_kernel(int64_t nnodes, int4* __restrict__ link, double4* __restrict__ m
       float4 o = make_float4((float)((r.x - hdr->center[0]) * ih),
                              (float)((r.y - hdr->center[1]) * ih),
                              (float)((r.z - hdr->center[2]) * ih), __int_as_float(lk.w));
+      if (!(fabsf(o.x) <= 1.f && fabsf(o.y) <= 1.f && fabsf(o.z) <= 1.f))
+        o.x = o.y = o.z = __int_as_float(0x7fffffff);  // outside the cube: tested in f64
       if (leaf) o.x = __int_as_float(cntb == 1 ? lk.y : lk.z - 1);
       wx[k] = o;
     }
@@ -1221,15 +1224,18 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
   // checked the flag themselves)
   int32_t* hsm = c->h_small;
   PHYS_CUDA(c, cudaMemcpyAsync(hsm, first + n, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-  PHYS_CUDA(c, cudaMemcpyAsync(hsm + 1, &c->d_hdr->dstar, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                               c->stream));
-  PHYS_CUDA(c, cudaMemcpyAsync(hsm + 2, c->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                               c->stream));
+  // status word and header lie in one block: one copy
+  const size_t hdr_at = reinterpret_cast<char*>(c->d_hdr) - reinterpret_cast<char*>(c->d_status);
+  char* block = reinterpret_cast<char*>(hsm + kHostStatus);
+  PHYS_CUDA(c, cudaMemcpyAsync(block, c->d_status, hdr_at + sizeof(TreeHeader),
+                               cudaMemcpyDeviceToHost, c->stream));
   PHYS_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (hsm[2] & kStatTimeout)
+  TreeHeader hh;
+  memcpy(&hh, block + hdr_at, sizeof hh);
+  if (hsm[kHostStatus] & kStatTimeout)
     return fail(c, PHYS_ERR_TIMEOUT, "radix sort of the descent keys: a bounded wait timed out");
   const int64_t nnodes = hsm[0];
-  const int dstar = hsm[1];
+  const int dstar = hh.dstar;
   if (nnodes < 1 || nnodes > (int64_t)n * (kMaxLevels + 1))
     return fail(c, PHYS_ERR_CUDA, "tree build produced %lld nodes for %lld bodies",
                 (long long)nnodes, (long long)n);
@@ -1414,6 +1420,7 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
   t->rec64 = rec64;
   t->wx = wx;
   t->kids = kids;
+  t->signs = hh.min_mass < 0.0;
   t->top = top;
   t->w32 = w32;
   t->w64 = w64;

@@ -401,8 +401,8 @@ walk2_kernel(int q64, int n, int nnodes, const Rec32x2* __restrict__ w, const Bo
 // coordinate is within 2^-25 of its value, their difference within 2^-23, so
 // the distance is within 2.1e-7 of the half size and the lane's choice is the
 // f64 one outside a band of 4e-7 (and 1e-6 relative) around side / theta;
-// inside it, or when the masses do not all have one sign (a centre of mass
-// may then lie outside the cube), the warp takes the reference's f64 test.
+// inside it, and for a centre of mass outside the cube (masses of both signs;
+// its f32 position is NaN), the warp takes the reference's f64 test.
 //
 // Few targets would leave most of the chip idle behind the longest walk, so
 // up to 131072 of them are split: the children of the cells of more than a
@@ -428,12 +428,17 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kXQ = 32;  // queue entries per warp
 constexpr float kXBand = 4e-7f;
 
-// Whether every pair of an evaluation is in exact_scale's range: masses of
-// one sign within [2^-190, 2^240 / n] or 0 (so are the sums over cells),
-// bodies and centres of mass within 2^98, softening.
+// Whether every pair of an evaluation is in exact_scale's range: masses within
+// [2^-190, 2^240 / n] or 0, bodies within 2^98, softening.  With masses of one
+// sign the sums over cells and the centres of mass are then in range as well;
+// with both (kSigns) record_in_range looks at the queued ones, in a kernel of
+// its own (the look, or only the flag for it, costs masses of one sign 2 to 7 %).
+__device__ __forceinline__ bool record_in_range(double4 r) {
+  return scale_pos_ok(r.x, r.y, r.z) && scale_mass_ok(r.w);
+}
 __device__ __forceinline__ bool walk_in_range(const TreeHeader* hdr, int64_t n, double eps2) {
   const double c = fmax(fmax(fabs(hdr->center[0]), fabs(hdr->center[1])), fabs(hdr->center[2]));
-  return scale_eps2_ok(eps2) && hdr->min_mass >= 0.0 && hdr->min_abs >= 0x1p-190 &&
+  return scale_eps2_ok(eps2) && hdr->min_abs >= 0x1p-190 &&
          hdr->max_abs * (double)n < 0x1p240 && c + 2.0 * hdr->half < 0x1p98;
 }
 
@@ -527,7 +532,7 @@ __device__ __forceinline__ void exact_store(double fx, double fy, double fz, dou
 constexpr int kXWarps = 4;  // warps per block
 constexpr int kXTargets = 32 * kXWarps;
 
-template <bool kWhole>
+template <bool kWhole, bool kSigns>
 __global__ void __launch_bounds__(32 * kXWarps, kWhole ? 6 : 4)
 walk_exact_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const float4* __restrict__ wx,
                   const Kids* __restrict__ kids, const double4* __restrict__ rec64,
@@ -580,9 +585,7 @@ walk_exact_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const float4
     const double ih = 1.0 / half;
     const float fx = (float)((t.x - hdr->center[0]) * ih), fy = (float)((t.y - hdr->center[1]) * ih),
                 fz = (float)((t.z - hdr->center[2]) * ih);
-    const bool coarse =
-        hdr->min_mass >= 0.0 &&
-        __all_sync(kFull, !valid || (isfinite(fx) && isfinite(fy) && isfinite(fz)));
+    const bool coarse = __all_sync(kFull, !valid || (isfinite(fx) && isfinite(fy) && isfinite(fz)));
     // the box around the warp's targets
     float bl[3] = {valid ? fx : INFINITY, valid ? fy : INFINITY, valid ? fz : INFINITY};
     float bh[3] = {valid ? fx : -INFINITY, valid ? fy : -INFINITY, valid ? fz : -INFINITY};
@@ -643,7 +646,7 @@ walk_exact_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const float4
         on = lane & j ? (on & ~m) | (y >> j & m) : (on & m) | (y & m) << j;
       }
       __syncwarp();
-      if (fast)
+      if (fast && (!kSigns || __all_sync(kFull, record_in_range(sr[lane]))))
         terms(std::true_type{}, on, ev);
       else
         terms(std::false_type{}, on, ev);
@@ -910,7 +913,8 @@ int bh_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force,
     if (tasks > 0) {
       double* part = nullptr;
       PHYS_TRY(ws_alloc(c, WS_DIRECT_PART, 3 * nt * tasks, &part));
-      PHYS_LAUNCH(c, walk_exact_kernel<false>, (int)min64(148 * 4, (int64_t)xgrid * tasks),
+      auto kernel = t.signs ? walk_exact_kernel<false, true> : walk_exact_kernel<false, false>;
+      PHYS_LAUNCH(c, kernel, (int)min64(148 * 4, (int64_t)xgrid * tasks),
                   32 * kXWarps, 0, q0, q1, n,
                   (int)t.nnodes, t.wx, t.kids, t.rec64, t.body64, t.perm, t.hdr, t.top, p->G, eps2,
                   (int)want_force, part, ox, oy, oz, c->d_counter, c->d_status);
@@ -918,7 +922,8 @@ int bh_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force,
                   t.body64, t.perm, t.hdr, t.top, p->G, eps2, want_force, part, ox, oy, oz,
                   c->d_counter, c->d_status);
     } else {
-      PHYS_LAUNCH(c, walk_exact_kernel<true>, xgrid, 32 * kXWarps, 0, q0, q1, n, (int)t.nnodes, t.wx,
+      auto kernel = t.signs ? walk_exact_kernel<true, true> : walk_exact_kernel<true, false>;
+      PHYS_LAUNCH(c, kernel, xgrid, 32 * kXWarps, 0, q0, q1, n, (int)t.nnodes, t.wx,
                   t.kids, t.rec64, t.body64, t.perm, t.hdr, t.top, p->G, eps2, (int)want_force,
                   (double*)nullptr, ox, oy, oz, c->d_counter, c->d_status);
     }
