@@ -84,8 +84,7 @@ struct __align__(16) Kids {
 // The exact walk's split over subtrees: the cells of more than `most` bodies
 // (upper cells) and their other children (tasks), in pre-order.
 struct TopTree {
-  int max_tasks = 0, max_top = 0;    // room in the arrays
-  int32_t* counts = nullptr;         // tasks << 16 | top nodes
+  int ntask = 0, ntop = 0;           // 0: one walk per target
   int32_t* task = nullptr;           // node of each task
   int4* top = nullptr;               // node, task (-1: upper cell), depth, -
   const int32_t* parent = nullptr;   // of every node
@@ -106,7 +105,7 @@ struct BhTree {
   const float4* wx = nullptr;
   const Kids* kids = nullptr;
   bool signs = false;                 // some mass is negative
-  TopTree top;                        // exact walk split over subtrees (max_tasks > 0)
+  TopTree top;                        // exact walk split over subtrees (ntask > 0)
   const Rec32* w32 = nullptr;         // F32C walk records
   const Rec32x2* w32x2 = nullptr;     // F32C paired walk records
   const Body32x2* body2 = nullptr;    // sorted bodies, paired layout
@@ -138,8 +137,8 @@ int com_long_chain(int64_t n);
 int com_long_cells(phys_ctx* c, int64_t n, int64_t nnodes, int64_t total, const int32_t* eoff,
                    const double4* eb, const TreeHeader* hdr, const int32_t* longs, double4* mc);
 // walk.cu
-// Tasks that the exact walk of this evaluation may be split into (0: one walk
-// per target).
+// Most tasks that the exact walk of this evaluation may be split into (0: one
+// walk per target).
 int exact_walk_tasks(const phys_ctx* c, int64_t n);
 int bh_group_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force,
                   double* ox, double* oy, double* oz);

@@ -972,15 +972,21 @@ top_tree_kernel(int64_t nnodes, const int4* __restrict__ link, const int32_t* __
 }
 
 // The tasks by falling number of bodies: the walk takes the long ones first.
+// nt = 0: the root as the one task.
 __global__ void __launch_bounds__(512)
-task_order_kernel(int max_tasks, int max_top, const int32_t* __restrict__ counts,
-                  const int4* __restrict__ link, const int32_t* __restrict__ task,
-                  int32_t* __restrict__ order, int32_t* __restrict__ queue) {
+task_order_kernel(int nt, const int4* __restrict__ link, int32_t* __restrict__ task,
+                  int4* __restrict__ top, int32_t* __restrict__ order,
+                  int32_t* __restrict__ queue) {
   wait_for_previous();
   __shared__ int bodies[512];
-  const int i = threadIdx.x, c = *counts, nt = c >> 16;
-  if (i == 0) *queue = 0;
-  if (nt > max_tasks || (c & 0xffff) > max_top) return;  // walked as one task
+  const int i = threadIdx.x;
+  if (i == 0) {
+    *queue = 0;
+    if (nt == 0) {
+      task[0] = order[0] = 0;
+      top[0] = make_int4(0, 0, 0, 0);
+    }
+  }
   if (i < nt) {
     const int4 l = link[task[i]];
     bodies[i] = l.z - l.y;
@@ -1273,20 +1279,58 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
   double4* mc = nullptr;
   PHYS_TRY(ws_alloc(c, WS_NODE_S, nnodes, &mc));
   float4* wx = nullptr;
+  TopTree top;
   if (exact) {
     int32_t* ncnt = nullptr;
     PHYS_TRY(ws_alloc(c, WS_KEEP, nnodes + 1, &ncnt));
-    int32_t* eoff = nullptr;
-    PHYS_TRY(ws_alloc(c, WS_EOFF, nnodes + 1, &eoff));
+    int32_t* eoff = nullptr;  // pairs before each node; then (tasks, top nodes) before each
+    PHYS_TRY(ws_alloc(c, WS_EOFF, 2 * (nnodes + 1), &eoff));
     PHYS_LAUNCH(c, node_count_kernel, grid_for(nnodes + 1), kBlock, 0, nnodes, link, ncnt);
     PHYS_TRY(scan_exclusive_i32(c, ncnt, eoff, nnodes + 1));
-    PHYS_CUDA(c, cudaMemcpyAsync(hsm, eoff + nnodes, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                 c->stream));
-    PHYS_CUDA(c, cudaStreamSynchronize(c->stream));
+    const int max_tasks = exact_walk_tasks(c, n);
+    if (max_tasks > 0) {
+      // the walk's tasks: their number comes back with that of the pairs
+      constexpr int kMaxTop = 4096;
+      int32_t *off = eoff + (nnodes + 1), *lists = nullptr;
+      PHYS_TRY(ws_alloc(c, WS_NODE_LO, nnodes, &kids));
+      PHYS_TRY(children());
+      PHYS_TRY(ws_alloc(c, WS_GROUPS, 4 * kMaxTop + 2 * max_tasks + 1, &lists));
+      top.top = reinterpret_cast<int4*>(lists);
+      top.task = lists + 4 * kMaxTop;
+      top.order = top.task + max_tasks;
+      top.queue = top.order + max_tasks;
+      top.parent = parent;
+      // finer tasks balance better and cost more walking and adding: 20000
+      // bodies 0.41 / 0.44 / 0.48 ms with n/16 / n/12 / n/8, 32768 0.62 / 0.58
+      // with n/16 / n/8, 65536 1.10 / 1.05 with n/8 / n/5; and they must fit
+      // (nested cells make up to ten tasks and more per n/16 of a disk), else
+      // the root is the one task (100 000 bodies in nested cells 2.11 ms, the
+      // kernel for more targets 2.34)
+      const int most =
+          (int)(n / (max_tasks >= 256 ? 16 : max_tasks >= 160 ? 12 : max_tasks >= 80 ? 8 : 5));
+      PHYS_LAUNCH(c, top_tree_kernel<false>, grid_for(nnodes + 1), kBlock, 0, nnodes, link, parent,
+                  most, ncnt, off, max_tasks, kMaxTop, top.task, top.top);
+      PHYS_TRY(scan_exclusive_i32(c, ncnt, off, nnodes + 1));
+      PHYS_LAUNCH(c, top_tree_kernel<true>, grid_for(nnodes + 1), kBlock, 0, nnodes, link, parent,
+                  most, ncnt, off, max_tasks, kMaxTop, top.task, top.top);
+      PHYS_CUDA(c, cudaMemcpy2DAsync(hsm, 4, eoff + nnodes, 4 * (nnodes + 1), 4, 2,
+                                     cudaMemcpyDeviceToHost, c->stream));
+      PHYS_CUDA(c, cudaStreamSynchronize(c->stream));
+      const int nt = hsm[1] >> 16, np = hsm[1] & 0xffff;
+      const bool fit = nt <= max_tasks && np <= kMaxTop;
+      top.ntask = fit ? nt : 1;
+      top.ntop = fit ? np : 1;
+      PHYS_LAUNCH(c, task_order_kernel, 1, 512, 0, fit ? nt : 0, link, top.task, top.top,
+                  top.order, top.queue);
+    } else {
+      PHYS_CUDA(c, cudaMemcpyAsync(hsm, eoff + nnodes, sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                   c->stream));
+      PHYS_CUDA(c, cudaStreamSynchronize(c->stream));
+    }
     const int64_t total = (uint32_t)hsm[0];
     if (total <= 0 || total >= (int64_t(1) << 31))
       return fail(c, PHYS_ERR_ARG, "exact centre of mass needs < 2^31 (cell, body) pairs");
-    // the pairs' slots take the child ids and the walk's records afterwards
+    // the pairs' slots take the walk's records (and the child ids) afterwards
     const int64_t room = std::max(total, nnodes * (int64_t)(sizeof(Kids) / sizeof(uint64_t)));
     uint64_t* ent = nullptr;
     PHYS_TRY(ws_alloc(c, WS_ENTRIES, room, &ent));
@@ -1313,50 +1357,21 @@ int bh_build(phys_ctx* c, const phys_params* p, bool need_f32, BhTree* t, bool n
     PHYS_LAUNCH(c, com_recurrence_kernel, grid_for(nnodes, 128, 1 << 30), 128, 0, nnodes, eoff, eb,
                 mc, link, c->d_hdr, full_com ? 0 : 1, com_long_chain(n), longs, c->d_status);
     PHYS_TRY(com_long_cells(c, n, nnodes, total, eoff, eb, c->d_hdr, longs, mc));
-    kids = reinterpret_cast<Kids*>(ent);
     wx = reinterpret_cast<float4*>(ent_alt);
-    PHYS_TRY(children());
+    if (!kids) {
+      kids = reinterpret_cast<Kids*>(ent);
+      PHYS_TRY(children());
+    }
   } else {
     PHYS_CUDA(c, cudaMemsetAsync(arrive, 0, sizeof(int32_t) * (nnodes + 1), c->stream));
     PHYS_LAUNCH(c, com_upward_kernel, grid_for(nnodes), kBlock, 0, nnodes, link, parent, nchild,
                 kids, arrive, body64, mc, c->d_status);
   }
   double4* rec64 = nullptr;
-  TopTree top;
   Rec32* w32 = nullptr;
   Rec64* w64 = nullptr;
   Rec32x2* w32x2 = nullptr;
-  if (exact) {
-    PHYS_TRY(ws_alloc(c, WS_NODE_PM, nnodes, &rec64));
-    top.max_tasks = exact_walk_tasks(c, n);
-    if (top.max_tasks > 0) {
-      int32_t *cnt2 = nullptr, *off2 = nullptr, *lists = nullptr;
-      top.max_top = 4096;
-      PHYS_TRY(ws_alloc(c, WS_NCOUNT, nnodes + 1, &cnt2));
-      PHYS_TRY(ws_alloc(c, WS_GROUP_OFF, nnodes + 1, &off2));
-      PHYS_TRY(ws_alloc(c, WS_GROUPS, 4 * top.max_top + 2 * top.max_tasks + 1, &lists));
-      top.top = reinterpret_cast<int4*>(lists);
-      top.task = lists + 4 * top.max_top;
-      top.order = top.task + top.max_tasks;
-      top.queue = top.order + top.max_tasks;
-      top.counts = off2 + nnodes;
-      top.parent = parent;
-      // finer tasks balance better and cost more walking and adding: 20000
-      // bodies 0.41 / 0.44 / 0.48 ms with n/16 / n/12 / n/8, 32768 0.62 / 0.58
-      // with n/16 / n/8, 65536 1.10 / 1.05 with n/8 / n/5; and they must fit
-      // (nested cells make up to ten tasks and more per n/16 of a disk; with
-      // too many the tree is walked as one task, 24000 bodies 0.96 ms for 0.49)
-      const int room = top.max_tasks;
-      const int most = (int)(n / (room >= 256 ? 16 : room >= 160 ? 12 : room >= 80 ? 8 : 5));
-      PHYS_LAUNCH(c, top_tree_kernel<false>, grid_for(nnodes + 1), kBlock, 0, nnodes, link, parent,
-                  most, cnt2, off2, top.max_tasks, top.max_top, top.task, top.top);
-      PHYS_TRY(scan_exclusive_i32(c, cnt2, off2, nnodes + 1));
-      PHYS_LAUNCH(c, top_tree_kernel<true>, grid_for(nnodes + 1), kBlock, 0, nnodes, link, parent,
-                  most, cnt2, off2, top.max_tasks, top.max_top, top.task, top.top);
-      PHYS_LAUNCH(c, task_order_kernel, 1, 512, 0, top.max_tasks, top.max_top, top.counts, link,
-                  top.task, top.order, top.queue);
-    }
-  }
+  if (exact) PHYS_TRY(ws_alloc(c, WS_NODE_PM, nnodes, &rec64));
 #ifndef WALK_PAIRED
 #define WALK_PAIRED 1
 #endif

@@ -507,13 +507,6 @@ __device__ __forceinline__ ExactTarget exact_target(const double4* body64, int64
   return ExactTarget{b.x, b.y, b.z, xmul(G, b.w)};
 }
 
-// Number of tasks; a tree with more top nodes than there is room for is
-// walked as one task, the root.
-__device__ __forceinline__ int top_tasks(const TopTree& top) {
-  const int c = *top.counts, nt = c >> 16;
-  return nt <= top.max_tasks && (c & 0xffff) <= top.max_top ? nt : 1;
-}
-
 // Force -> output of one target (a = F / m unless the force is wanted).
 __device__ __forceinline__ void exact_store(double fx, double fy, double fz, double mi,
                                             uint32_t i, int want_force, double* ox, double* oy,
@@ -550,7 +543,7 @@ walk_exact_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const float4
   __shared__ int qnode[kXWarps][kXQ];
   __shared__ unsigned qmask[kXWarps][kXQ];    // lanes that take it
   __shared__ unsigned qlevels[kXWarps][kXQ];  // 0: those of the entry before
-  const int ntask = kWhole ? 1 : top_tasks(top);
+  const int ntask = kWhole ? 1 : top.ntask;
   const double theta2 = hdr->theta2, half = hdr->half;
   for (int d = threadIdx.x; d < kMaxLevels; d += blockDim.x) {
     s2d[d] = hdr->s2[d];
@@ -575,8 +568,8 @@ walk_exact_kernel(int64_t q0, int64_t n, int64_t nbody, int nnodes, const float4
       run = it - task * nrun;
     }
     if (run >= nrun || task >= ntask) break;
-    if (!kWhole && ntask > 1) task = top.order[task];
-    const int root = ntask == 1 ? 0 : top.task[task];
+    if (!kWhole) task = top.order[task];
+    const int root = kWhole ? 0 : top.task[task];
     const int64_t p = q0 + run * 32 + lane;
     const bool valid = p < n;
     const int p0 = (int)(p - lane);
@@ -823,7 +816,7 @@ exact_combine_kernel(int64_t q0, int64_t n, const float4* __restrict__ wx,
   const bool valid = p < n;
   const ExactTarget t = exact_target(body64, valid ? p : q0, true, G);
   const double theta2 = hdr->theta2;
-  const int ntop = top_tasks(top) == 1 ? 1 : *top.counts & 0xffff;
+  const int ntop = top.ntop;
   unsigned ninter = 0;
   NestedSum sum;
   double outer[kMaxLevels + 1][3];
@@ -832,13 +825,10 @@ exact_combine_kernel(int64_t q0, int64_t n, const float4* __restrict__ wx,
   for (int i0 = 0; i0 < ntop; i0 += kStage) {
     __syncthreads();
     const int i = i0 + (int)threadIdx.x;
-    if (threadIdx.x < kStage) {
-      const int4 e = ntop == 1 ? make_int4(0, 0, 0, 0)
-                               : i < ntop ? top.top[i] : make_int4(0, -1, 0, 0);
-      const bool gate = e.x == 0 || (__float_as_int(wx[e.x].w) & kMetaGate);
-      se[threadIdx.x] = make_int4(e.x, e.y, e.z, gate);
-      sr[threadIdx.x] = rec64[e.x];
-    }
+    const int4 e = i < ntop ? top.top[i] : make_int4(0, -1, 0, 0);
+    const bool gate = e.x == 0 || (__float_as_int(wx[e.x].w) & kMetaGate);
+    se[threadIdx.x] = make_int4(e.x, e.y, e.z, gate);
+    sr[threadIdx.x] = rec64[e.x];
     __syncthreads();
     for (int k0 = 0; k0 < min(kStage, ntop - i0); k0 += kAhead) {
       // the contributions of several tasks are read together
@@ -888,8 +878,8 @@ int exact_walk_tasks(const phys_ctx* c, int64_t n) {
   int64_t q0 = 0, q1 = n;
   target_range(c, n, q0, q1);
   const int64_t nt = q1 - q0;
-  // `part` holds 24 bytes per task and target: at most 100 MB, 200 MB for
-  // more than 65536 targets (64 tasks)
+  // `part` holds 24 bytes per task that the tree has and target: at most 100 MB,
+  // 200 MB for more than 65536 targets (64 tasks)
   if (nt <= 0 || nt > 131072) return 0;
   return (int)std::max<int64_t>(64, min64(512, (int64_t(1) << 22) / nt));
 }
@@ -908,7 +898,7 @@ int bh_walk(phys_ctx* c, const phys_params* p, const BhTree& t, bool want_force,
   if (p->flags & PHYS_FLAG_GROUP_WALK) {
     PHYS_TRY(bh_group_walk(c, p, t, want_force, ox, oy, oz));
   } else if (p->precision == PHYS_F64_EXACT) {
-    const int tasks = t.top.max_tasks;
+    const int tasks = t.top.ntask;
     const int xgrid = (int)ceil_div(nt > 0 ? nt : 1, kXTargets);
     if (tasks > 0) {
       double* part = nullptr;
