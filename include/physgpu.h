@@ -326,9 +326,10 @@ int phys_ensemble_autotune(phys_ctx* ctx, const phys_params* p, double dt, int64
  * uploaded state (which is left unchanged).  phys_adjoint_direct returns L
  * and dL/dx0, dL/dv0, dL/dm (each output may be NULL) by a reverse sweep
  * through the acceleration's Jacobian and the Verlet step.  The positions of
- * every step are kept where they fit in 256 MiB (24 bytes per body and step);
- * else (x, v) is checkpointed every `checkpoint` steps and each segment
- * recomputed, with the same results bit for bit.
+ * every step are kept where they fit in 256 MiB (24 bytes per body and step)
+ * and that much can be allocated; else (x, v) is checkpointed every
+ * `checkpoint` steps and each segment recomputed, with the same results bit
+ * for bit.
  * phys_trajectory_loss is the same forward pass only (finite differences). */
 int phys_adjoint_direct(phys_ctx* ctx, const phys_params* p, double dt, int64_t nsteps,
                         int64_t checkpoint, const double* tx, const double* ty, const double* tz,

@@ -20,8 +20,8 @@
 //     (J^T w)_j = G sum_{i != j} K_ij (m_j w_i - m_i w_j)
 //     (dA/dm)^T w)_j = G sum_{i != j} (r_ij . w_i) / s^3
 // Positions are kept for a whole segment of steps (the trajectory, where it
-// fits in kHistoryBytes; else `checkpoint` steps, with (x, v) kept at the
-// segment starts and the segments before the last recomputed,
+// fits in kHistoryBytes and can be allocated; else `checkpoint` steps, with
+// (x, v) kept at the segment starts and the segments before the last recomputed,
 // deterministically, bit for bit, during the reverse sweep).
 //
 // A forward step is two kernels, the sliced force sum and one that adds up the
@@ -310,15 +310,11 @@ int vjp(phys_ctx* c, const phys_params* p, Adj& a, const double* x) {
   return PHYS_OK;
 }
 
-int setup(phys_ctx* c, int64_t T, int64_t K, bool reverse, Adj& a) {
-  const int64_t n = c->n;
-  a.n = n;
-  a.T = T;
-  if (reverse && (T + 1) * 3 * n * (int64_t)sizeof(double) <= kHistoryBytes)
-    K = std::max<int64_t>(T, 1);
+// Everything but the partial sums, for segments of K steps.
+int setup_segments(phys_ctx* c, int64_t K, bool reverse, Adj& a) {
+  const int64_t n = a.n, T = a.T;
   a.K = reverse ? std::min<int64_t>(K, std::max<int64_t>(T, 1)) : 0;
   a.nck = reverse ? std::max<int64_t>(ceil_div(T, a.K), 1) : 0;
-  a.plan = f64_plan(n, INT64_MAX);
   const size_t doubles = 9 * n + a.nck * 6 * n + (a.K + 1) * 3 * n + 13 * n;
   int st = PHYS_OK;
   double* b = (double*)ws_get(c, WS_ADJ0, sizeof(double) * doubles, &st);
@@ -333,6 +329,15 @@ int setup(phys_ctx* c, int64_t T, int64_t K, bool reverse, Adj& a) {
   a.abar = b; b += 3 * n;
   a.mbar = b; b += n;
   a.tgt = b; b += 3 * n;
+  return PHYS_OK;
+}
+
+int setup(phys_ctx* c, int64_t T, int64_t K, bool reverse, Adj& a) {
+  const int64_t n = c->n;
+  a.n = n;
+  a.T = T;
+  a.plan = f64_plan(n, INT64_MAX);
+  int st = PHYS_OK;
   a.fpart = (double*)ws_get(c, WS_ADJ1, sizeof(double) * 3 * n * a.plan.slices, &st);
   if (st) return st;
   a.vpart = (double*)ws_get(c, WS_ADJ2, sizeof(double) * 4 * n * a.plan.slices, &st);
@@ -340,7 +345,12 @@ int setup(phys_ctx* c, int64_t T, int64_t K, bool reverse, Adj& a) {
   a.lpart = (double*)ws_get(c, WS_ADJ3, sizeof(double) * (148 * 8 + 8), &st);
   if (st) return st;
   a.loss = a.lpart + 148 * 8;
-  return PHYS_OK;
+  if (reverse && K < T && (T + 1) * 3 * n * (int64_t)sizeof(double) <= kHistoryBytes) {
+    st = setup_segments(c, T, reverse, a);
+    if (st != PHYS_ERR_OOM) return st;
+    c->err.clear();  // no room for every step: the caller's interval
+  }
+  return setup_segments(c, K, reverse, a);
 }
 
 int copy_d2d(phys_ctx* c, double* dst, const double* src, int64_t count) {
