@@ -395,10 +395,10 @@ __device__ __forceinline__ double exact_scale(double a, double x) {
   const double z = __fma_rn(__fma_rn(-s3, z1, 1.0), z1, z1);
   return div_recip(a, s3, z);
 }
+// Positions within +-2^98 have |r|^2 < 3 x 2^198, which leaves 2^198 below 2^200.
 __host__ __device__ inline bool scale_eps2_ok(double eps2) {
-  return eps2 >= 0x1p-200 && eps2 < 0x1p199;
+  return eps2 >= 0x1p-200 && eps2 < 0x1p197;
 }
-// Coordinates within +-2^98: |r|^2 < 3 x 2^198.
 __device__ __forceinline__ bool scale_pos_ok(double x, double y, double z) {
   return fmax(fmax(fabs(x), fabs(y)), fabs(z)) < 0x1p98 && x == x && y == y && z == z;
 }
