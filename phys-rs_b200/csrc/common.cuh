@@ -402,6 +402,10 @@ __host__ __device__ inline bool scale_eps2_ok(double eps2) {
 __device__ __forceinline__ bool scale_pos_ok(double x, double y, double z) {
   return fmax(fmax(fabs(x), fabs(y)), fabs(z)) < 0x1p98 && x == x && y == y && z == z;
 }
+// |r|^2 + eps^2 in [2^-200, 2^200).
+__device__ __forceinline__ bool scale_square_ok(double x) {
+  return (unsigned)__double2hiint(x) - (823u << 20) < (400u << 20);
+}
 // |v| in [2^-250, 2^250) or 0.
 __device__ __forceinline__ bool scale_mass_ok(double v) {
   return ((unsigned)__double2hiint(v) & 0x7fffffffu) - (773u << 20) < (500u << 20) || v == 0.0;

@@ -26,9 +26,8 @@ namespace {
 // (the next chunk's terms are read while the current chunk's are added).  A
 // skipped term (j == i, past the end) is stored as +-0: the sum starts from
 // +0 and so is never -0, and adding a zero leaves every value as it is.  A
-// lane whose source, or a block one of whose targets, is outside
-// exact_scale's range forms its terms again with the library's square root
-// and division.
+// chunk with a source, or a block with a target, outside exact_scale's range
+// takes the library's square root and division instead.
 //
 // The floor of any exact form is the ordered chain, N - 1 additions of 8.2
 // cycles (4.3 us at N = 1024; the adding warp takes 10.6 per source), and for
@@ -58,20 +57,20 @@ struct TickArgs {
 // kProd = 6, 8 warps, 8 targets: warps 1-3 and 5-7 produce, so that no
 // producer shares warp 0's scheduler (warps go to an SM's four schedulers by
 // index) while a block has an SM to itself (N = 1024: 9.5 us a launch inside a
-// graph, 13.0 with the other layout); kProd = 4, 5 warps, 10 targets, four
-// blocks per SM: more adding warps per SM once there are more blocks than SMs
-// (N = 4096: 68 us against 78).
-// kFast: eps^2 is in exact_scale's range; else (no softening) every pair
-// takes the library's operations.
-template <bool kFast>
-__device__ __forceinline__ double pair_weight(double a, double x) {
-  return kFast ? exact_scale(a, x) : exact_scale_ieee(a, x);
-}
-
+// graph, 13.0 with the other layout), and up to two such blocks an SM (a tick
+// of 1500 bodies 19.1 against 22.0 us, of 2368 26.9 against 32.4); kProd = 4, 5
+// warps, 10 targets, four blocks per SM: more adding warps per SM once there
+// are more blocks (N = 4096: 68 us against 78).
+// kSoft: eps^2 alone keeps |r|^2 + eps^2 in exact_scale's range; else (no
+// softening) every pair is looked at, and a chunk with one outside (coincident
+// bodies) is formed again.  Against library operations for all of these, and
+// for masses or positions out of range against both forms in turn: a tick of
+// 1500 bodies 35.8 -> 19.3 us without softening, 50.1 -> 28.6 with masses of
+// 1e-103 (31.8 before either form had the branch-free weight).
 constexpr int x_block(int prod) { return prod == 6 ? 256 : 32 * (prod + 1); }
 constexpr int x_targets(int prod) { return prod == 6 ? 8 : 10; }
 
-template <int kProd, bool kTick, bool kFast>
+template <int kProd, bool kTick, bool kSoft>
 __global__ void __launch_bounds__(x_block(kProd), kProd == 6 ? 2 : 4)
 direct_exact_kernel(int64_t n, int64_t t0, int64_t t1, const double* __restrict__ x,
                     const double* __restrict__ y, const double* __restrict__ z,
@@ -107,8 +106,11 @@ direct_exact_kernel(int64_t n, int64_t t0, int64_t t1, const double* __restrict_
       const int64_t j = k * (int64_t)32 + lane;
       const double4 src = load(j);
       if (k >= kProd) pair_sync(1 + kProd + p);
+      bool in_range = __all_sync(0xffffffffu, targets_ok && scale_pos_ok(src.x, src.y, src.z) &&
+                                                  scale_mass_ok(src.w));
+      bool pairs_ok = true;
 #pragma unroll 1
-      for (int tg = 0; tg < kXT; tg += kXGroup) {
+      for (int tg = 0; tg < kXT && in_range; tg += kXGroup) {
         // every weight of the group first: a store between two of them would
         // keep the second pair's chain behind the first's
         double rx[kXGroup], ry[kXGroup], rz[kXGroup], wt[kXGroup];
@@ -117,8 +119,11 @@ direct_exact_kernel(int64_t n, int64_t t0, int64_t t1, const double* __restrict_
           const int t = tg + u;
           const double4 T = tgt[t];
           rx[u] = xsub(src.x, T.x), ry[u] = xsub(src.y, T.y), rz[u] = xsub(src.z, T.z);
-          wt[u] = pair_weight<kFast>(xmul(T.w, src.w), xadd(xlen2(rx[u], ry[u], rz[u]), eps2));
-          if (j >= n || j == i0 + t) wt[u] = 0.0;
+          const double x2 = xadd(xlen2(rx[u], ry[u], rz[u]), eps2);
+          wt[u] = exact_scale(xmul(T.w, src.w), x2);
+          const bool none = j >= n || j == i0 + t;
+          if (!kSoft) pairs_ok &= none || scale_square_ok(x2);
+          if (none) wt[u] = 0.0;
         }
 #pragma unroll
         for (int u = 0; u < kXGroup; ++u) {
@@ -127,12 +132,13 @@ direct_exact_kernel(int64_t n, int64_t t0, int64_t t1, const double* __restrict_
           term[p][2 * kXT + tg + u][lane] = xmul(rz[u], wt[u]);
         }
       }
-      if (kFast && !(targets_ok && scale_pos_ok(src.x, src.y, src.z) && scale_mass_ok(src.w))) {
-        for (int t = 0; t < kXT; ++t) {  // out of range: this lane's terms again
+      if (!kSoft) in_range &= __all_sync(0xffffffffu, pairs_ok);
+      if (!in_range) {
+        for (int t = 0; t < kXT; ++t) {
           const double4 T = tgt[t];
-          if (j >= n || j == i0 + t) continue;
           const double rx = xsub(src.x, T.x), ry = xsub(src.y, T.y), rz = xsub(src.z, T.z);
-          const double wt = exact_scale_ieee(xmul(T.w, src.w), xadd(xlen2(rx, ry, rz), eps2));
+          double wt = exact_scale_ieee(xmul(T.w, src.w), xadd(xlen2(rx, ry, rz), eps2));
+          if (j >= n || j == i0 + t) wt = 0.0;
           term[p][t][lane] = xmul(rx, wt);
           term[p][kXT + t][lane] = xmul(ry, wt);
           term[p][2 * kXT + t][lane] = xmul(rz, wt);
@@ -194,13 +200,13 @@ template <bool kTick>
 int launch_exact(phys_ctx* c, const phys_params* p, int64_t t0, int64_t t1, const double* x,
                  const double* y, const double* z, int want_force, double* ox, double* oy,
                  double* oz, const TickArgs& tick) {
-  const bool solo = t1 - t0 <= 148 * x_targets(6);  // each block has an SM to itself
+  const bool solo = t1 - t0 <= 2 * 148 * x_targets(6);
   const int64_t blocks = ceil_div(t1 - t0, solo ? x_targets(6) : x_targets(4));
   const double eps2 = p->eps * p->eps;
-  const bool fast = scale_eps2_ok(eps2);
-  auto kernel = solo ? (fast ? direct_exact_kernel<6, kTick, true>
+  const bool soft = scale_eps2_ok(eps2);
+  auto kernel = solo ? (soft ? direct_exact_kernel<6, kTick, true>
                              : direct_exact_kernel<6, kTick, false>)
-                     : (fast ? direct_exact_kernel<4, kTick, true>
+                     : (soft ? direct_exact_kernel<4, kTick, true>
                              : direct_exact_kernel<4, kTick, false>);
   PHYS_LAUNCH(c, kernel, (int)blocks, solo ? x_block(6) : x_block(4), 0, c->n, t0, t1, x, y, z,
               c->m, p->G, eps2, want_force, ox, oy, oz, tick, c->d_status);
