@@ -36,11 +36,13 @@
 // division, by itself.  Masses of both signs have the same steps wherever the
 // running mass is positive; their running masses are summed in turn.
 //
-// Tree phase of the exact form, one chain per cell before against segments
-// (Plummer spheres): 10 000 bodies 0.59 -> 0.32 ms, 100 000 4.8 -> 1.26 ms,
-// 300 000 9.6 -> 2.2 ms, 2^20 (longest chain 387 000) 25.7 -> 9.8 ms.  The
-// candidates' steps bound it: 7 FP64 operations each, a dependent chain of 57
-// cycles a body.
+// Tree phase of an exact evaluation, one chain per cell before against
+// segments: Plummer spheres of 10 000 bodies 0.82 -> 0.35 ms, 100 000 4.2 ->
+// 1.28 ms, 300 000 7.3 -> 2.1 ms, 2^20 16.1 -> 8.6 and 18.3 -> 9.9 ms (two
+// seeds; the longest chain decides); in a plane 0.84 -> 0.46, 4.4 -> 1.5 and
+// 25.6 -> 9.3 ms at 10 000, 100 000 and 2^20; masses of both signs 7.0 -> 3.3
+// and 66 -> 33 ms at 100 000 and 2^20.  The candidates' steps bound it: 7 FP64
+// operations each, a dependent chain of 57 cycles a body.
 #include "bh.cuh"
 
 namespace phys {

@@ -381,7 +381,9 @@ __device__ __forceinline__ bool div_recip_num_ok(double a) {
 // of both positions), a the product of two scale_mass_ok values (the sign of
 // a zero result may differ from the library's).  Elsewhere the caller takes
 // exact_scale_ieee.  4 x 10^10 random pairs over these ranges equal the
-// library's results.
+// library's results (one run of a program of its own, as were the comparisons
+// of the hard roots and of inv_cubed below; the tests keep the edges of the
+// ranges and whole sums).
 __device__ __forceinline__ double exact_scale(double a, double x) {
   double y0;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));

@@ -414,14 +414,16 @@ walk2_kernel(int q64, int n, int nnodes, const Rec32x2* __restrict__ w, const Bo
 // 10 000 bodies and n/8, so it must not start last.  Split against whole
 // walks: 0.29 / 0.96 ms at 10 000 bodies, 0.58 / 1.21 at 32768, 1.05 / 1.54 at
 // 65536, 1.57 / 1.89 at 100 000, 4.8 / 4.9 at 300 000 (and a block per pair in
-// grid order: 0.32 at 10 000, 0.86 at 32768, 1.27 at 65536).
+// grid order: 0.32 at 10 000, 0.86 at 32768, 1.27 at 65536).  Masses of both
+// signs: 0.20 ms at 10 000, 1.7 at 100 000, 13.9 at 2^20 (a node per step 1.19,
+// 2.5 and 18.0; every cell in f64 with the library's weights 0.26, 3.25, 24.8).
 //
 // Bound by the terms: 3300 entries a warp at 300 000 bodies (2100 per target),
 // 38 FP64 instructions and about as many others each, at 47 % of the FP64
 // pipe; without them the traversal takes 1.1 of 5.0 ms.  Two entries at a time
 // and 24 warps an SM do best on a full chip (four: 17.3 ms at 2^20), four with
-// 16 warps when the tasks' tails show (0.32 against 0.34 ms at 10 000, in grid order).  One
-// walk per target, a node per step and its term evaluated in place, took 19.8
+// 16 warps when the tasks' tails show (0.32 against 0.34 ms at 10 000, in grid
+// order).  One walk per target, a node per step and its term evaluated in place, took 19.8
 // ms at 2^20 bodies against 15.5; split, a node per step, 0.44 at 10 000.
 // ---------------------------------------------------------------------------
 constexpr unsigned kFull = 0xffffffffu;
